@@ -1,0 +1,358 @@
+// otg_order.cuh — canonical order of query results, (query << 32 | id) items with an optional
+// distance, in CSR form: ids ascending per query, or (distance, id) ascending per query.
+//
+// By runs: a counting pass places every item in its query's run, and each run is sorted on the chip
+// (one warp up to kRunSortMax items, one block up to kBlockRunMax). Bound by the passes over the
+// items (about 40 bytes each) where the radix sorts it replaces move 24 bytes of every item per
+// 8-bit digit (13 passes for distances: three keys of 20, 64 and 15 bits).
+// By bits: dense id results as one row of bits per query; see order_by_bits.
+#pragma once
+
+#include "otg_query.cuh"
+
+namespace otg
+{
+
+// the count of every query and each item's slot in its query's run (the lanes of a warp that hold
+// the same query take their slots with one atomic)
+__global__ void query_slots_kernel(const u64* __restrict__ items, u64 m, u32* __restrict__ cnt, u32* __restrict__ slot)
+{
+  const u32 lane = threadIdx.x & 31;
+  const u64 stride = u64(gridDim.x) * blockDim.x;
+  for (u64 base = blockIdx.x * u64(blockDim.x) + (threadIdx.x & ~31u); base < m; base += stride)
+  {
+    const u64 i = base + lane;
+    const bool v = i < m;
+    const u32 q = v ? u32(items[i] >> 32) : 0xffffffffu;
+    const u32 peers = __match_any_sync(~0u, q);
+    const int leader = __ffs(int(peers)) - 1;
+    u32 b = 0;
+    if (v && int(lane) == leader)
+      b = atomicAdd(&cnt[q], u32(__popc(peers)));
+    b = __shfl_sync(~0u, b, leader);
+    if (v)
+      slot[i] = b + __popc(peers & ((1u << lane) - 1u));
+  }
+}
+__global__ void query_scatter_kernel(const u64* __restrict__ items, const double* __restrict__ dist, const u32* __restrict__ slot, u64 m,
+                                     const u64* __restrict__ off, u32* __restrict__ ids, double* __restrict__ distOut)
+{
+  for (u64 i = blockIdx.x * u64(blockDim.x) + threadIdx.x; i < m; i += u64(gridDim.x) * blockDim.x)
+  {
+    const u64 it = items[i];
+    const u64 to = off[u32(it >> 32)] + slot[i];
+    ids[to] = u32(it);
+    if (dist)
+      distOut[to] = dist[i];
+  }
+}
+
+// sort key of an item: the distance's bits (distances are >= 0, so bit order is value order), then
+// the id; without distances the id alone
+template<bool DIST>
+struct RunKey
+{
+  u64 d;
+  u32 id;
+  __device__ __forceinline__ bool less(const RunKey& o) const { return DIST ? (d < o.d || (d == o.d && id < o.id)) : id < o.id; }
+};
+
+template<bool DIST>
+__device__ __forceinline__ RunKey<DIST> run_load(const u32* ids, const double* dist, u64 i)
+{
+  RunKey<DIST> k;
+  k.id = ids[i];
+  k.d = DIST ? u64(__double_as_longlong(dist[i])) : 0;
+  return k;
+}
+
+// ascending bitonic sort of one key per lane
+template<bool DIST>
+__device__ __forceinline__ void run_sort_lanes(RunKey<DIST>& v, u32 lane)
+{
+#pragma unroll
+  for (u32 k = 2; k <= 32; k <<= 1)
+#pragma unroll
+    for (u32 j = k >> 1; j > 0; j >>= 1)
+    {
+      RunKey<DIST> o;
+      o.id = __shfl_xor_sync(~0u, v.id, j);
+      o.d = DIST ? __shfl_xor_sync(~0u, v.d, j) : 0;
+      const bool up = (lane & k) == 0, lower = (lane & j) == 0;
+      const bool take = (lower == up) ? o.less(v) : v.less(o);
+      if (take)
+        v = o;
+    }
+}
+
+// One warp per query sorts its run in place: each 32 items in registers, then every item's place is
+// its place among its 32 plus the counts of smaller items in the other sorted groups (binary
+// searches in shared memory). Runs above kRunSortMax go to the list longRuns[2 ...] (longRuns[0]
+// counts them) for run_sort_block_kernel. A bitonic network over 128 items takes twice the steps.
+constexpr u32 kRunSortMax = 256;
+constexpr int kRunSortWarps = 8;
+template<bool DIST>
+__global__ void __launch_bounds__(kRunSortWarps * 32) run_sort_kernel(const u64* __restrict__ off, u64 nq, u32* __restrict__ ids, double* __restrict__ dist,
+                                                                    u32* __restrict__ longRuns, u32 longCap)
+{
+  __shared__ u64 sd[DIST ? kRunSortWarps : 1][DIST ? kRunSortMax : 1];
+  __shared__ u32 si[kRunSortWarps][kRunSortMax];
+  const u32 lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const u64 warps = u64(gridDim.x) * kRunSortWarps;
+  for (u64 q = u64(blockIdx.x) * kRunSortWarps + w; q < nq; q += warps)
+  {
+    const u64 b = off[q];
+    const u64 len64 = off[q + 1] - b;
+    if (len64 <= 1)
+      continue;
+    if (len64 > kRunSortMax)
+    {
+      if (lane == 0)
+      {
+        const u32 at = atomicAdd(longRuns, 1u);
+        if (at < longCap)
+          longRuns[2 + at] = u32(q);
+      }
+      continue;
+    }
+    const u32 len = u32(len64);
+    if (len <= 32)
+    {
+      RunKey<DIST> v{ ~0ull, ~0u };
+      if (lane < len)
+        v = run_load<DIST>(ids, dist, b + lane);
+      run_sort_lanes<DIST>(v, lane);
+      if (lane < len)
+      {
+        ids[b + lane] = v.id;
+        if (DIST)
+          dist[b + lane] = __longlong_as_double((long long)v.d);
+      }
+      continue;
+    }
+    const u32 groups = (len + 31) >> 5;
+    for (u32 g = 0; g < groups; ++g)
+    {
+      const u32 i = g * 32 + lane;
+      RunKey<DIST> v{ ~0ull, ~0u };
+      if (i < len)
+        v = run_load<DIST>(ids, dist, b + i);
+      run_sort_lanes<DIST>(v, lane);
+      si[w][i] = v.id;
+      if (DIST)
+        sd[w][i] = v.d;
+    }
+    __syncwarp();
+    for (u32 g = 0; g < groups; ++g)
+    {
+      const u32 i = g * 32 + lane;
+      if (i >= len) // the padding of the last group sorts last in it
+        continue;
+      const RunKey<DIST> v{ DIST ? sd[w][i] : 0, si[w][i] };
+      u32 rank = lane;
+      for (u32 h = 0; h < groups; ++h)
+      {
+        if (h == g)
+          continue;
+        u32 lo = 0;
+#pragma unroll
+        for (u32 s = 16; s > 0; s >>= 1)
+        {
+          const u32 j = h * 32 + lo + s - 1;
+          const RunKey<DIST> o{ DIST ? sd[w][j] : 0, si[w][j] };
+          if (o.less(v))
+            lo += s;
+        }
+        const RunKey<DIST> o{ DIST ? sd[w][h * 32 + lo] : 0, si[w][h * 32 + lo] };
+        rank += lo + (o.less(v) ? 1u : 0u);
+      }
+      ids[b + rank] = v.id;
+      if (DIST)
+        dist[b + rank] = __longlong_as_double((long long)v.d);
+    }
+    __syncwarp();
+  }
+}
+
+// One block per listed run sorts it in place with a bitonic network in shared memory (dynamic: 12 or
+// 4 bytes per item); runs above kBlockRunMax are only counted, in longRuns[1].
+constexpr u32 kBlockRunMax = 8192;
+constexpr int kBlockSortThreads = 512;
+template<bool DIST>
+__global__ void __launch_bounds__(kBlockSortThreads) run_sort_block_kernel(const u64* __restrict__ off, u32* __restrict__ ids, double* __restrict__ dist,
+                                                                         u32* __restrict__ longRuns, u32 longCap)
+{
+  extern __shared__ u64 runMem[];
+  u64* sd = runMem;
+  u32* si = reinterpret_cast<u32*>(runMem + (DIST ? kBlockRunMax : 0));
+  const u32 n = min(longRuns[0], longCap);
+  for (u32 r = blockIdx.x; r < n; r += gridDim.x)
+  {
+    const u32 q = longRuns[2 + r];
+    const u64 b = off[q];
+    const u64 len64 = off[q + 1] - b;
+    if (len64 > kBlockRunMax)
+    {
+      if (threadIdx.x == 0)
+        atomicAdd(longRuns + 1, 1u);
+      continue;
+    }
+    const u32 len = u32(len64);
+    u32 P = 512;
+    while (P < len)
+      P <<= 1;
+    for (u32 i = threadIdx.x; i < P; i += kBlockSortThreads)
+    {
+      si[i] = i < len ? ids[b + i] : ~0u;
+      if (DIST)
+        sd[i] = i < len ? u64(__double_as_longlong(dist[b + i])) : ~0ull;
+    }
+    __syncthreads();
+    for (u32 k = 2; k <= P; k <<= 1)
+      for (u32 j = k >> 1; j > 0; j >>= 1)
+      {
+        for (u32 t = threadIdx.x; t < P / 2; t += kBlockSortThreads)
+        {
+          const u32 i = ((t & ~(j - 1)) << 1) | (t & (j - 1)), x = i + j;
+          const RunKey<DIST> a{ DIST ? sd[i] : 0, si[i] }, c{ DIST ? sd[x] : 0, si[x] };
+          const bool swap = (i & k) == 0 ? c.less(a) : a.less(c);
+          if (swap)
+          {
+            si[i] = c.id;
+            si[x] = a.id;
+            if (DIST)
+            {
+              sd[i] = c.d;
+              sd[x] = a.d;
+            }
+          }
+        }
+        __syncthreads();
+      }
+    for (u32 i = threadIdx.x; i < len; i += kBlockSortThreads)
+    {
+      ids[b + i] = si[i];
+      if (DIST)
+        dist[b + i] = __longlong_as_double((long long)sd[i]);
+    }
+    __syncthreads();
+  }
+}
+
+// ---- order by bits. A row is a whole number of chunks of kBitChunk bits (256 words, one warp's work).
+// Rows of a single tree's queries are all rowChunks long; those of a forest start at rowBase[q].
+constexpr u32 kBitChunk = 8192;
+
+__global__ void bit_rows_kernel(const u32* __restrict__ qTree, const u64* __restrict__ treeOff, u64 nq, u32* __restrict__ rowChunks)
+{
+  for (u64 q = blockIdx.x * u64(blockDim.x) + threadIdx.x; q < nq; q += u64(gridDim.x) * blockDim.x)
+  {
+    const u32 t = qTree[q];
+    rowChunks[q] = u32((treeOff[t + 1] - treeOff[t] + kBitChunk - 1) / kBitChunk);
+  }
+}
+// zeroes the *chunks chunks in use
+__global__ void bit_clear_kernel(uint4* __restrict__ bits, const u64* __restrict__ chunks)
+{
+  const u64 n = *chunks * (kBitChunk / 128);
+  for (u64 i = blockIdx.x * u64(blockDim.x) + threadIdx.x; i < n; i += u64(gridDim.x) * blockDim.x)
+    bits[i] = make_uint4(0u, 0u, 0u, 0u);
+}
+__global__ void bit_mark_kernel(const u64* __restrict__ items, u64 m, const u64* __restrict__ rowBase, u32 rowChunks, u32* __restrict__ bits)
+{
+  for (u64 i = blockIdx.x * u64(blockDim.x) + threadIdx.x; i < m; i += u64(gridDim.x) * blockDim.x)
+  {
+    const u64 it = items[i];
+    const u32 q = u32(it >> 32), id = u32(it);
+    const u64 row = rowBase ? rowBase[q] : u64(q) * rowChunks;
+    atomicOr(&bits[row * (kBitChunk / 32) + (id >> 5)], 1u << (id & 31));
+  }
+}
+// set bits per chunk, one warp each (a chunk past the *used ones counts 0)
+__global__ void bit_count_kernel(const uint4* __restrict__ bits, u64 chunks, const u64* __restrict__ used, u32* __restrict__ cnt)
+{
+  const u32 lane = threadIdx.x & 31;
+  const u64 n = used ? *used : chunks;
+  for (u64 c = (blockIdx.x * u64(blockDim.x) + threadIdx.x) >> 5; c < chunks; c += (u64(gridDim.x) * blockDim.x) >> 5)
+  {
+    u32 s = 0;
+    if (c < n)
+    {
+      const uint4 a = bits[c * 64 + lane], b = bits[c * 64 + 32 + lane];
+      s = __popc(a.x) + __popc(a.y) + __popc(a.z) + __popc(a.w) + __popc(b.x) + __popc(b.y) + __popc(b.z) + __popc(b.w);
+    }
+    for (int o = 16; o > 0; o >>= 1)
+      s += __shfl_xor_sync(~0u, s, o);
+    if (lane == 0)
+      cnt[c] = s;
+  }
+}
+// one warp per chunk writes its ids; the chunks' offsets at the rows' first chunks are the result's.
+// m bounds the ids written (the items marked).
+__global__ void bit_write_kernel(const u32* __restrict__ bits, const u64* __restrict__ off, u64 chunks, const u64* __restrict__ rowBase, u64 nq, u32 rowChunks,
+                                 u64* __restrict__ offsets, u32* __restrict__ ids, u64 m)
+{
+  const u32 lane = threadIdx.x & 31;
+  const u64 tid = blockIdx.x * u64(blockDim.x) + threadIdx.x, threads = u64(gridDim.x) * blockDim.x;
+  for (u64 q = tid; q <= nq; q += threads)
+    offsets[q] = off[rowBase ? rowBase[q] : q * rowChunks];
+  for (u64 c = tid >> 5; c < chunks; c += threads >> 5)
+  {
+    u64 at = off[c];
+    if (off[c + 1] == at)
+      continue;
+    // the row that holds chunk c: its first id in this chunk
+    u64 row = 0;
+    if (rowBase)
+    {
+      u64 lo = 0, hi = nq; // the last row that starts at or before c (rows are not empty)
+      while (hi - lo > 1)
+      {
+        const u64 mid = (lo + hi) >> 1;
+        if (rowBase[mid] <= c)
+          lo = mid;
+        else
+          hi = mid;
+      }
+      row = rowBase[lo];
+    }
+    else
+      row = c / rowChunks * rowChunks;
+    const u32 first = u32(c - row) * kBitChunk;
+    for (u32 k = 0; k < kBitChunk / 32; k += 32)
+    {
+      const u32 word = bits[c * (kBitChunk / 32) + k + lane];
+      const u32 n = __popc(word);
+      u32 incl = n;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1)
+      {
+        const u32 y = __shfl_up_sync(~0u, incl, o);
+        if (lane >= u32(o))
+          incl += y;
+      }
+      const u32 total = __shfl_sync(~0u, incl, 31);
+      if (total >= 256)
+      {
+        // dense: one word after another, one bit per lane, so that the lanes write neighbours
+        for (u32 j = 0; j < 32; ++j)
+        {
+          const u32 wj = __shfl_sync(~0u, word, j);
+          const u64 to = at + __shfl_sync(~0u, incl - n, j) + __popc(wj & ((1u << lane) - 1u));
+          if (((wj >> lane) & 1u) && to < m)
+            ids[to] = first + (k + j) * 32 + lane;
+        }
+      }
+      else
+      {
+        u64 to = at + incl - n;
+        for (u32 b = word; b; b &= b - 1, ++to)
+          if (to < m)
+            ids[to] = first + (k + lane) * 32 + u32(__ffs(int(b)) - 1);
+      }
+      at += total;
+    }
+  }
+}
+
+} // namespace otg

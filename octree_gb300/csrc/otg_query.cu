@@ -18,6 +18,7 @@
 // then ordered with stable radix sorts into CSR form: ids ascending per query, or by
 // (distance, id) for kNN and rays, or (i, j) pairs ascending for collisions.
 #include "otg_query.cuh"
+#include "otg_order.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -1096,14 +1097,18 @@ static int status_of(u32 h)
   return OTG_OK;
 }
 
-// Runs launch(appender) until the append buffer was large enough; items end in c.items.
+// Runs launch(appender) until the append buffer was large enough; items end in c.items. `most` bounds
+// the items (queries times entities): below kItemFloor of them the buffer holds that bound, as a
+// second run costs the whole search again and a larger pooled buffer costs nothing (rays through 1M
+// boxes have 75 hits each where the guess was 16: their search ran twice, 2 x 3.4 ms).
+constexpr u64 kItemFloor = u64(8) << 20;
 template<typename F>
-static int collect(Collected& c, bool withDist, u64 guess, F&& launch, cudaStream_t st)
+static int collect(Collected& c, bool withDist, u64 guess, u64 most, F&& launch, cudaStream_t st)
 {
   cudaError_t e;
   if ((e = c.count.ensure(sizeof(unsigned long long) * 4, st)))
     return cuda_status(e, "allocating counters");
-  u64 cap = std::max<u64>(guess, 1024);
+  u64 cap = std::max<u64>(std::max<u64>(guess, 1024), std::min(most, kItemFloor));
   for (int attempt = 0; attempt < 3; ++attempt)
   {
     if ((e = c.items.ensure(sizeof(u64) * cap, st)) || (withDist && (e = c.dist.ensure(sizeof(double) * cap, st))))
@@ -1135,107 +1140,116 @@ static int collect(Collected& c, bool withDist, u64 guess, F&& launch, cudaStrea
   return OTG_ERR_OUT_OF_MEMORY;
 }
 
-// ---- canonical order of (query, id) results by counting: each query's run, sorted by one warp
-// items (query << 32 | id): the count of every query and each item's slot in its query's run
-// (the lanes of a warp that hold the same query take their slots with one atomic)
-__global__ void query_slots_kernel(const u64* __restrict__ items, u64 m, u32* __restrict__ cnt, u32* __restrict__ slot)
+// The counting order of (query, id[, distance]) items: counts and slots, offsets, items into their
+// runs, each run sorted on the chip (otg_order.cuh). done = false when some run is longer than
+// kBlockRunMax: the caller then orders the whole result by radix sorts (the items are unchanged).
+static int order_by_runs(Collected& c, u64 nq, ResultState& r, bool withDist, cudaStream_t st, bool& done)
 {
-  const u32 lane = threadIdx.x & 31;
-  const u64 stride = u64(gridDim.x) * blockDim.x;
-  for (u64 base = blockIdx.x * u64(blockDim.x) + (threadIdx.x & ~31u); base < m; base += stride)
+  const u64 m = c.m;
+  done = false;
+  // runs longer than kBlockRunMax on average certainly include long ones (counting them would also
+  // put every item's atomic on a few counters)
+  if (m >= (u64(1) << 32) || nq >= (u64(1) << 31) || m > u64(kBlockRunMax) * nq)
+    return OTG_OK;
+  TmpBuf cnt, slot, tileSums, longRuns;
+  const u64 tiles = (nq + kScanTile - 1) / kScanTile;
+  // the list of runs above kRunSortMax: at most m / kRunSortMax of them, after its two counters
+  const u64 longCap = m / kRunSortMax + 1;
+  cudaError_t e;
+  if ((e = cnt.ensure(sizeof(u32) * nq, st)) || (e = slot.ensure(sizeof(u32) * m, st)) || (e = tileSums.ensure(sizeof(u64) * (tiles + 1), st)) ||
+      (e = longRuns.ensure(sizeof(u32) * (2 + longCap), st)))
+    return cuda_status(e, "allocating the result order");
+  cudaMemsetAsync(cnt.p, 0, sizeof(u32) * nq, st);
+  cudaMemsetAsync(longRuns.p, 0, sizeof(u32) * 2, st);
+  query_slots_kernel<<<blocks_for(m), 256, 0, st>>>(c.items.as<u64>(), m, cnt.as<u32>(), slot.as<u32>());
+  scan_reduce_kernel<<<u32(tiles), kScanThreads, 0, st>>>(cnt.as<u32>(), nq, tileSums.as<u64>());
+  scan_tiles_kernel<<<1, kScanThreads, 0, st>>>(tileSums.as<u64>(), tiles);
+  scan_apply_kernel<<<u32(tiles), kScanThreads, 0, st>>>(cnt.as<u32>(), nq, tileSums.as<u64>(), r.offsets.as<u64>());
+  query_scatter_kernel<<<blocks_for(m), 256, 0, st>>>(c.items.as<u64>(), withDist ? c.dist.as<double>() : nullptr, slot.as<u32>(), m, r.offsets.as<u64>(),
+                                                      r.ids.as<u32>(), withDist ? r.dist.as<double>() : nullptr);
+  const u32 grid = u32(std::min<u64>((nq + kRunSortWarps - 1) / kRunSortWarps, 152 * 8));
+  const u32 longGrid = u32(std::min<u64>(longCap, 152 * 2));
+  const u64* off = r.offsets.as<u64>();
+  if (withDist)
   {
-    const u64 i = base + lane;
-    const bool v = i < m;
-    const u32 q = v ? u32(items[i] >> 32) : 0xffffffffu;
-    const u32 peers = __match_any_sync(~0u, q);
-    const int leader = __ffs(int(peers)) - 1;
-    u32 b = 0;
-    if (v && int(lane) == leader)
-      b = atomicAdd(&cnt[q], u32(__popc(peers)));
-    b = __shfl_sync(~0u, b, leader);
-    if (v)
-      slot[i] = b + __popc(peers & ((1u << lane) - 1u));
-  }
-}
-__global__ void query_scatter_kernel(const u64* __restrict__ items, const u32* __restrict__ slot, u64 m, const u64* __restrict__ off, u32* __restrict__ ids)
-{
-  for (u64 i = blockIdx.x * u64(blockDim.x) + threadIdx.x; i < m; i += u64(gridDim.x) * blockDim.x)
-  {
-    const u64 it = items[i];
-    ids[off[u32(it >> 32)] + slot[i]] = u32(it);
-  }
-}
-// One warp per query sorts its run of ids ascending: up to 32 in registers, up to kRunSortMax in
-// shared memory (bitonic networks, padded with ~0); longer runs are only counted in *longRuns (the
-// caller then orders the whole result another way).
-constexpr u32 kRunSortMax = 1024;
-constexpr int kRunSortWarps = 8;
-__global__ void __launch_bounds__(kRunSortWarps * 32) run_sort_kernel(const u64* __restrict__ off, u64 nq, u32* __restrict__ ids, u32* __restrict__ longRuns)
-{
-  __shared__ u32 buf[kRunSortWarps][kRunSortMax];
-  const u32 lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const u64 warps = u64(gridDim.x) * kRunSortWarps;
-  for (u64 q = u64(blockIdx.x) * kRunSortWarps + w; q < nq; q += warps)
-  {
-    const u64 b = off[q];
-    const u32 len = u32(off[q + 1] - b);
-    if (len <= 1)
-      continue;
-    if (len > kRunSortMax)
+    run_sort_kernel<true><<<grid, kRunSortWarps * 32, 0, st>>>(off, nq, r.ids.as<u32>(), r.dist.as<double>(), longRuns.as<u32>(), u32(longCap));
+    if (m > kRunSortMax)
     {
-      if (lane == 0)
-        atomicAdd(longRuns, 1u);
-      continue;
+      if ((e = cudaFuncSetAttribute(run_sort_block_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kBlockRunMax * 12))))
+        return cuda_status(e, "configuring the run sort");
+      run_sort_block_kernel<true><<<longGrid, kBlockSortThreads, kBlockRunMax * 12, st>>>(off, r.ids.as<u32>(), r.dist.as<double>(), longRuns.as<u32>(),
+                                                                                        u32(longCap));
     }
-    if (len <= 32)
-    {
-      u32 v = lane < len ? ids[b + lane] : ~0u;
-#pragma unroll
-      for (u32 k = 2; k <= 32; k <<= 1)
-#pragma unroll
-        for (u32 j = k >> 1; j > 0; j >>= 1)
-        {
-          const u32 o = __shfl_xor_sync(~0u, v, j);
-          const bool up = (lane & k) == 0, lower = (lane & j) == 0;
-          v = (lower == up) ? min(v, o) : max(v, o);
-        }
-      if (lane < len)
-        ids[b + lane] = v;
-      continue;
-    }
-    u32 P = 64;
-    while (P < len)
-      P <<= 1;
-    u32* s = buf[w];
-    for (u32 i = lane; i < P; i += 32)
-      s[i] = i < len ? ids[b + i] : ~0u;
-    __syncwarp();
-    for (u32 k = 2; k <= P; k <<= 1)
-      for (u32 j = k >> 1; j > 0; j >>= 1)
-      {
-        for (u32 i = lane; i < P; i += 32)
-        {
-          const u32 x = i ^ j;
-          if (x > i)
-          {
-            const u32 a = s[i], c = s[x];
-            if ((a > c) == ((i & k) == 0))
-            {
-              s[i] = c;
-              s[x] = a;
-            }
-          }
-        }
-        __syncwarp();
-      }
-    for (u32 i = lane; i < len; i += 32)
-      ids[b + i] = s[i];
-    __syncwarp();
   }
+  else
+  {
+    run_sort_kernel<false><<<grid, kRunSortWarps * 32, 0, st>>>(off, nq, r.ids.as<u32>(), nullptr, longRuns.as<u32>(), u32(longCap));
+    if (m > kRunSortMax)
+      run_sort_block_kernel<false><<<longGrid, kBlockSortThreads, kBlockRunMax * 4, st>>>(off, r.ids.as<u32>(), nullptr, longRuns.as<u32>(), u32(longCap));
+  }
+  u32 tooLong = 0;
+  if ((e = cudaGetLastError()) || (e = cudaMemcpyAsync(&tooLong, longRuns.as<u32>() + 1, sizeof(u32), cudaMemcpyDeviceToHost, st)) ||
+      (e = cudaStreamSynchronize(st)))
+    return cuda_status(e, "finishing result");
+  done = tooLong == 0;
+  return OTG_OK;
 }
 
-// CSR result with ids ascending per query; ids are below idLimit
-static int finish_sorted_ids(Collected& c, u64 nq, ResultState& r, cudaStream_t st, u64 idLimit = u64(1) << 32)
+// The order of dense id results by bitmaps: one row of bits per query (a row of a forest's query is
+// as long as its tree), set by the items, counted per chunk, and written out ascending. Taken where
+// the rows are at most 16 bytes per item: below that density the counting order moves less.
+// Two ids of a query are never equal (a query takes each entity once), so no item is lost in a bit.
+static int order_by_bits(Collected& c, u64 nq, ResultState& r, const TreeState& t, const u32* qTree, cudaStream_t st, bool& done)
+{
+  const u64 m = c.m;
+  done = false;
+  u64 rowMax = t.n;
+  if (qTree)
+  {
+    rowMax = 0;
+    for (size_t i = 0; i + 1 < t.treeOffHost.size(); ++i)
+      rowMax = std::max<u64>(rowMax, t.treeOffHost[i + 1] - t.treeOffHost[i]);
+  }
+  const u64 rowChunks = (rowMax + kBitChunk - 1) / kBitChunk;
+  if (rowChunks == 0 || nq > (u64(1) << 31) / rowChunks || nq * rowChunks * (kBitChunk / 8) > 16 * m)
+    return OTG_OK;
+  const u64 chunks = nq * rowChunks; // a bound for a forest
+  TmpBuf bits, cnt, off, sums, base, qcnt, qsums;
+  const u64 tiles = (chunks + kScanTile - 1) / kScanTile, qtiles = (nq + kScanTile - 1) / kScanTile;
+  cudaError_t e;
+  if ((e = bits.ensure(chunks * (kBitChunk / 8), st)) || (e = cnt.ensure(sizeof(u32) * chunks, st)) || (e = off.ensure(sizeof(u64) * (chunks + 1), st)) ||
+      (e = sums.ensure(sizeof(u64) * (tiles + 1), st)))
+    return cuda_status(e, "allocating the result bitmaps");
+  const u64* rowBase = nullptr;
+  if (qTree)
+  {
+    if ((e = base.ensure(sizeof(u64) * (nq + 1), st)) || (e = qcnt.ensure(sizeof(u32) * nq, st)) || (e = qsums.ensure(sizeof(u64) * (qtiles + 1), st)))
+      return cuda_status(e, "allocating the result bitmaps");
+    bit_rows_kernel<<<blocks_for(nq), 256, 0, st>>>(qTree, t.treeOff.as<u64>(), nq, qcnt.as<u32>());
+    scan_reduce_kernel<<<u32(qtiles), kScanThreads, 0, st>>>(qcnt.as<u32>(), nq, qsums.as<u64>());
+    scan_tiles_kernel<<<1, kScanThreads, 0, st>>>(qsums.as<u64>(), qtiles);
+    scan_apply_kernel<<<u32(qtiles), kScanThreads, 0, st>>>(qcnt.as<u32>(), nq, qsums.as<u64>(), base.as<u64>());
+    rowBase = base.as<u64>();
+    bit_clear_kernel<<<blocks_for(chunks * 64), 256, 0, st>>>(bits.as<uint4>(), rowBase + nq);
+  }
+  else
+    cudaMemsetAsync(bits.p, 0, chunks * (kBitChunk / 8), st);
+  bit_mark_kernel<<<blocks_for(m), 256, 0, st>>>(c.items.as<u64>(), m, rowBase, u32(rowChunks), bits.as<u32>());
+  bit_count_kernel<<<blocks_for(chunks * 32), 256, 0, st>>>(bits.as<uint4>(), chunks, rowBase ? rowBase + nq : nullptr, cnt.as<u32>());
+  scan_reduce_kernel<<<u32(tiles), kScanThreads, 0, st>>>(cnt.as<u32>(), chunks, sums.as<u64>());
+  scan_tiles_kernel<<<1, kScanThreads, 0, st>>>(sums.as<u64>(), tiles);
+  scan_apply_kernel<<<u32(tiles), kScanThreads, 0, st>>>(cnt.as<u32>(), chunks, sums.as<u64>(), off.as<u64>());
+  bit_write_kernel<<<blocks_for(chunks * 32), 256, 0, st>>>(bits.as<u32>(), off.as<u64>(), chunks, rowBase, nq, u32(rowChunks), r.offsets.as<u64>(),
+                                                            r.ids.as<u32>(), m);
+  e = cudaStreamSynchronize(st);
+  if (e || (e = cudaGetLastError()))
+    return cuda_status(e, "finishing result");
+  done = true;
+  return OTG_OK;
+}
+
+// CSR result with ids ascending per query (qTree: the trees of a forest's queries)
+static int finish_sorted_ids(Collected& c, u64 nq, ResultState& r, cudaStream_t st, const TreeState& t, const u32* qTree)
 {
   const u64 m = c.m;
   r.nq = nq;
@@ -1246,37 +1260,20 @@ static int finish_sorted_ids(Collected& c, u64 nq, ResultState& r, cudaStream_t 
     return cuda_status(e, "allocating result");
   if (m == 0)
     return cuda_status(cudaMemsetAsync(r.offsets.p, 0, sizeof(u64) * (nq + 1), st), "result offsets");
-  // runs longer than kRunSortMax on average certainly include long ones: straight to the radix sort
-  // (counting them would also put every item's atomic on a few counters)
-  if (m < (u64(1) << 32) && nq < (u64(1) << 31) && m <= u64(kRunSortMax) * nq)
-  {
-    // counting order: counts and slots, offsets, ids into their runs, each run sorted by a warp
-    TmpBuf cnt, slot, tileSums, longRuns;
-    const u64 tiles = (nq + kScanTile - 1) / kScanTile;
-    if ((e = cnt.ensure(sizeof(u32) * nq, st)) || (e = slot.ensure(sizeof(u32) * m, st)) || (e = tileSums.ensure(sizeof(u64) * (tiles + 1), st)) ||
-        (e = longRuns.ensure(sizeof(u32), st)))
-      return cuda_status(e, "allocating the result order");
-    cudaMemsetAsync(cnt.p, 0, sizeof(u32) * nq, st);
-    cudaMemsetAsync(longRuns.p, 0, sizeof(u32), st);
-    query_slots_kernel<<<blocks_for(m), 256, 0, st>>>(c.items.as<u64>(), m, cnt.as<u32>(), slot.as<u32>());
-    scan_reduce_kernel<<<u32(tiles), kScanThreads, 0, st>>>(cnt.as<u32>(), nq, tileSums.as<u64>());
-    scan_tiles_kernel<<<1, kScanThreads, 0, st>>>(tileSums.as<u64>(), tiles);
-    scan_apply_kernel<<<u32(tiles), kScanThreads, 0, st>>>(cnt.as<u32>(), nq, tileSums.as<u64>(), r.offsets.as<u64>());
-    query_scatter_kernel<<<blocks_for(m), 256, 0, st>>>(c.items.as<u64>(), slot.as<u32>(), m, r.offsets.as<u64>(), r.ids.as<u32>());
-    run_sort_kernel<<<u32(std::min<u64>((nq + kRunSortWarps - 1) / kRunSortWarps, 152 * 8)), kRunSortWarps * 32, 0, st>>>(r.offsets.as<u64>(), nq,
-                                                                                                                          r.ids.as<u32>(), longRuns.as<u32>());
-    u32 hl = 0;
-    if ((e = cudaGetLastError()) || (e = cudaMemcpyAsync(&hl, longRuns.p, sizeof(u32), cudaMemcpyDeviceToHost, st)) || (e = cudaStreamSynchronize(st)))
-      return cuda_status(e, "finishing result");
-    if (hl == 0)
-      return OTG_OK;
-    // some query holds more than kRunSortMax ids: the whole result by radix sort instead (the items
-    // are unchanged)
-  }
+  bool done = false;
+  // short runs sort faster in a warp than a row of bits is swept: bitmaps from 1024 ids per query on
+  if (m >= u64(kRunSortMax) * nq)
+    if (int rc = order_by_bits(c, nq, r, t, qTree, st, done))
+      return rc;
+  if (!done)
+    if (int rc = order_by_runs(c, nq, r, false, st, done))
+      return rc;
+  if (done)
+    return OTG_OK;
   TmpBuf vals, qid;
   if ((e = vals.ensure(sizeof(u32) * m, st)) || (e = qid.ensure(sizeof(u32) * m, st)))
     return cuda_status(e, "allocating sort values");
-  const u32 idBits = std::min<u32>(32, std::max<u32>(1, bit_count(std::max<u64>(idLimit, 1) - 1)));
+  const u32 idBits = std::min<u32>(32, std::max<u32>(1, bit_count(std::max<u64>(t.n, 1) - 1)));
   if (idBits < 32)
     pack_items_kernel<<<blocks_for(m), 256, 0, st>>>(c.items.as<u64>(), m, idBits);
   if (int rc = sort_pairs_u64(c.items.as<u64>(), vals.as<u32>(), m, idBits + bit_count(nq), st, c.errp()))
@@ -1287,7 +1284,8 @@ static int finish_sorted_ids(Collected& c, u64 nq, ResultState& r, cudaStream_t 
   return cuda_status(e ? e : cudaGetLastError(), "finishing result");
 }
 
-// CSR result ordered by (query, distance, id): three stable radix sorts (id, distance, query)
+// CSR result ordered by (query, distance, id): by runs, or with three stable radix sorts (id, distance,
+// query) where a run is too long for a block's shared memory
 static int finish_by_distance(Collected& c, u64 nq, u64 nEntities, ResultState& r, cudaStream_t st)
 {
   const u64 m = c.m;
@@ -1299,6 +1297,11 @@ static int finish_by_distance(Collected& c, u64 nq, u64 nEntities, ResultState& 
     return cuda_status(e, "allocating result");
   if (m == 0)
     return cuda_status(cudaMemsetAsync(r.offsets.p, 0, sizeof(u64) * (nq + 1), st), "result offsets");
+  bool done = false;
+  if (int rc = order_by_runs(c, nq, r, true, st, done))
+    return rc;
+  if (done)
+    return OTG_OK;
   TmpBuf perm, k32, k64;
   if ((e = perm.ensure(sizeof(u32) * m, st)) || (e = k32.ensure(sizeof(u32) * m, st)) || (e = k64.ensure(sizeof(u64) * m, st)))
     return cuda_status(e, "allocating sort buffers");
@@ -1437,7 +1440,7 @@ static int range_impl(const TreeState& t, const void* ranges, u64 nq, int mode, 
     return cuda_status(e, "allocating the work counter");
   int launchRc = OTG_OK;
   int rc = collect(
-    c, false, nq * 32,
+    c, false, nq * 32, nq * t.n,
     [&](Appender a, u32* err) {
       if (algo == OTG_ALGO_PLAIN_FP64)
         range_plain_kernel<T><<<u32((nq + 127) / 128), 128, 0, st>>>(tv, (const T*)d, u32(nq), mode, tl, a, err);
@@ -1460,7 +1463,7 @@ static int range_impl(const TreeState& t, const void* ranges, u64 nq, int mode, 
     return rc;
   r.filterTests = c.tests; // the FP32 pre-tests of the batched kernel and the ones left to FP64
   r.rechecks = c.rechecks;
-  return finish_sorted_ids(c, nq, r, st, t.n);
+  return finish_sorted_ids(c, nq, r, st, t, qTree);
 }
 
 template<typename T>
@@ -1480,7 +1483,7 @@ static int pick_impl(const TreeState& t, const void* pts, u64 nq, double tol, in
     return cuda_status(e, "allocating the work counter");
   int launchRc = OTG_OK;
   int rc = collect(
-    c, false, nq * 8,
+    c, false, nq * 8, nq * t.n,
     [&](Appender a, u32* err) {
       if (algo == OTG_ALGO_PLAIN_FP64)
         pick_plain_kernel<T><<<u32((nq + 127) / 128), 128, 0, st>>>(tv, (const T*)d, u32(nq), tl, a, err);
@@ -1501,7 +1504,7 @@ static int pick_impl(const TreeState& t, const void* pts, u64 nq, double tol, in
     return launchRc;
   if (rc)
     return rc;
-  return finish_sorted_ids(c, nq, r, st, t.n);
+  return finish_sorted_ids(c, nq, r, st, t, qTree);
 }
 
 template<typename T>
@@ -1522,7 +1525,7 @@ static int frustum_impl(const TreeState& t, const void* planes, u64 np, u64 nq, 
     return cuda_status(e, "allocating the work counter");
   int launchRc = OTG_OK;
   int rc = collect(
-    c, false, std::max<u64>(nq * 64, t.n / 4),
+    c, false, std::max<u64>(nq * 64, t.n / 4), nq * t.n,
     [&](Appender a, u32* err) {
       if (algo == OTG_ALGO_PLAIN_FP64)
         frustum_plain_kernel<T><<<u32((nq + 127) / 128), 128, 0, st>>>(tv, (const T*)d, u32(np), u32(nq), tl, a, err);
@@ -1543,7 +1546,7 @@ static int frustum_impl(const TreeState& t, const void* planes, u64 np, u64 nq, 
     return launchRc;
   if (rc)
     return rc;
-  return finish_sorted_ids(c, nq, r, st, t.n);
+  return finish_sorted_ids(c, nq, r, st, t, qTree);
 }
 
 template<typename T>
@@ -1564,7 +1567,7 @@ static int plane_impl(const TreeState& t, const void* planes, u64 nq, bool posit
     return cuda_status(e, "allocating the work counter");
   int launchRc = OTG_OK;
   int rc = collect(
-    c, false, std::max<u64>(nq * 64, positive ? t.n : t.n / 16),
+    c, false, std::max<u64>(nq * 64, positive ? t.n : t.n / 16), nq * t.n,
     [&](Appender a, u32* err) {
       if (algo == OTG_ALGO_PLAIN_FP64)
         plane_plain_kernel<T><<<u32((nq + 127) / 128), 128, 0, st>>>(tv, (const T*)d, u32(nq), positive ? 1 : 0, tl, a, err);
@@ -1586,7 +1589,7 @@ static int plane_impl(const TreeState& t, const void* planes, u64 nq, bool posit
     return launchRc;
   if (rc)
     return rc;
-  return finish_sorted_ids(c, nq, r, st, t.n);
+  return finish_sorted_ids(c, nq, r, st, t, qTree);
 }
 
 // conditions given in host memory are checked here; device conditions are checked by the kernels
@@ -1659,7 +1662,7 @@ static int query_impl(const TreeState& t, const QueryCond* conds, const u64* off
     return cuda_status(e, "allocating the work counter");
   int launchRc = OTG_OK;
   int rc = collect(
-    c, false, std::max<u64>(nq * 64, t.n / 4),
+    c, false, std::max<u64>(nq * 64, t.n / 4), nq * t.n,
     [&](Appender a, u32* err) {
       if (algo == OTG_ALGO_PLAIN_FP64)
         query_plain_kernel<T><<<u32((nq + 127) / 128), 128, 0, st>>>(tv, qp, u32(nq), tl, a, err);
@@ -1681,7 +1684,7 @@ static int query_impl(const TreeState& t, const QueryCond* conds, const u64* off
     return launchRc;
   if (rc)
     return rc;
-  return finish_sorted_ids(c, nq, r, st, t.n);
+  return finish_sorted_ids(c, nq, r, st, t, nullptr);
 }
 
 template<typename T>
@@ -1720,7 +1723,7 @@ static int knn_impl(const TreeState& t, const void* pts, u64 nq, const u32* k, u
   const int bucket = knn_heap_bucket(kMax);
   Collected c;
   int rc = collect(
-    c, true, nq * 16,
+    c, true, nq * 16, nq * t.n,
     [&](Appender a, u32* err) {
       launch_knn_threshold<T>(bucket, u32((nq + 127) / 128), st, tv, (const T*)d, u32(nq), (const u32*)dk, kAll, F0, tl, F.as<T>(), err);
       knn_collect_kernel<T><<<u32((nq + 127) / 128), 128, 0, st>>>(tv, (const T*)d, u32(nq), F.as<T>(), tl, a, err);
@@ -1754,7 +1757,7 @@ static int ray_impl(const TreeState& t, const void* rays, u64 nq, double tol, do
       return cuda_status(e, "allocating the work counter");
     int launchRc = OTG_OK;
     rc = collect(
-      c, true, nq * 16,
+      c, true, nq * 16, nq * t.n,
       [&](Appender a, u32* err) {
         if (algo == OTG_ALGO_PLAIN_FP64)
           ray_all_plain_kernel<T><<<u32((nq + 127) / 128), 128, 0, st>>>(tv, (const T*)d, u32(nq), tl, ti, md, a, err);
@@ -1779,7 +1782,7 @@ static int ray_impl(const TreeState& t, const void* rays, u64 nq, double tol, do
     if (cudaError_t e = M.ensure(sizeof(T) * nq, st))
       return cuda_status(e, "allocating ray thresholds");
     rc = collect(
-      c, true, nq * 4,
+      c, true, nq * 4, nq * t.n,
       [&](Appender a, u32* err) {
         ray_first_threshold_kernel<T><<<u32((nq + 127) / 128), 128, 0, st>>>(tv, (const T*)d, u32(nq), tl, ti, md, M.as<T>(), err);
         ray_first_collect_kernel<T><<<u32((nq + 127) / 128), 128, 0, st>>>(tv, (const T*)d, u32(nq), tl, ti, M.as<T>(), a, err);
@@ -1817,7 +1820,7 @@ static int collide_impl(const TreeState& a, const TreeState& b, bool self, doubl
   CollideSearch search;
   int searchRc = OTG_OK;
   int rc = collect(
-    c, false, a.n * 4,
+    c, false, a.n * 4, 0,
     [&](Appender ap, u32* err) {
       if (filtered)
         searchRc = collide_search_filtered(const_cast<TreeState&>(a), const_cast<TreeState&>(b), self, tol, ap, err, search, st);
