@@ -17,6 +17,7 @@
 //   Query<And / Or>     core/ot_query.h:864-1026
 //   PickSearch          core/ot_query.h:425-466
 #include "otg_query.cuh"
+#include "otg_ray.cuh"
 
 namespace otg
 {
@@ -252,9 +253,13 @@ struct BatchArgs
   u32 splitCap;       // item capacity of the work buffer
   u32 splitDepth;     // depth of the subtrees that become items
   // range on FP64 point trees: one RangeQ per query (FP32 pre-tests); set only where out.count has
-  // three slots (the item count, then the pre-tests and the undecided ones, added at the end)
+  // three slots (the item count, then the pre-tests and the undecided ones, added at the end).
+  // Rays on FP64 box trees with FP32 images: one RayPrep per query.
   const void* prep = nullptr;
+  float tolUp = 0.f, tolIncUp = 0.f; // tol and tolInc rounded up (rays)
 };
+
+constexpr u32 kCandBuf = 64;
 
 template<typename T, int KIND, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32) batch_query_kernel(BatchArgs<T, KIND> a)
@@ -262,6 +267,9 @@ __global__ void __launch_bounds__(WARPS * 32) batch_query_kernel(BatchArgs<T, KI
   static_assert(KIND >= kRange && KIND <= kPick, "every query kind has its own setup, node test and entity test below");
   using G = GeoD<T>;
   constexpr bool kRangeF32 = KIND == kRange && sizeof(T) == 8;
+  constexpr bool kRayPre = KIND == kRayAll && sizeof(T) == 8;
+  __shared__ RayF32 rayF[kRayPre ? WARPS : 1];
+  __shared__ u32 candMem[kRayPre ? WARPS : 1][kRayPre ? kCandBuf : 1];
   __shared__ RangeF32 rangeF[kRangeF32 ? WARPS : 1];
   __shared__ u32 stackMem[WARPS][kWideStack];
   __shared__ u64 itemMem[WARPS][kItemBuf];
@@ -394,11 +402,51 @@ __global__ void __launch_bounds__(WARPS * 32) batch_query_kernel(BatchArgs<T, KI
     }
     else if constexpr (KIND == kRayAll)
     {
-      ray.make(a.q + u64(q) * 6, a.q + u64(q) * 6 + 3, a.tol, a.tolInc);
-      skip = !ray.valid;
+      bool made = false;
+      if constexpr (kRayPre)
+        if (a.prep)
+        {
+          const RayPrep* p = static_cast<const RayPrep*>(a.prep) + q;
+          const u32 flags = p->flags;
+          __syncwarp(); // the previous ray's setup is read by every lane before it changes
+          if (lane == 0)
+            ray_f32_of(*p, rayF[w]);
+          __syncwarp();
+          skip = !(flags & kRayValid);
+          useF32 = (flags & kRayF32) != 0;
+          made = true;
+        }
+      if (!made)
+      {
+        ray.make(a.q + u64(q) * 6, a.q + u64(q) * 6 + 3, a.tol, a.tolInc);
+        skip = !ray.valid;
+      }
     }
     if (skip)
       continue;
+    u32 nCand = 0; // entities of this ray that may be hit, not yet tested exactly
+    // the exact test of the last min(32, nCand) buffered entities, one per lane: candidates of many
+    // nodes fill the lanes (an FP64 instruction costs the same for one lane as for 32)
+    auto test_cands = [&]() {
+      if constexpr (kRayPre)
+      {
+        const u32 take = min(nCand, 32u);
+        nCand -= take;
+        bool hit = false;
+        double en = 0.0, ex = 0.0;
+        u32 id = 0;
+        if (lane < take)
+        {
+          const u32 e = candMem[w][nCand + lane];
+          hit = ray_box_exact(a.q + u64(q) * 6, static_cast<const RayPrep*>(a.prep) + q, tv.geom + u64(e) * 6, a.tol, a.tolInc, en, ex) &&
+                (a.maxDist == T(0) || en <= a.maxDist);
+          if (hit)
+            id = tv.ids[e] - idBase;
+        }
+        __syncwarp();
+        sink_put(sink, a.out, lane, hit, q, id, en);
+      }
+    };
     // ---- node test of one node (run by one lane per child)
     auto enters = [&](u32 node, bool& contained) -> bool {
       const T* nb = tv.nodeBox + u64(node) * 6;
@@ -462,6 +510,14 @@ __global__ void __launch_bounds__(WARPS * 32) batch_query_kernel(BatchArgs<T, KI
       else if constexpr (KIND == kRayAll)
       {
         T en, ex;
+        if constexpr (kRayPre)
+          if (a.prep)
+          {
+            const int rel = useF32 ? ray_box_f32(rayF[w], a.tolUp, a.tolIncUp, tv.nodeImg[2 * size_t(node)], tv.nodeImg[2 * size_t(node) + 1]).rel : 2;
+            if (rel != 2)
+              return rel == 1;
+            return ray_node_exact(a.q + u64(q) * 6, static_cast<const RayPrep*>(a.prep) + q, nb, a.tol, a.tolInc, en, ex);
+          }
         return ray.hit_node(nb, nb + 3, en, ex);
       }
     };
@@ -560,6 +616,19 @@ __global__ void __launch_bounds__(WARPS * 32) batch_query_kernel(BatchArgs<T, KI
           const u32 e = oy + (f - oex);
           bool hit = false;
           double d = 0.0;
+          if constexpr (kRayPre)
+            if (a.prep)
+            {
+              const bool may = v && (!useF32 || ray_box_f32(rayF[w], a.tolUp, a.tolIncUp, tv.boxImg[2 * size_t(e)], tv.boxImg[2 * size_t(e) + 1]).rel != 0);
+              const u32 bal = __ballot_sync(~0u, may);
+              if (may)
+                candMem[w][nCand + __popc(bal & ((1u << lane) - 1))] = e;
+              nCand += __popc(bal);
+              __syncwarp();
+              if (nCand >= 32)
+                test_cands();
+              continue;
+            }
           if (v)
           {
             if constexpr (KIND == kRange)
@@ -697,6 +766,9 @@ __global__ void __launch_bounds__(WARPS * 32) batch_query_kernel(BatchArgs<T, KI
       if (bad)
         break;
     }
+    if constexpr (kRayPre)
+      if (nCand)
+        test_cands();
     if (bad && lane == 0)
       atomicOr(a.err, kErrStack);
     sink_flush(sink, a.out, lane);
@@ -820,7 +892,23 @@ template<typename T>
 int batch_ray_all(const TreeView<T>& tv, const T* rays, u32 nq, T tol, T tolInc, T maxDist, Appender out, u32* work, u32* err, cudaStream_t st,
                   int shape, size_t workBytes)
 {
-  return launch_batch<T, kRayAll>(BatchArgs<T, kRayAll>{ tv, rays, 0, nq, 0, tol, tolInc, maxDist, out, work, err }, shape, st, workBytes);
+  BatchArgs<T, kRayAll> a{ tv, rays, 0, nq, 0, tol, tolInc, maxDist, out, work, err };
+  TmpBuf prep;
+  if constexpr (sizeof(T) == 8)
+  {
+    // FP64 box trees with FP32 images: the setup by one thread per ray, most tests in FP32
+    if (tv.nodeImg && tv.boxImg && tv.isBox && nq)
+    {
+      if (cudaError_t e = prep.ensure(sizeof(RayPrep) * nq, st))
+        return cuda_status(e, "allocating the ray setup");
+      if (int rc = ray_prepare(rays, nq, double(tol), double(tolInc), prep.as<RayPrep>(), st))
+        return rc;
+      a.prep = prep.p;
+      a.tolUp = float_ru_host(double(tol));
+      a.tolIncUp = float_ru_host(double(tolInc));
+    }
+  }
+  return launch_batch<T, kRayAll>(a, shape, st, workBytes);
 }
 
 template int batch_range<double>(const TreeView<double>&, const double*, u32, int, double, Appender, u32*, u32*, cudaStream_t, int, size_t);

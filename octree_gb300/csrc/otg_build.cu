@@ -1555,7 +1555,9 @@ int build_tree(TreeState& t, const void* entities, u64 n, u32 maxDepth, const vo
   t.maxElem = maxElem;
   t.built = false;
   t.countsKnown = false;
-  t.image32 = false;
+  t.image32 = t.boxImage32 = false;
+  t.imageTests = 0;
+  t.respanned = false;
   t.inserted = false;
   t.retired.clear();
   t.trees = 0;
@@ -2043,7 +2045,9 @@ int build_forest(TreeState& t, const void* entities, const u64* treeOffsets, u32
   t.maxElem = maxElem;
   t.built = false;
   t.countsKnown = false;
-  t.image32 = false;
+  t.image32 = t.boxImage32 = false;
+  t.imageTests = 0;
+  t.respanned = false;
   t.inserted = false;
   t.retired.clear();
   t.trees = trees;
@@ -2214,7 +2218,8 @@ int set_entities(TreeState& t, const void* entities, u64 n, int mem, cudaStream_
     else
       gather_kernel<float, 3, kGatherPerThread><<<blocks, 256, 0, st>>>((const float*)src, t.sortedIds.as<u32>(), n, t.sortedGeom.as<float>());
   }
-  t.image32 = false; // the FP32 filter images follow the geometry
+  t.image32 = t.boxImage32 = false; // the FP32 filter images follow the geometry
+  t.respanned = true;
   if ((e = cudaGetLastError()))
     return cuda_status(e, "gathering entities");
   if (mem == OTG_MEM_HOST && (e = cudaStreamSynchronize(st)))

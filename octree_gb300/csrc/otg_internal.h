@@ -21,6 +21,7 @@
 
 #include <cuda_runtime.h>
 #include <functional>
+#include <mutex>
 #include <string>
 #include <utility>
 #include <vector>
@@ -200,6 +201,8 @@ struct TreeState
       cudaEventDestroy(fork);
     if (join)
       cudaEventDestroy(join);
+    if (imageReady)
+      cudaEventDestroy(imageReady);
   }
 
   int scalar = OTG_SCALAR_F64;
@@ -247,7 +250,15 @@ struct TreeState
   DevBuf stOrder, stChildBegin, stSeg, stDepth, stGeom, stCtl;
   DevBuf geom32;     // FP32 image of sortedGeom for the query filters (built on first use)
   DevBuf nodeBox32;  // FP32 outward-rounded node boxes for the query filters
-  bool image32 = false;
+  DevBuf boxImg32;   // FP32 outward-rounded box entities (box trees; built when queries are worth it)
+  bool image32 = false, boxImage32 = false;
+  // Queries of one tree may run on several threads and streams: the images are built under the
+  // mutex, and every stream that uses them waits for the event recorded after their kernels.
+  std::mutex imageMutex;
+  cudaEvent_t imageReady = nullptr;
+  u64 imageTests = 0; // entity tests of the box queries since the build (use_box_images)
+  // set_entities changed the geometry: entities may lie outside their nodes
+  bool respanned = false;
   // a bulk Insert changed the tree: nodes may own entities beside their children and child links
   // may skip levels, which the static array layout cannot hold
   bool inserted = false;

@@ -705,21 +705,59 @@ static void host_bounds(double v, float& lo, float& hi)
     hi = std::nextafter(f, kInf);
 }
 
+// box entities rounded outward: {min rounded down, 0}, {max rounded up, 0}
 template<typename T>
-static int ensure_image32_impl(TreeState& t, cudaStream_t st)
+__global__ void entity_box_image_kernel(const T* __restrict__ geom, u64 n, float4* __restrict__ out)
 {
-  if (t.image32)
-    return OTG_OK;
+  for (u64 i = blockIdx.x * u64(blockDim.x) + threadIdx.x; i < n; i += u64(gridDim.x) * blockDim.x)
+  {
+    float v[6];
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+    {
+      v[c] = __double2float_rd(double(geom[i * 6 + c]));
+      v[3 + c] = __double2float_ru(double(geom[i * 6 + 3 + c]));
+    }
+    out[2 * i] = make_float4(v[0], v[1], v[2], 0.f);
+    out[2 * i + 1] = make_float4(v[3], v[4], v[5], 0.f);
+  }
+}
+
+template<typename T>
+static int ensure_image32_impl(TreeState& t, cudaStream_t st, bool boxes)
+{
+  const bool isBox = t.kind != OTG_KIND_POINTS;
+  boxes = boxes && isBox;
+  std::lock_guard<std::mutex> g(t.imageMutex);
   cudaError_t e;
-  if ((e = t.geom32.ensure(sizeof(float4) * std::max<u64>(t.n, 1))) || (e = t.nodeBox32.ensure(sizeof(float4) * 2 * std::max<u64>(t.nodeCount, 1))))
-    return cuda_status(e, "allocating the FP32 tree image");
-  if (t.kind == OTG_KIND_POINTS && t.n)
-    point_image_kernel<T><<<blocks_for(t.n), 256, 0, st>>>(t.sortedGeom.as<T>(), t.n, t.geom32.as<float4>());
-  node_image_kernel<T><<<blocks_for(t.nodeCount), 256, 0, st>>>(t.nodeBox.as<T>(), t.kind != OTG_KIND_POINTS ? t.nodeMax.as<T>() : nullptr, t.nodeCount,
-                                                                 t.nodeBox32.as<float4>());
-  if ((e = cudaGetLastError()))
+  const bool build = !t.image32 || (boxes && !t.boxImage32);
+  // the stream that builds orders itself after the streams that built or use the earlier images
+  if (t.imageReady && (e = cudaStreamWaitEvent(st, t.imageReady, 0)))
+    return cuda_status(e, "waiting for the FP32 tree image");
+  if (!build)
+    return OTG_OK;
+  if (!t.imageReady && (e = cudaEventCreateWithFlags(&t.imageReady, cudaEventDisableTiming)))
+    return cuda_status(e, "creating the image event");
+  if (!t.image32)
+  {
+    if ((!isBox && (e = t.geom32.ensure(sizeof(float4) * std::max<u64>(t.n, 1)))) || (e = t.nodeBox32.ensure(sizeof(float4) * 2 * std::max<u64>(t.nodeCount, 1))))
+      return cuda_status(e, "allocating the FP32 tree image");
+    if (!isBox && t.n)
+      point_image_kernel<T><<<blocks_for(t.n), 256, 0, st>>>(t.sortedGeom.as<T>(), t.n, t.geom32.as<float4>());
+    node_image_kernel<T><<<blocks_for(t.nodeCount), 256, 0, st>>>(t.nodeBox.as<T>(), isBox ? t.nodeMax.as<T>() : nullptr, t.nodeCount,
+                                                                   t.nodeBox32.as<float4>());
+  }
+  if (boxes && !t.boxImage32)
+  {
+    if ((e = t.boxImg32.ensure(sizeof(float4) * 2 * std::max<u64>(t.n, 1))))
+      return cuda_status(e, "allocating the FP32 box image");
+    if (t.n)
+      entity_box_image_kernel<T><<<blocks_for(t.n), 256, 0, st>>>(t.sortedGeom.as<T>(), t.n, t.boxImg32.as<float4>());
+  }
+  if ((e = cudaGetLastError()) || (e = cudaEventRecord(t.imageReady, st)))
     return cuda_status(e, "building the FP32 tree image");
   t.image32 = true;
+  t.boxImage32 = t.boxImage32 || boxes;
   return OTG_OK;
 }
 
@@ -910,9 +948,29 @@ static int knn_filtered_impl(TreeState& t, const T* pts, const u32* dk, u64 nq, 
   return OTG_OK;
 }
 
-int ensure_image32(TreeState& t, cudaStream_t st)
+int ensure_image32(TreeState& t, cudaStream_t st, bool boxes)
 {
-  return t.scalar == OTG_SCALAR_F64 ? ensure_image32_impl<double>(t, st) : ensure_image32_impl<float>(t, st);
+  return t.scalar == OTG_SCALAR_F64 ? ensure_image32_impl<double>(t, st, boxes) : ensure_image32_impl<float>(t, st, boxes);
+}
+
+int use_box_images(TreeState& t, TreeView<double>& tv, u64 tests, cudaStream_t st)
+{
+  if (t.kind == OTG_KIND_POINTS)
+    return OTG_OK;
+  {
+    // building the images moves 80 bytes of every entity and a test that they spare reads 48 and takes
+    // some 30 FP64 operations: worth it from about one test per entity on, so that a tree rebuilt for
+    // a few queries does not pay for them
+    std::lock_guard<std::mutex> g(t.imageMutex);
+    t.imageTests += tests;
+    if (!t.boxImage32 && t.imageTests < t.n)
+      return OTG_OK;
+  }
+  if (int rc = ensure_image32(t, st, true))
+    return rc;
+  tv.nodeImg = t.nodeBox32.as<float4>();
+  tv.boxImg = t.boxImg32.as<float4>();
+  return OTG_OK;
 }
 
 int knn_filtered(TreeState& t, const void* dpts, const u32* dk, u64 nq, u32 kAll, double maxDist, double tol, ResultState& r, cudaStream_t st)

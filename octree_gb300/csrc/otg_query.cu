@@ -19,6 +19,7 @@
 // (distance, id) for kNN and rays, or (i, j) pairs ascending for collisions.
 #include "otg_query.cuh"
 #include "otg_order.cuh"
+#include "otg_ray.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -1750,6 +1751,10 @@ static int ray_impl(const TreeState& t, const void* rays, u64 nq, double tol, do
   T md = maxDist < 0 ? Lim<T>::max() : T(maxDist);
   Collected c;
   int rc;
+  if constexpr (sizeof(T) == 8)
+    if (algo != OTG_ALGO_PLAIN_FP64)
+      if (int rci = use_box_images(const_cast<TreeState&>(t), tv, nq * 256, st))
+        return rci;
   if (!first)
   {
     TmpBuf work;
@@ -1779,15 +1784,30 @@ static int ray_impl(const TreeState& t, const void* rays, u64 nq, double tol, do
   }
   else
   {
-    if (cudaError_t e = M.ensure(sizeof(T) * nq, st))
-      return cuda_status(e, "allocating ray thresholds");
+    TmpBuf work;
+    if (algo == OTG_ALGO_PLAIN_FP64)
+    {
+      if (cudaError_t e = M.ensure(sizeof(T) * nq, st))
+        return cuda_status(e, "allocating ray thresholds");
+    }
+    else if (cudaError_t e = work.ensure(ray_first_work_bytes(nq), st))
+      return cuda_status(e, "allocating the ray list");
+    int launchRc = OTG_OK;
     rc = collect(
       c, true, nq * 4, nq * t.n,
       [&](Appender a, u32* err) {
+        if (algo != OTG_ALGO_PLAIN_FP64)
+        {
+          // entities outside their nodes (set_entities) are found in the walk's own order only
+          launchRc = ray_first<T>(tv, tv.isBox && !t.respanned, (const T*)d, u32(nq), tl, ti, md, a, work.as<u32>(), err, st);
+          return;
+        }
         ray_first_threshold_kernel<T><<<u32((nq + 127) / 128), 128, 0, st>>>(tv, (const T*)d, u32(nq), tl, ti, md, M.as<T>(), err);
         ray_first_collect_kernel<T><<<u32((nq + 127) / 128), 128, 0, st>>>(tv, (const T*)d, u32(nq), tl, ti, M.as<T>(), a, err);
       },
       st);
+    if (launchRc)
+      return launchRc;
   }
   if (rc)
     return rc;

@@ -31,6 +31,7 @@ struct TreeView
   // float4 per node) and round-to-nearest entities; null where a kernel takes the FP64 tests only
   const float4* nodeImg = nullptr;
   const float4* pointImg = nullptr;
+  const float4* boxImg = nullptr; // box trees: {min rounded down}, {max rounded up} (two float4 per entity)
 };
 
 // root node and id base of query q (node t is the root of tree t in a forest)
@@ -364,8 +365,12 @@ inline std::string query_key(const char* op, int algo, bool forest, bool f64, in
   return tune_key(name.c_str(), f64, kind, n, nq);
 }
 
-// FP32 images of a built tree for the query filters (otg_knn.cu): built on first use after a build
-int ensure_image32(TreeState& t, cudaStream_t st);
+// FP32 images of a built tree for the query filters (otg_knn.cu): built on first use after a build.
+// boxes: the box entities' images too (DevBuf boxImg32), which only some queries read.
+int ensure_image32(TreeState& t, cudaStream_t st, bool boxes = false);
+// Sets tv's images for a query on an FP64 box tree when they are there, or when the tree's queries
+// since its build are worth building them: `tests` estimates the entity tests of this call.
+int use_box_images(TreeState& t, TreeView<double>& tv, u64 tests, cudaStream_t st);
 
 // filtered candidate search of CollisionDetection (otg_collide.cu)
 struct CollideSearch
