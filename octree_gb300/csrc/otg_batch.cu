@@ -236,6 +236,94 @@ __device__ __forceinline__ int range_point_f32(const float4 p, const RangeF32& f
   return anyOut ? 0 : (allIn ? 1 : 2);
 }
 
+// ---- FP32 tests of boxes and points against planes (frustum and plane kinds)
+// The exact test (GetBoxPlaneRelationAD, internal_geometry_module.h:254-280) compares the projections of
+// the box's farthest and nearest corner, smax and smin, with dist -+ tol. Here both are summed in FP32
+// over the box's corners (outward-rounded images of FP64 trees, the values themselves in FP32 trees).
+// With M_d the largest coordinate of the root box, E = 2^-19 (sum |n_d| M_d + |dist| + tol) is 32
+// units of roundoff of the largest sum possible, which covers the images, the products and sums here
+// (under 12 units) and the exact test's own rounding, in FP32 trees too (under 10). Each plane keeps
+// the four thresholds
+//   smax < a: certainly negative   smax > b: certainly not   smin > c: certainly positive   smin < d: certainly not
+// and what they leave undecided takes the exact test. Values outside the FP32 range make E infinite or
+// NaN, which decides nothing.
+// A node certainly positive for every plane of a frustum holds only entities that pass (they lie in the
+// node, and E also spans their own tests' rounding): its subtree is taken untested. 64 frusta, 64
+// planes and 8 half-spaces on 1M FP64 boxes: kernels 4.27 ms with exact tests, every entity of a frustum
+// tested and contained runs copied one by one, 0.35 ms now.
+struct PlaneF32
+{
+  float n[3], a, b, c, d, pad;
+};
+constexpr u32 kMaxPlanes = 8; // planes per query that the FP32 tests take
+
+__device__ __forceinline__ void plane_f32(const PlaneF32& p, const float lo[3], const float hi[3], float& smin, float& smax)
+{
+  smin = smax = 0.f;
+#pragma unroll
+  for (int d = 0; d < 3; ++d)
+  {
+    const float x = p.n[d] * lo[d], y = p.n[d] * hi[d];
+    smin += fminf(x, y);
+    smax += fmaxf(x, y);
+  }
+}
+
+// planes {dist, n} of one query, lanes 0 .. np - 1 (np <= kMaxPlanes); rootBox: {min, size}
+template<typename T>
+__device__ __forceinline__ void plane_thresholds(const T* pl, u32 np, const T* rootBox, T tol, u32 lane, PlaneF32* out)
+{
+  if (lane < np)
+  {
+    PlaneF32 p;
+    const float d = float(pl[4 * lane]), t = float(tol);
+    float e = fabsf(d) + fabsf(t);
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+    {
+      p.n[c] = float(pl[4 * lane + 1 + c]);
+      const float lo = float(rootBox[c]), hi = float(T(rootBox[c] + rootBox[3 + c]));
+      e += fabsf(p.n[c]) * fmaxf(fabsf(lo), fabsf(hi));
+    }
+    e = e * 0x1p-19f + 0x1p-120f;
+    p.a = (d - t) - e;
+    p.b = (d - t) + e;
+    p.c = (d + t) + e;
+    p.d = (d + t) - e;
+    p.pad = 0.f;
+    out[lane] = p;
+  }
+}
+
+// the exact tests of undecided nodes and entities, out of line (see range_node_enters_fp64)
+template<typename T>
+__device__ __noinline__ bool frustum_node_exact(const T* nb, const T* pl, u32 np, T tol)
+{
+  for (u32 i = 0; i < np; ++i) // :779-795 first Hit selects, first Negative prunes
+  {
+    const int rel = GeoD<T>::box_plane(nb, nb + 3, pl[4 * i], pl + 4 * i + 1, tol);
+    if (rel == 1)
+      return true;
+    if (rel == 0)
+      return false;
+  }
+  return true;
+}
+// GetEntityPlaneRelation (ot_query.h:586-602) of a point or box
+template<typename T>
+__device__ __noinline__ int entity_plane_exact(const T* g, int isBox, const T* pl, T tol)
+{
+  if (!isBox)
+    return GeoD<T>::point_plane(g, pl[0], pl + 1, tol);
+  T bsize[3] = { T(g[3] - g[0]), T(g[4] - g[1]), T(g[5] - g[2]) };
+  return GeoD<T>::box_plane(g, bsize, pl[0], pl + 1, tol);
+}
+template<typename T>
+__device__ __noinline__ int node_plane_exact(const T* nb, const T* pl, T tol)
+{
+  return GeoD<T>::box_plane(nb, nb + 3, pl[0], pl + 1, tol);
+}
+
 template<typename T, int KIND>
 struct BatchArgs
 {
@@ -257,6 +345,7 @@ struct BatchArgs
   // Rays on FP64 box trees with FP32 images: one RayPrep per query.
   const void* prep = nullptr;
   float tolUp = 0.f, tolIncUp = 0.f; // tol and tolInc rounded up (rays)
+  bool planeF32 = false;             // FP32 plane tests: images (FP64 trees), entities in their nodes
 };
 
 constexpr u32 kCandBuf = 64;
@@ -268,6 +357,10 @@ __global__ void __launch_bounds__(WARPS * 32) batch_query_kernel(BatchArgs<T, KI
   using G = GeoD<T>;
   constexpr bool kRangeF32 = KIND == kRange && sizeof(T) == 8;
   constexpr bool kRayPre = KIND == kRayAll && sizeof(T) == 8;
+  constexpr bool kPlanes = KIND == kFrustum || KIND == kPlane || KIND == kPlanePositive;
+  // kinds that take whole subtrees untested
+  constexpr bool kWhole = KIND == kRange || KIND == kPlanePositive || KIND == kFrustum;
+  __shared__ PlaneF32 planeF[kPlanes ? WARPS : 1][kPlanes ? kMaxPlanes : 1];
   __shared__ RayF32 rayF[kRayPre ? WARPS : 1];
   __shared__ u32 candMem[kRayPre ? WARPS : 1][kRayPre ? kCandBuf : 1];
   __shared__ RangeF32 rangeF[kRangeF32 ? WARPS : 1];
@@ -424,6 +517,42 @@ __global__ void __launch_bounds__(WARPS * 32) batch_query_kernel(BatchArgs<T, KI
     }
     if (skip)
       continue;
+    bool planeTests = false;
+    if constexpr (kPlanes)
+      if (a.planeF32 && a.np <= kMaxPlanes)
+      {
+        planeTests = true;
+        __syncwarp(); // the previous query's planes are read by every lane before they change
+        plane_thresholds<T>(pl, a.np, tv.nodeBox + u64(root) * 6, a.tol, lane, planeF[w]);
+        __syncwarp();
+      }
+    // the FP32 corners of a node or entity for the plane tests
+    auto corners = [&](bool isNode, u32 i, float lo[3], float hi[3]) {
+      if constexpr (sizeof(T) == 8)
+      {
+        if (!isNode && !tv.isBox)
+        {
+          const float4 p = tv.pointImg[i];
+          lo[0] = hi[0] = p.x, lo[1] = hi[1] = p.y, lo[2] = hi[2] = p.z;
+          return;
+        }
+        const float4* img = isNode ? tv.nodeImg : tv.boxImg;
+        const float4 x = img[2 * size_t(i)], y = img[2 * size_t(i) + 1];
+        lo[0] = x.x, lo[1] = x.y, lo[2] = x.z;
+        hi[0] = y.x, hi[1] = y.y, hi[2] = y.z;
+      }
+      else
+      {
+        const bool point = !isNode && !tv.isBox;
+        const T* g = isNode ? tv.nodeBox + u64(i) * 6 : tv.geom + u64(i) * (point ? 3 : 6);
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+        {
+          lo[c] = g[c];
+          hi[c] = point ? g[c] : (isNode ? g[c] + g[3 + c] : g[3 + c]);
+        }
+      }
+    };
     u32 nCand = 0; // entities of this ray that may be hit, not yet tested exactly
     // the exact test of the last min(32, nCand) buffered entities, one per lane: candidates of many
     // nodes fill the lanes (an FP64 instruction costs the same for one lane as for 32)
@@ -483,24 +612,39 @@ __global__ void __launch_bounds__(WARPS * 32) batch_query_kernel(BatchArgs<T, KI
         contained = G::range_contains_min_size(r, nmin, nsize, a.tol);
         return true;
       }
-      else if constexpr (KIND == kFrustum)
+      else if constexpr (kPlanes)
       {
-        for (u32 i = 0; i < a.np; ++i) // :779-795 first Hit selects, first Negative prunes
+        const u32 np = KIND == kFrustum ? a.np : 1u;
+        if (planeTests)
         {
-          const int rel = G::box_plane(nb, nb + 3, pl[4 * i], pl + 4 * i + 1, a.tol);
-          if (rel == 1)
-            return true;
-          if (rel == 0)
-            return false;
+          float lo[3], hi[3];
+          corners(true, node, lo, hi);
+          bool decided = true, positive = true;
+          for (u32 i = 0; i < np; ++i)
+          {
+            const PlaneF32& p = planeF[w][i];
+            float smin, smax;
+            plane_f32(p, lo, hi, smin, smax);
+            if (smax < p.a)
+              return false; // (of a frustum: the planes before this one are positive)
+            if (smin > p.c)
+              continue;
+            positive = false;
+            decided = (smax > p.b) & (smin < p.d); // certainly hit
+            break;
+          }
+          if (decided)
+          {
+            contained = positive && KIND != kPlane;
+            return KIND == kPlane ? !positive : true; // :620-621 PlaneSearch enters only nodes the plane hits
+          }
         }
-        return true;
-      }
-      else if constexpr (KIND == kPlane)
-        return G::box_plane(nb, nb + 3, pl[0], pl + 1, a.tol) == 1; // :620-621 only nodes the plane hits
-      else if constexpr (KIND == kPlanePositive)
-      {
-        const int rel = G::box_plane(nb, nb + 3, pl[0], pl + 1, a.tol); // :702-710 negative prunes, positive takes the subtree
-        contained = rel == 2;
+        if constexpr (KIND == kFrustum)
+          return frustum_node_exact<T>(nb, pl, np, a.tol);
+        const int rel = node_plane_exact<T>(nb, pl, a.tol);
+        if (KIND == kPlane)
+          return rel == 1;
+        contained = rel == 2; // :702-710 negative prunes, positive takes the subtree
         return rel != 0;
       }
       else if constexpr (KIND == kQuery)
@@ -571,27 +715,64 @@ __global__ void __launch_bounds__(WARPS * 32) batch_query_kernel(BatchArgs<T, KI
         bad = true;
         break;
       }
-      bool whole = false;
-      if constexpr (KIND == kRange || KIND == kPlanePositive)
+      // Contained nodes: whole subtrees without entity tests (range :549-567, positive side :711-726); a
+      // subtree is one run of sortedIds. The runs of the popped nodes are copied together, with one
+      // reservation. In the first launch of a
+      // split batch a large one is left to its children, which become items: one warp copying half
+      // of a tree would be the last to end.
+      bool whole = false, expand = false;
+      if constexpr (kWhole)
       {
-        whole = act && (entry & kContained);
-        // whole subtrees without entity tests (range :549-567, positive side :711-726); a subtree is
-        // one run of sortedIds
-        u32 cm = __ballot_sync(~0u, whole);
-        if (cm)
-          sink_flush(sink, a.out, lane);
-        while (cm)
+        const bool cont = act && (entry & kContained);
+        if (__any_sync(~0u, cont))
         {
-          const int src = __ffs(int(cm)) - 1;
-          cm &= cm - 1;
-          const u32 y = __shfl_sync(~0u, L.y, src), len = __shfl_sync(~0u, L.w, src) - y;
+          if (cont && a.phase == 1 && (L.x >> kChildShift) != 0u && L.w - L.y > 1024u)
+          {
+            // only where the children hold the rest of the run: a run may also hold entities of no
+            // reachable node (locations outside the grid)
+            u32 held = L.z - L.y;
+            for (u32 c = 0; c < (L.x >> kChildShift); ++c)
+            {
+              const uint4 C = tv.link[(L.x & kFirstChildMask) + c];
+              held += C.w - C.y;
+            }
+            expand = held == L.w - L.y;
+          }
+          whole = cont;
+          const u32 len = cont ? (expand ? L.z : L.w) - L.y : 0u;
+          u32 incl = len;
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1)
+          {
+            const u32 y = __shfl_up_sync(~0u, incl, o);
+            if (lane >= u32(o))
+              incl += y;
+          }
+          const u32 total = __shfl_sync(~0u, incl, 31);
           unsigned long long base = 0;
-          if (lane == 0)
-            base = a.out.reserve(len);
+          if (lane == 0 && total)
+            base = a.out.reserve(total);
           base = __shfl_sync(~0u, base, 0);
-          for (u32 i = lane; i < len; i += 32)
-            if (base + i < a.out.capacity)
-              a.out.items[base + i] = (u64(q) << 32) | (tv.ids[y + i] - idBase);
+          const u64 room = base < a.out.capacity ? a.out.capacity - base : 0;
+          const u32 end = u32(min(u64(total), room));
+          const u32* __restrict__ src = tv.ids;
+          u64* __restrict__ dst = a.out.items + base;
+          for (u32 f0 = 0; f0 < end; f0 += 128)
+          {
+            u32 id[4];
+#pragma unroll
+            for (u32 k = 0; k < 4; ++k)
+            {
+              const u32 f = f0 + k * 32 + lane;
+              const u32 o = owner(incl, min(f, total - 1));
+              const u32 oy = __shfl_sync(~0u, L.y, o), oex = __shfl_sync(~0u, incl - len, o);
+              id[k] = f < end ? src[oy + (f - oex)] : 0u;
+            }
+#pragma unroll
+            for (u32 k = 0; k < 4; ++k)
+              if (f0 + k * 32 + lane < end)
+                dst[f0 + k * 32 + lane] = (u64(q) << 32) | (id[k] - idBase);
+          }
         }
       }
       const bool tests = act && !whole;
@@ -659,36 +840,46 @@ __global__ void __launch_bounds__(WARPS * 32) batch_query_kernel(BatchArgs<T, KI
                 hit = (a.mode == OTG_RANGE_OVERLAP) ? (G::box_relation(r, bx, a.tol) == -1) : G::contains_box_no_tol(r, bx);
               }
             }
-            else if constexpr (KIND == kFrustum)
+            else if constexpr (kPlanes)
             {
-              bool neg = false;
-              for (u32 i = 0; i < a.np && !neg; ++i)
+              const u32 np = KIND == kFrustum ? a.np : 1u;
+              const T* g = tv.geom + u64(e) * (tv.isBox ? 6 : 3);
+              bool decided = false;
+              if (planeTests)
               {
-                int rel;
-                if (tv.isBox)
+                float lo[3], hi[3];
+                corners(false, e, lo, hi);
+                bool neg = false, sure = true, cut = true;
+                for (u32 i = 0; i < np; ++i)
                 {
-                  const T* bx = tv.geom + u64(e) * 6;
-                  T bsize[3] = { T(bx[3] - bx[0]), T(bx[4] - bx[1]), T(bx[5] - bx[2]) };
-                  rel = G::box_plane(bx, bsize, pl[4 * i], pl + 4 * i + 1, a.tol);
+                  const PlaneF32& p = planeF[w][i];
+                  float smin, smax;
+                  plane_f32(p, lo, hi, smin, smax);
+                  neg |= smax < p.a;
+                  sure &= smax > p.b;
+                  if (KIND == kPlane)
+                  {
+                    cut = smin < p.d;
+                    neg |= smin > p.c; // not hit
+                  }
+                }
+                decided = neg | (sure & cut);
+                hit = !neg;
+              }
+              if (!decided)
+              {
+                if constexpr (KIND == kFrustum)
+                {
+                  hit = true;
+                  for (u32 i = 0; i < np && hit; ++i)
+                    hit = entity_plane_exact<T>(g, tv.isBox, pl + 4 * i, a.tol) != 0;
                 }
                 else
-                  rel = G::point_plane(tv.geom + u64(e) * 3, pl[4 * i], pl + 4 * i + 1, a.tol);
-                neg = rel == 0;
+                {
+                  const int rel = entity_plane_exact<T>(g, tv.isBox, pl, a.tol);
+                  hit = KIND == kPlane ? rel == 1 : rel != 0;
+                }
               }
-              hit = !neg;
-            }
-            else if constexpr (KIND == kPlane || KIND == kPlanePositive)
-            {
-              int rel; // ot_query.h:586-602 GetEntityPlaneRelation
-              if (tv.isBox)
-              {
-                const T* bx = tv.geom + u64(e) * 6;
-                T bsize[3] = { T(bx[3] - bx[0]), T(bx[4] - bx[1]), T(bx[5] - bx[2]) };
-                rel = G::box_plane(bx, bsize, pl[0], pl + 1, a.tol);
-              }
-              else
-                rel = G::point_plane(tv.geom + u64(e) * 3, pl[0], pl + 1, a.tol);
-              hit = KIND == kPlane ? rel == 1 : rel != 0;
             }
             else if constexpr (KIND == kQuery)
             {
@@ -710,7 +901,7 @@ __global__ void __launch_bounds__(WARPS * 32) batch_query_kernel(BatchArgs<T, KI
       }
       // children of the popped nodes, tested before they are pushed
       {
-        const u32 cnt = tests ? (L.x >> kChildShift) : 0u;
+        const u32 cnt = (tests || expand) ? (L.x >> kChildShift) : 0u;
         u32 incl = cnt;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1)
@@ -727,8 +918,15 @@ __global__ void __launch_bounds__(WARPS * 32) batch_query_kernel(BatchArgs<T, KI
           const u32 ofc = __shfl_sync(~0u, L.x & kFirstChildMask, o), oex = __shfl_sync(~0u, incl - cnt, o);
           bool keep = false, contained = false;
           const u32 child = ofc + (f - oex);
+          bool free = false; // a contained node's child
+          if constexpr (kWhole)
+            free = __shfl_sync(~0u, expand, o);
           if (f < total)
-            keep = enters(child, contained);
+          {
+            keep = contained = free;
+            if (!free)
+              keep = enters(child, contained);
+          }
           if (a.phase == 1)
           {
             // subtrees at the split depth become items for any warp
@@ -864,17 +1062,33 @@ int batch_range(const TreeView<T>& tv, const T* ranges, u32 nq, int mode, T tol,
   }
   return launch_batch<T, kRange>(a, shape, st, workBytes);
 }
+// whether the plane kinds test in FP32: FP64 trees need their images, and every entity lies in its node
+template<typename T>
+static bool plane_filter(const TreeView<T>& tv)
+{
+  if (sizeof(T) == 8)
+    return tv.inNodes && tv.nodeImg && (tv.isBox ? tv.boxImg : tv.pointImg);
+  return tv.inNodes;
+}
 template<typename T>
 int batch_frustum(const TreeView<T>& tv, const T* planes, u32 np, u32 nq, T tol, Appender out, u32* work, u32* err, cudaStream_t st, int shape, size_t workBytes)
 {
-  return launch_batch<T, kFrustum>(BatchArgs<T, kFrustum>{ tv, planes, np, nq, 0, tol, T(0), T(0), out, work, err }, shape, st, workBytes);
+  BatchArgs<T, kFrustum> a{ tv, planes, np, nq, 0, tol, T(0), T(0), out, work, err };
+  a.planeF32 = plane_filter(tv);
+  return launch_batch<T, kFrustum>(a, shape, st, workBytes);
 }
 template<typename T>
 int batch_plane(const TreeView<T>& tv, const T* planes, u32 nq, bool positive, T tol, Appender out, u32* work, u32* err, cudaStream_t st, int shape, size_t workBytes)
 {
   if (positive)
-    return launch_batch<T, kPlanePositive>(BatchArgs<T, kPlanePositive>{ tv, planes, 1, nq, 0, tol, T(0), T(0), out, work, err }, shape, st, workBytes);
-  return launch_batch<T, kPlane>(BatchArgs<T, kPlane>{ tv, planes, 1, nq, 0, tol, T(0), T(0), out, work, err }, shape, st, workBytes);
+  {
+    BatchArgs<T, kPlanePositive> a{ tv, planes, 1, nq, 0, tol, T(0), T(0), out, work, err };
+    a.planeF32 = plane_filter(tv);
+    return launch_batch<T, kPlanePositive>(a, shape, st, workBytes);
+  }
+  BatchArgs<T, kPlane> a{ tv, planes, 1, nq, 0, tol, T(0), T(0), out, work, err };
+  a.planeF32 = plane_filter(tv);
+  return launch_batch<T, kPlane>(a, shape, st, workBytes);
 }
 template<typename T>
 int batch_query_program(const TreeView<T>& tv, const QueryProgram<T>& qp, u32 nq, T tol, Appender out, u32* work, u32* err, cudaStream_t st, int shape, size_t workBytes)

@@ -953,23 +953,25 @@ int ensure_image32(TreeState& t, cudaStream_t st, bool boxes)
   return t.scalar == OTG_SCALAR_F64 ? ensure_image32_impl<double>(t, st, boxes) : ensure_image32_impl<float>(t, st, boxes);
 }
 
-int use_box_images(TreeState& t, TreeView<double>& tv, u64 tests, cudaStream_t st)
+int use_images(TreeState& t, TreeView<double>& tv, u64 tests, cudaStream_t st)
 {
-  if (t.kind == OTG_KIND_POINTS)
-    return OTG_OK;
+  const bool isBox = t.kind != OTG_KIND_POINTS;
   {
-    // building the images moves 80 bytes of every entity and a test that they spare reads 48 and takes
-    // some 30 FP64 operations: worth it from about one test per entity on, so that a tree rebuilt for
-    // a few queries does not pay for them
+    // building the images moves 80 bytes of every box (40 of a point) and a test that they spare reads 48
+    // and takes some 30 FP64 operations: worth it from about one test per entity on, so that a tree
+    // rebuilt for a few queries does not pay for them
     std::lock_guard<std::mutex> g(t.imageMutex);
     t.imageTests += tests;
-    if (!t.boxImage32 && t.imageTests < t.n)
+    if (!(isBox ? t.boxImage32 : t.image32) && t.imageTests < t.n)
       return OTG_OK;
   }
-  if (int rc = ensure_image32(t, st, true))
+  if (int rc = ensure_image32(t, st, isBox))
     return rc;
   tv.nodeImg = t.nodeBox32.as<float4>();
-  tv.boxImg = t.boxImg32.as<float4>();
+  if (isBox)
+    tv.boxImg = t.boxImg32.as<float4>();
+  else
+    tv.pointImg = t.geom32.as<float4>();
   return OTG_OK;
 }
 

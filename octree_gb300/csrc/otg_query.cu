@@ -1520,6 +1520,10 @@ static int frustum_impl(const TreeState& t, const void* planes, u64 np, u64 nq, 
     return empty_result(nq, r, false, st);
   Collected c;
   auto tv = view<T>(t, qTree);
+  if constexpr (sizeof(T) == 8)
+    if (algo != OTG_ALGO_PLAIN_FP64) // a view meets about a sixteenth of the entities
+      if (int rci = use_images(const_cast<TreeState&>(t), tv, nq * (t.n / 16 + 1), st))
+        return rci;
   T tl = tol_of<T>(tol);
   TmpBuf work;
   if (cudaError_t e = work.ensure(batch_work_bytes(nq), st))
@@ -1562,6 +1566,13 @@ static int plane_impl(const TreeState& t, const void* planes, u64 nq, bool posit
     return empty_result(nq, r, false, st);
   Collected c;
   auto tv = view<T>(t, qTree);
+  if constexpr (sizeof(T) == 8)
+    if (algo != OTG_ALGO_PLAIN_FP64)
+    {
+      const u64 edge = u64(std::cbrt(double(t.n))) + 1; // a plane meets a few layers of edge * edge entities
+      if (int rci = use_images(const_cast<TreeState&>(t), tv, nq * 4 * edge * edge, st))
+        return rci;
+    }
   T tl = tol_of<T>(tol);
   TmpBuf work;
   if (cudaError_t e = work.ensure(batch_work_bytes(nq), st))
@@ -1752,8 +1763,8 @@ static int ray_impl(const TreeState& t, const void* rays, u64 nq, double tol, do
   Collected c;
   int rc;
   if constexpr (sizeof(T) == 8)
-    if (algo != OTG_ALGO_PLAIN_FP64)
-      if (int rci = use_box_images(const_cast<TreeState&>(t), tv, nq * 256, st))
+    if (algo != OTG_ALGO_PLAIN_FP64 && tv.isBox)
+      if (int rci = use_images(const_cast<TreeState&>(t), tv, nq * 256, st))
         return rci;
   if (!first)
   {

@@ -31,6 +31,7 @@ struct TreeView
   // float4 per node) and round-to-nearest entities; null where a kernel takes the FP64 tests only
   const float4* nodeImg = nullptr;
   const float4* pointImg = nullptr;
+  bool inNodes = true; // every entity lies in its node's box (not after set_entities)
   const float4* boxImg = nullptr; // box trees: {min rounded down}, {max rounded up} (two float4 per entity)
 };
 
@@ -297,9 +298,11 @@ static inline int sort_pairs_u32(u32* keys, u32* vals, u64 m, u32 bits, cudaStre
 template<typename T>
 static inline TreeView<T> view(const TreeState& t, const u32* qTree = nullptr)
 {
-  return TreeView<T>{ t.nodeLink.as<uint4>(), t.nodeBox.as<T>(), t.nodeMax.as<T>(), t.sortedIds.as<u32>(), t.sortedGeom.as<T>(), u32(t.n),
+  TreeView<T> tv{ t.nodeLink.as<uint4>(), t.nodeBox.as<T>(), t.nodeMax.as<T>(), t.sortedIds.as<u32>(), t.sortedGeom.as<T>(), u32(t.n),
                       t.kind != OTG_KIND_POINTS ? 1 : 0, u32(t.nodeCount), qTree, qTree ? t.treeOff.as<u64>() : nullptr,
                       t.nodeDepth.as<unsigned char>() };
+  tv.inNodes = !t.respanned;
+  return tv;
 }
 
 template<typename T>
@@ -368,9 +371,9 @@ inline std::string query_key(const char* op, int algo, bool forest, bool f64, in
 // FP32 images of a built tree for the query filters (otg_knn.cu): built on first use after a build.
 // boxes: the box entities' images too (DevBuf boxImg32), which only some queries read.
 int ensure_image32(TreeState& t, cudaStream_t st, bool boxes = false);
-// Sets tv's images for a query on an FP64 box tree when they are there, or when the tree's queries
-// since its build are worth building them: `tests` estimates the entity tests of this call.
-int use_box_images(TreeState& t, TreeView<double>& tv, u64 tests, cudaStream_t st);
+// Sets tv's images for a query on an FP64 tree when they are there, or when the tree's queries since
+// its build are worth building them: `tests` estimates the entity tests of this call.
+int use_images(TreeState& t, TreeView<double>& tv, u64 tests, cudaStream_t st);
 
 // filtered candidate search of CollisionDetection (otg_collide.cu)
 struct CollideSearch
