@@ -1,25 +1,37 @@
 // otg_collide.cu — candidate search of CollisionDetection (core/ot_query.h:1308-1497 two trees,
 // :1690-1914 one tree) with an FP32 filter.
 //
-// One warp per entity of the first tree walks the other tree (entities of shallow nodes first, as
-// their walks are the longest; the rest are taken from a shared counter): a node is entered when
-// its MBR may meet the box, its own entities are tested by the lanes in parallel (coalesced loads
-// of their images), and its children are tested in parallel. The test runs on an FP32 image of both boxes rounded
-// outward (minimum and maximum rounded down, and rounded up with the tolerance added), which
-// decides GetBoxRelation (general.h:262-289) for all but rounding-level cases:
-//   certainly overlapped  a.min + tol < b.max and b.min + tol < a.max hold in every dimension
-//   certainly not         b.max + tol < a.min or a.max + tol < b.min holds in some dimension
-// (the first is the "overlapped" branch of every dimension; the second makes that dimension
-// "separated" or "adjacent", either of which excludes "overlapped"). The undecided rest is
-// re-tested with the exact predicate in the tree's scalar type, so the candidate set equals
-// {pairs with GetBoxRelation == Overlapped} exactly. In a single tree only pairs whose second
-// position follows the first are searched, so each pair is tested once.
+// One warp walks the other tree for a packet of 32 entities of the first tree that follow each other
+// in it at the same depth, and so lie close together. A stack entry is a node and the mask of the
+// entities whose boxes may meet it. The node's own entities are tested by the lanes in parallel
+// against each box of the mask (read from shared memory), its children against the packet's common
+// box first and then box by box. Entities of shallow nodes (large boxes, long walks, little in common)
+// come first, one to a packet; packets are taken from a shared counter.
+// Bound by instruction issue and by the latency of the node loads. One entity per warp spends a walk of
+// the upper levels on every box: 4M clustered FP64 boxes with themselves took 6.67 ms and now take 1.90 ms,
+// 8M against 16M 9.39 and 2.24 ms.
+//
+// The test runs on FP32 images of the second tree's boxes, lo = rd(min) and hi = ru(max). With M the
+// largest coordinate of the two root boxes and of the first box, and G = 2^-20 (M + tol), four bounds per dimension of the
+// first box decide GetBoxRelation (general.h:262-289) for all but a few pairs:
+//   certainly not         hi < a.min - tol - G or lo > a.max + tol + G in some dimension
+//   certainly overlapped  hi > a.min + tol + G and lo < a.max - tol - G in every dimension
+// G is eight times the images' rounding and, in FP32 trees, the rounding of the predicate itself: the
+// first makes that dimension "separated" or "adjacent" in its arithmetic, either of which excludes
+// "overlapped", the second is its "overlapped" branch. The rest is re-tested with the exact predicate
+// in the tree's scalar type, so the candidate set equals {pairs with GetBoxRelation == Overlapped}.
+// A certain overlap is also deeper than any rounding in the reference's tree walk, which prunes by
+// node boxes that hold the two: such pairs are marked (kPairSure) and spared the walk's rules in
+// collide_filter_kernel. In a single tree only pairs whose second position follows the first are
+// searched, so each pair is tested once.
 #include "otg_query.cuh"
+
+#include <cmath>
 
 namespace otg
 {
 
-constexpr int kPairBuf = 256;
+constexpr u32 kPairBuf = 128;
 
 struct CollideCounters
 {
@@ -29,229 +41,308 @@ struct CollideCounters
   u32 pad;
 };
 
-// per entity 12 floats in 3 float4: minD xyz, maxD xyz (rounded down), minU xyz, maxU xyz (rounded up, + tol)
-template<typename T>
-__global__ void box_image_kernel(const T* __restrict__ geom, u64 n, float tolHi, float4* __restrict__ out)
-{
-  for (u64 i = blockIdx.x * u64(blockDim.x) + threadIdx.x; i < n; i += u64(gridDim.x) * blockDim.x)
-  {
-    float v[12];
-#pragma unroll
-    for (int c = 0; c < 3; ++c)
-    {
-      const double mn = double(geom[i * 6 + c]), mx = double(geom[i * 6 + 3 + c]);
-      v[c] = __double2float_rd(mn);
-      v[3 + c] = __double2float_rd(mx);
-      v[6 + c] = __fadd_ru(__double2float_ru(mn), tolHi);
-      v[9 + c] = __fadd_ru(__double2float_ru(mx), tolHi);
-    }
-    out[3 * i] = make_float4(v[0], v[1], v[2], v[3]);
-    out[3 * i + 1] = make_float4(v[4], v[5], v[6], v[7]);
-    out[3 * i + 2] = make_float4(v[8], v[9], v[10], v[11]);
-  }
-}
-
-// node MBRs for one call: {min rounded down, 0}, {max rounded up + tol rounded up, 0}
-__global__ void node_tol_image_kernel(const float4* __restrict__ nodes32, u64 m, float tolHi, float4* __restrict__ out)
-{
-  for (u64 i = blockIdx.x * u64(blockDim.x) + threadIdx.x; i < m; i += u64(gridDim.x) * blockDim.x)
-  {
-    const float4 mx = nodes32[2 * i + 1];
-    out[2 * i] = nodes32[2 * i];
-    out[2 * i + 1] = make_float4(__fadd_ru(mx.x, tolHi), __fadd_ru(mx.y, tolHi), __fadd_ru(mx.z, tolHi), 0.f);
-  }
-}
-
-struct BoxImg
-{
-  float mnD[3], mxD[3], mnU[3], mxU[3];
-};
-
-__device__ __forceinline__ BoxImg load_img(const float4* __restrict__ img, u32 i)
-{
-  const float4 a = img[3 * size_t(i)], b = img[3 * size_t(i) + 1], c = img[3 * size_t(i) + 2];
-  BoxImg r;
-  r.mnD[0] = a.x;
-  r.mnD[1] = a.y;
-  r.mnD[2] = a.z;
-  r.mxD[0] = a.w;
-  r.mxD[1] = b.x;
-  r.mxD[2] = b.y;
-  r.mnU[0] = b.z;
-  r.mnU[1] = b.w;
-  r.mnU[2] = c.x;
-  r.mxU[0] = c.y;
-  r.mxU[1] = c.z;
-  r.mxU[2] = c.w;
-  return r;
-}
-
-// 1: certainly overlapped, -1: certainly not, 0: undecided in FP32
-__device__ __forceinline__ int img_relation(const BoxImg& a, const BoxImg& b)
-{
-  bool ov = true, sep = false;
-#pragma unroll
-  for (int c = 0; c < 3; ++c)
-  {
-    ov &= (a.mnU[c] < b.mxD[c]) & (b.mnU[c] < a.mxD[c]);
-    sep |= (b.mxU[c] < a.mnD[c]) | (a.mxU[c] < b.mnD[c]);
-  }
-  return ov ? 1 : (sep ? -1 : 0);
-}
-
 template<typename T>
 struct CollideArgs
 {
-  const float4* imgA;
   const T* geomA;
   u32 nA;
-  const u32* order; // processing order of the A entities
-  const u32* ownerA; // node holding each A entity (kNoOwner: none reachable, skipped)
-  const float4* imgB;
+  const u32* order;    // processing order of the A entities
+  const u32* ownerA;   // node holding each A entity (kNoOwner: none reachable, skipped)
+  const u32* singles;  // entities at the front of the order that are walked one by one
+  const T* rootA;      // root boxes {min, size}
+  const T* rootB;
+  const float4* imgB;  // per entity {min rounded down}, {max rounded up}
   const T* geomB;
   const uint4* linkB;
-  const float4* nodeB; // node MBRs of tree B: min rounded down, max + tol rounded up (2 float4 per node)
+  const float4* nodeB; // per node {min rounded down}, {max rounded up}
   u32 nB, nNodesB;
-  float tolHi;
+  u32 stackCap;        // entries of a warp's stack
   T tol;
   int selfMode;
   int swapOut; // two trees searched from the second tree's entities: emit (walked position, entity position)
+  // Entities lie in their nodes. If not (set_entities), which pairs are found depends on the nodes that a
+  // box enters: node boxes are then tested without G (tolHi: tol rounded up), and no overlap is marked.
+  int sure;
+  float tolHi;
   Appender out;
   CollideCounters* ctr;
   u32* err;
 };
 
-template<typename T, int WARPS>
-__global__ void __launch_bounds__(WARPS * 32) collide_box_kernel(CollideArgs<T> a)
+// a warp's shared memory: the packet's bounds (a.min - tol - G, position; a.max + tol + G; a.min + tol + G;
+// a.max - tol - G), the children's boxes, the pair buffer, the stack (a multiple of 4 entries, so that
+// every warp's part starts on 16 bytes)
+struct CollideWarpMem
 {
-  __shared__ u32 stackMem[WARPS][kStack];
-  __shared__ u64 pairMem[WARPS][kPairBuf];
+  float4 box[32][4];
+  float4 child[8][2];
+  u64 pairs[kPairBuf];
+};
+static_assert(sizeof(CollideWarpMem) % 16 == 0, "warps' parts start on 16 bytes");
+__host__ __device__ constexpr size_t collide_warp_bytes(u32 stackCap) { return sizeof(CollideWarpMem) + size_t(stackCap) * (sizeof(uint4) + sizeof(u32)); }
+
+__device__ __forceinline__ bool apart(float4 a0, float4 a1, float4 lo, float4 hi)
+{
+  return (hi.x < a0.x) | (hi.y < a0.y) | (hi.z < a0.z) | (a1.x < lo.x) | (a1.y < lo.y) | (a1.z < lo.z);
+}
+
+template<typename T>
+__device__ __noinline__ bool boxes_overlap_exact(const T* a, const T* b, T tol)
+{
+  T ea[6], eb[6];
+  load_box(a, ea);
+  load_box(b, eb);
+  return GeoD<T>::box_relation(ea, eb, tol) == -1;
+}
+
+template<typename T, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32) collide_packet_kernel(CollideArgs<T> a)
+{
+  extern __shared__ __align__(16) unsigned char collideMem[];
   const u32 lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  u32* stack = stackMem[w];
-  u64* pbuf = pairMem[w];
+  unsigned char* mem = collideMem + w * collide_warp_bytes(a.stackCap);
+  CollideWarpMem& W = *reinterpret_cast<CollideWarpMem*>(mem);
+  uint4* stackL = reinterpret_cast<uint4*>(mem + sizeof(CollideWarpMem));
+  u32* stackM = reinterpret_cast<u32*>(stackL + a.stackCap);
   const u32 lt = (1u << lane) - 1;
-  unsigned long long tests = 0, rechecks = 0;
+  u32 tests = 0, rechecks = 0;
+  const u32 singles = min(*a.singles, a.nA);
+  const u32 items = singles + (a.nA - singles + 31) / 32;
+  float M = 0.f; // of the header comment
+#pragma unroll
+  for (int c = 0; c < 3; ++c)
+  {
+    M = fmaxf(M, fmaxf(fabsf(float(a.rootA[c])), fabsf(float(T(a.rootA[c] + a.rootA[3 + c])))));
+    M = fmaxf(M, fmaxf(fabsf(float(a.rootB[c])), fabsf(float(T(a.rootB[c] + a.rootB[3 + c])))));
+  }
+  const float tolf = float(a.tol);
+  const uint4 root = a.linkB[0];
+  auto flush = [&](u32 n) {
+    unsigned long long b0 = 0;
+    if (lane == 0)
+      b0 = a.out.reserve(n);
+    b0 = __shfl_sync(~0u, b0, 0);
+    for (u32 t = lane; t < n; t += 32)
+      if (b0 + t < a.out.capacity)
+        a.out.items[b0 + t] = W.pairs[t];
+    __syncwarp();
+  };
   for (;;)
   {
     u32 item = 0;
     if (lane == 0)
       item = atomicAdd(&a.ctr->work, 1u);
     item = __shfl_sync(~0u, item, 0);
-    if (item >= a.nA)
+    if (item >= items)
       break;
-    const u32 i = a.order ? a.order[item] : item;
-    if (a.ownerA && a.ownerA[i] == kNoOwner)
-      continue; // an entity that no node reachable from the root holds takes part in no pair
-    const BoxImg me = load_img(a.imgA, i);
-    u32 nbuf = 0;
-    if (lane == 0)
-      stack[0] = 0;
-    __syncwarp();
-    int sp = 1;
-    u32 visits = 0;
+    const u32 first = item < singles ? item : singles + (item - singles) * 32;
+    const u32 count = item < singles ? 1u : min(32u, a.nA - first);
+    u32 i = 0xffffffffu;
+    bool valid = false;
+    float4 a0 = make_float4(INFINITY, INFINITY, INFINITY, 0.f), a1 = make_float4(-INFINITY, -INFINITY, -INFINITY, 0.f);
+    float4 n0 = a0, n1 = a1; // the bounds for node boxes
+    if (lane < count)
+    {
+      i = a.order[first + lane];
+      // an entity that no node reachable from the root holds takes part in no pair
+      valid = a.ownerA[i] != kNoOwner;
+      T e[6];
+      load_box(a.geomA + u64(i) * 6, e);
+      // round-to-nearest: G is many times the roundings here (this box may lie outside the root box
+      // after set_entities)
+      const float mn[3] = { float(e[0]), float(e[1]), float(e[2]) }, mx[3] = { float(e[3]), float(e[4]), float(e[5]) };
+      float far = M;
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+        far = fmaxf(far, fmaxf(fabsf(mn[c]), fabsf(mx[c])));
+      const float up = tolf + ((far + tolf) * 0x1p-20f + 0x1p-140f);
+      // a bound that is no finite number excludes nothing
+      auto below = [](float v) { return fabsf(v) < INFINITY ? v : -INFINITY; };
+      auto above = [](float v) { return fabsf(v) < INFINITY ? v : INFINITY; };
+      if (valid)
+      {
+        a0 = make_float4(below(mn[0] - up), below(mn[1] - up), below(mn[2] - up), 0.f);
+        a1 = make_float4(above(mx[0] + up), above(mx[1] + up), above(mx[2] + up), 0.f);
+      }
+      n0 = a0;
+      n1 = a1;
+      if (valid && !a.sure)
+      {
+        n0 = make_float4(__double2float_rd(double(e[0])), __double2float_rd(double(e[1])), __double2float_rd(double(e[2])), 0.f);
+        n1 = make_float4(__fadd_ru(__double2float_ru(double(e[3])), a.tolHi), __fadd_ru(__double2float_ru(double(e[4])), a.tolHi),
+                         __fadd_ru(__double2float_ru(double(e[5])), a.tolHi), 0.f);
+      }
+      a0.w = __uint_as_float(i);
+      W.box[lane][0] = a0;
+      W.box[lane][1] = a1;
+      W.box[lane][2] = make_float4(mn[0] + up, mn[1] + up, mn[2] + up, 0.f);
+      W.box[lane][3] = make_float4(mx[0] - up, mx[1] - up, mx[2] - up, 0.f);
+    }
+    // the packet's common box and first position
+    float4 u0 = a0, u1 = a1;
+    u32 iMin = valid ? i : 0xffffffffu;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+    {
+      u0.x = fminf(u0.x, __shfl_xor_sync(~0u, u0.x, o));
+      u0.y = fminf(u0.y, __shfl_xor_sync(~0u, u0.y, o));
+      u0.z = fminf(u0.z, __shfl_xor_sync(~0u, u0.z, o));
+      u1.x = fmaxf(u1.x, __shfl_xor_sync(~0u, u1.x, o));
+      u1.y = fmaxf(u1.y, __shfl_xor_sync(~0u, u1.y, o));
+      u1.z = fmaxf(u1.z, __shfl_xor_sync(~0u, u1.z, o));
+      iMin = min(iMin, __shfl_xor_sync(~0u, iMin, o));
+    }
+    const u32 all = __ballot_sync(~0u, valid);
+    if (!all)
+      continue;
+    u32 sp = 1, visits = 0, nbuf = 0;
     bool bad = false;
+    if (lane == 0)
+    {
+      stackL[0] = root;
+      stackM[0] = all;
+    }
+    __syncwarp();
     while (sp > 0)
     {
-      const u32 node = stack[--sp];
+      --sp;
+      const uint4 L = stackL[sp];
+      const u32 mask = stackM[sp];
       __syncwarp();
-      const uint4 L = a.linkB[node];
-      if (L.z > a.nB || L.y > L.z || ++visits > a.nNodesB)
+      const u32 fc = L.x & kFirstChildMask, cc = L.x >> kChildShift;
+      if (L.z > a.nB || L.y > L.z || ++visits > a.nNodesB || cc > 8u || u64(fc) + cc > a.nNodesB || sp + cc > a.stackCap)
       {
         bad = true;
         break;
       }
-      const u32 jb = a.selfMode ? max(L.y, i + 1) : L.y;
+      // the children's boxes and links on their way while the entities are tested
+      float4 cl = make_float4(0.f, 0.f, 0.f, 0.f), ch = cl;
+      uint4 cL = make_uint4(0u, 0u, 0u, 0u);
+      if (lane < cc)
+      {
+        cl = a.nodeB[2 * size_t(fc + lane)];
+        ch = a.nodeB[2 * size_t(fc + lane) + 1];
+        cL = a.linkB[fc + lane];
+        if (!a.sure)
+          ch = make_float4(__fadd_ru(ch.x, a.tolHi), __fadd_ru(ch.y, a.tolHi), __fadd_ru(ch.z, a.tolHi), 0.f);
+      }
+      const u32 jb = a.selfMode ? max(L.y, iMin + 1) : L.y;
       for (u32 base = jb; base < L.z; base += 32)
       {
         const u32 j = base + lane;
-        bool hit = false;
+        bool in = false;
+        float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
         if (j < L.z)
         {
-          const int rel = img_relation(me, load_img(a.imgB, j));
-          hit = rel == 1;
-          if (rel == 0)
-          {
-            T ea[6], eb[6];
-            load_box(a.geomA + u64(i) * 6, ea);
-            load_box(a.geomB + u64(j) * 6, eb);
-            hit = GeoD<T>::box_relation(ea, eb, a.tol) == -1;
-            ++rechecks;
-          }
-          ++tests;
+          lo = a.imgB[2 * size_t(j)];
+          hi = a.imgB[2 * size_t(j) + 1];
+          in = !apart(u0, u1, lo, hi);
         }
-        const u32 bal = __ballot_sync(~0u, hit);
-        if (bal)
+        if (!__any_sync(~0u, in))
+          continue;
+        for (u32 mm = mask; mm; mm &= mm - 1)
         {
+          const u32 l = u32(__ffs(int(mm))) - 1;
+          const float4 b0 = W.box[l][0], b1 = W.box[l][1];
+          const u32 il = __float_as_uint(b0.w);
+          const bool cand = in && !apart(b0, b1, lo, hi) && (!a.selfMode || j > il);
+          ++tests;
+          if (!__any_sync(~0u, cand))
+            continue;
+          bool hit = false, sure = false;
+          if (cand)
+          {
+            const float4 c0 = W.box[l][2], c1 = W.box[l][3];
+            sure = (hi.x > c0.x) & (hi.y > c0.y) & (hi.z > c0.z) & (lo.x < c1.x) & (lo.y < c1.y) & (lo.z < c1.z);
+            hit = sure;
+            if (!sure)
+            {
+              hit = boxes_overlap_exact<T>(a.geomA + u64(il) * 6, a.geomB + u64(j) * 6, a.tol);
+              ++rechecks;
+            }
+          }
+          const u32 bal = __ballot_sync(~0u, hit);
+          if (!bal)
+            continue;
           if (nbuf + 32 > kPairBuf)
           {
-            unsigned long long b0 = 0;
-            if (lane == 0)
-              b0 = a.out.reserve(nbuf);
-            b0 = __shfl_sync(~0u, b0, 0);
-            for (u32 t = lane; t < nbuf; t += 32)
-              if (b0 + t < a.out.capacity)
-                a.out.items[b0 + t] = pbuf[t];
-            __syncwarp();
+            flush(nbuf);
             nbuf = 0;
           }
           if (hit)
-            pbuf[nbuf + __popc(bal & lt)] = a.swapOut ? ((u64(j) << 32) | i) : ((u64(i) << 32) | j);
+          {
+            const u64 mark = sure && a.sure ? kPairSure : 0;
+            W.pairs[nbuf + __popc(bal & lt)] = (a.swapOut ? ((u64(j) << 32) | il) : ((u64(il) << 32) | j)) | mark;
+          }
           nbuf += __popc(bal);
           __syncwarp();
         }
       }
-      const u32 fc = L.x & kFirstChildMask, cc = L.x >> kChildShift;
       if (cc)
       {
-        if (u64(fc) + cc > a.nNodesB || sp + int(cc) > kStack)
+        // the subtree must reach the packet's box, and in a single tree hold a position after its first
+        const bool ok = lane < cc && !apart(u0, u1, cl, ch) && (!a.selfMode || cL.w > iMin + 1);
+        u32 bal = __ballot_sync(~0u, ok);
+        if (ok)
         {
-          bad = true;
-          break;
+          cl.w = __uint_as_float(cL.w);
+          W.child[lane][0] = cl;
+          W.child[lane][1] = ch;
         }
-        bool keep = false;
-        if (lane < cc)
+        __syncwarp();
+        while (bal)
         {
-          const u32 ch = fc + lane;
-          const float4 mn = a.nodeB[2 * size_t(ch)], mx = a.nodeB[2 * size_t(ch) + 1];
-          const float nmn[3] = { mn.x, mn.y, mn.z }, nmx[3] = { mx.x, mx.y, mx.z };
-          keep = true;
-#pragma unroll
-          for (int c = 0; c < 3; ++c)
-            keep &= !((nmx[c] < me.mnD[c]) | (me.mxU[c] < nmn[c]));
-          if (keep && a.selfMode)
-            keep = a.linkB[ch].w > i + 1; // the subtree holds a position after this entity
+          const u32 k = u32(__ffs(int(bal))) - 1;
+          bal &= bal - 1;
+          const float4 nl = W.child[k][0], nh = W.child[k][1];
+          const bool keep = ((mask >> lane) & 1u) && !apart(n0, n1, nl, nh) && (!a.selfMode || __float_as_uint(nl.w) > i + 1);
+          const u32 m = __ballot_sync(~0u, keep);
+          if (m)
+          {
+            if (lane == k)
+            {
+              stackL[sp] = cL;
+              stackM[sp] = m;
+            }
+            ++sp;
+          }
         }
-        const u32 bal = __ballot_sync(~0u, keep);
-        if (keep)
-          stack[sp + __popc(bal & lt)] = fc + lane;
-        sp += __popc(bal);
         __syncwarp();
       }
     }
     if (bad && lane == 0)
       atomicOr(a.err, kErrStack);
     if (nbuf)
-    {
-      unsigned long long b0 = 0;
-      if (lane == 0)
-        b0 = a.out.reserve(nbuf);
-      b0 = __shfl_sync(~0u, b0, 0);
-      for (u32 t = lane; t < nbuf; t += 32)
-        if (b0 + t < a.out.capacity)
-          a.out.items[b0 + t] = pbuf[t];
-    }
+      flush(nbuf);
     __syncwarp();
   }
+  // a box test is one lane's: every lane counts the tests it took part in
+  unsigned long long t = tests, r = rechecks;
   for (int o = 16; o > 0; o >>= 1)
   {
-    tests += __shfl_xor_sync(~0u, tests, o);
-    rechecks += __shfl_xor_sync(~0u, rechecks, o);
+    t += __shfl_xor_sync(~0u, t, o);
+    r += __shfl_xor_sync(~0u, r, o);
   }
   if (lane == 0)
   {
-    atomicAdd(&a.ctr->tests, tests);
-    atomicAdd(&a.ctr->rechecks, rechecks);
+    atomicAdd(&a.ctr->tests, t);
+    atomicAdd(&a.ctr->rechecks, r);
   }
+}
+
+// entities of nodes above depth `cut` come first in the order (sorted owner depths)
+__global__ void collide_singles_kernel(const u32* __restrict__ keys, u32 n, u32 cut, u32* __restrict__ singles)
+{
+  u32 lo = 0, hi = n;
+  while (lo < hi)
+  {
+    const u32 mid = (lo + hi) >> 1;
+    if (keys[mid] < cut)
+      lo = mid + 1;
+    else
+      hi = mid;
+  }
+  *singles = lo;
 }
 
 // processing order: entities of shallow nodes (large boxes, long walks) first
@@ -266,31 +357,25 @@ __global__ void owner_depth_key_kernel(const u32* __restrict__ owner, const unsi
   }
 }
 
-static void host_ru(double v, float& hi)
-{
-  float f = float(v);
-  if (double(f) < v)
-    f = std::nextafter(f, __builtin_huge_valf());
-  hi = f;
-}
-
 template<typename T, int WARPS>
 static int launch_collide(const CollideArgs<T>& a, cudaStream_t st)
 {
+  const size_t smem = collide_warp_bytes(a.stackCap) * WARPS;
   int dev = 0, sms = 0, per = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (!e)
     e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (!e)
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, collide_box_kernel<T, WARPS>, WARPS * 32, 0);
+    e = cudaFuncSetAttribute(collide_packet_kernel<T, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+  if (!e)
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, collide_packet_kernel<T, WARPS>, WARPS * 32, smem);
   if (e)
     return cuda_status(e, "configuring the collision kernel");
   const u32 grid = u32(std::max<u64>(1, std::min<u64>(u64(sms) * std::max(per, 1), (u64(a.nA) + WARPS - 1) / WARPS)));
-  collide_box_kernel<T, WARPS><<<grid, WARPS * 32, 0, st>>>(a);
+  collide_packet_kernel<T, WARPS><<<grid, WARPS * 32, smem, st>>>(a);
   return cuda_status(cudaGetLastError(), "launching the collision kernel");
 }
 
-// Per-call state of the filtered search: the tolerance-specific FP32 images of both trees.
 template<typename T>
 static int collide_search_impl(TreeState& A, TreeState& B, bool self, bool swapOut, double tol, Appender out, u32* err, CollideSearch& s,
                                cudaStream_t st)
@@ -298,45 +383,46 @@ static int collide_search_impl(TreeState& A, TreeState& B, bool self, bool swapO
   cudaError_t e;
   if (!s.ready)
   {
-    if (int rc = ensure_image32(B, st))
+    if (int rc = ensure_image32(B, st, true))
       return rc;
-    const T tl = tol < 0 ? base_tol<T>() : T(tol);
-    host_ru(double(tl), s.tolHi);
-    if ((e = s.imgA.ensure(sizeof(float4) * 3 * std::max<u64>(A.n, 1))) || (!self && (e = s.imgB.ensure(sizeof(float4) * 3 * std::max<u64>(B.n, 1)))) ||
-        (e = s.ctr.ensure(sizeof(CollideCounters))) || (e = s.nodesB.ensure(sizeof(float4) * 2 * std::max<u64>(B.nodeCount, 1))))
-      return cuda_status(e, "allocating the collision images");
-    node_tol_image_kernel<<<blocks_for(B.nodeCount), 256, 0, st>>>(B.nodeBox32.as<float4>(), B.nodeCount, s.tolHi, s.nodesB.as<float4>());
-    box_image_kernel<T><<<blocks_for(A.n), 256, 0, st>>>(A.sortedGeom.as<T>(), A.n, s.tolHi, s.imgA.as<float4>());
-    if (!self)
-      box_image_kernel<T><<<blocks_for(B.n), 256, 0, st>>>(B.sortedGeom.as<T>(), B.n, s.tolHi, s.imgB.as<float4>());
-    s.ready = true;
-  }
-  if (!s.orderReady)
-  {
     TmpBuf keys;
-    if ((e = keys.ensure(sizeof(u32) * std::max<u64>(A.n, 1), st)) || (e = s.order.ensure(sizeof(u32) * std::max<u64>(A.n, 1))))
+    if ((e = s.ctr.ensure(sizeof(CollideCounters) + sizeof(u32), st)) || (e = keys.ensure(sizeof(u32) * std::max<u64>(A.n, 1), st)) ||
+        (e = s.order.ensure(sizeof(u32) * std::max<u64>(A.n, 1), st)))
       return cuda_status(e, "allocating the collision order");
     owner_depth_key_kernel<<<blocks_for(A.n), 256, 0, st>>>(A.ownerNode.as<u32>(), A.nodeDepth.as<unsigned char>(), A.n, keys.as<u32>(), s.order.as<u32>());
     if (int rc = sort_pairs_u32(keys.as<u32>(), s.order.as<u32>(), A.n, 5, st, err))
       return rc;
-    s.orderReady = true;
+    // One to a packet above the depth whose cells hold 256 nodes of the walked tree on average: the
+    // walks of such boxes are long, and 32 of them in one warp would end last.
+    u32 cut = 0;
+    while (cut < 19 && (B.nodeCount >> (3 * cut)) > 256)
+      ++cut;
+    collide_singles_kernel<<<1, 1, 0, st>>>(keys.as<u32>(), u32(A.n), cut, reinterpret_cast<u32*>(s.ctr.as<CollideCounters>() + 1));
+    s.ready = true;
   }
   CollideArgs<T> a{};
   a.order = s.order.as<u32>();
   a.ownerA = A.ownerNode.as<u32>();
-  a.imgA = s.imgA.as<float4>();
+  a.singles = reinterpret_cast<const u32*>(s.ctr.as<CollideCounters>() + 1);
+  a.rootA = A.nodeBox.as<T>();
+  a.rootB = B.nodeBox.as<T>();
   a.geomA = A.sortedGeom.as<T>();
   a.nA = u32(A.n);
-  a.imgB = self ? s.imgA.as<float4>() : s.imgB.as<float4>();
+  a.imgB = B.boxImg32.as<float4>();
   a.geomB = B.sortedGeom.as<T>();
   a.linkB = B.nodeLink.as<uint4>();
-  a.nodeB = s.nodesB.as<float4>();
+  a.nodeB = B.nodeBox32.as<float4>();
   a.nB = u32(B.n);
   a.nNodesB = u32(B.nodeCount);
-  a.tolHi = s.tolHi;
+  // depth first: at most 7 entries per level beside the current node's 8 children
+  a.stackCap = (7 * (B.D + 1) + 9 + 3) & ~3u;
   a.tol = tol < 0 ? base_tol<T>() : T(tol);
   a.selfMode = self ? 1 : 0;
   a.swapOut = swapOut ? 1 : 0;
+  a.sure = !A.respanned && !B.respanned;
+  a.tolHi = float(a.tol);
+  if (double(a.tolHi) < double(a.tol))
+    a.tolHi = std::nextafter(a.tolHi, __builtin_huge_valf());
   a.out = out;
   a.ctr = s.ctr.as<CollideCounters>();
   a.err = err;

@@ -355,4 +355,74 @@ __global__ void bit_write_kernel(const u32* __restrict__ bits, const u64* __rest
   }
 }
 
+// ---- pairs: one warp per 32 neighbouring a's sorts their runs of b's by rank (the count of smaller b's in
+// the run: runs average a few items) and writes (a, b); a run above kPairRunMax is only counted.
+constexpr u32 kPairRunMax = 1024;
+constexpr u32 kPairTile = 512;
+__global__ void __launch_bounds__(256) pair_write_kernel(const u64* __restrict__ off, u64 nA, const u32* __restrict__ bs, uint2* __restrict__ out,
+                                                         u32* __restrict__ tooLong)
+{
+  __shared__ u32 sb[8][kPairTile];
+  __shared__ u32 so[8][33];
+  const u32 lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const u64 warps = u64(gridDim.x) * 8;
+  for (u64 g = u64(blockIdx.x) * 8 + w; g * 32 < nA; g += warps)
+  {
+    const u64 a0 = g * 32;
+    const u64 base = off[a0];
+    const u64 at = off[min(a0 + lane + 1, nA)]; // runs past the last one are empty
+    const u64 total = __shfl_sync(~0u, at, 31) - base;
+    if (total == 0)
+      continue;
+    const u64 prev = __shfl_up_sync(~0u, at, 1);
+    const u64 len = at - (lane ? prev : base);
+    if (__any_sync(~0u, len > kPairRunMax))
+    {
+      if (lane == 0)
+        atomicAdd(tooLong, 1u);
+      continue;
+    }
+    const u32 T = u32(total); // at most 32 * kPairRunMax
+    so[w][lane + 1] = u32(at - base);
+    if (lane == 0)
+      so[w][0] = 0;
+    const bool tile = T <= kPairTile;
+    if (tile)
+      for (u32 t = lane; t < T; t += 32)
+        sb[w][t] = bs[base + t];
+    __syncwarp();
+    for (u32 t = lane; t < T; t += 32)
+    {
+      u32 r = 0; // the run of item t: the last one that starts at or before it
+#pragma unroll
+      for (u32 s = 16; s > 0; s >>= 1)
+        if (so[w][r + s] <= t)
+          r += s;
+      const u32 b0 = so[w][r], b1 = so[w][r + 1];
+      u32 rank = 0;
+      u32 v;
+      if (tile)
+      {
+        v = sb[w][t];
+        for (u32 x = b0; x < b1; ++x)
+          rank += sb[w][x] < v ? 1u : 0u;
+      }
+      else
+      {
+        v = bs[base + t];
+        for (u32 x = b0; x < b1; ++x)
+          rank += bs[base + x] < v ? 1u : 0u;
+      }
+      out[base + b0 + rank] = make_uint2(u32(a0) + r, v);
+    }
+    __syncwarp();
+  }
+}
+// (a << bBits | b) into (a, b)
+__global__ void unpack_pairs_kernel(const u64* __restrict__ items, u64 m, u32 bBits, uint2* __restrict__ out)
+{
+  for (u64 i = blockIdx.x * u64(blockDim.x) + threadIdx.x; i < m; i += u64(gridDim.x) * blockDim.x)
+    out[i] = make_uint2(u32(items[i] >> bBits), u32(items[i] & ((u64(1) << bBits) - 1)));
+}
+
 } // namespace otg

@@ -375,15 +375,15 @@ int ensure_image32(TreeState& t, cudaStream_t st, bool boxes = false);
 // its build are worth building them: `tests` estimates the entity tests of this call.
 int use_images(TreeState& t, TreeView<double>& tv, u64 tests, cudaStream_t st);
 
-// filtered candidate search of CollisionDetection (otg_collide.cu)
+// filtered candidate search of CollisionDetection (otg_collide.cu): pairs of sorted positions
+// (first << 32 | second), with kPairSure set where the walk's rules need no check (positions are
+// below 2^30)
+constexpr u64 kPairSure = u64(1) << 31;
 struct CollideSearch
 {
-  DevBuf imgA, imgB, ctr; // tolerance-specific FP32 box images, counters
-  DevBuf order;           // processing order of the first tree's entities
-  DevBuf nodesB;          // the second tree's node MBRs with the tolerance added
-  float tolHi = 0.f;
+  TmpBuf ctr;   // counters
+  TmpBuf order; // processing order of the first tree's entities
   bool ready = false;
-  bool orderReady = false;
 };
 int collide_search_filtered(TreeState& A, TreeState& B, bool self, double tol, Appender out, u32* err, CollideSearch& s, cudaStream_t st);
 int collide_search_stats(const CollideSearch& s, u64& tests, u64& rechecks, cudaStream_t st);
