@@ -716,42 +716,83 @@ __global__ void location_export_kernel(const T* __restrict__ geom, const u32* __
 }
 
 // ---------------------------------------------------------------- 5. gather into tree order
-// Random reads of whole entities: every thread issues the loads of kGatherPerThread entities
-// before storing any of them, so many sectors are in flight per thread.
-constexpr int kGatherPerThread = 4;
-constexpr int kGatherWide = 8; // the single-tree gather that runs beside the emission
-
-template<typename T, int W, int G>
-__global__ void __launch_bounds__(256) gather_kernel(const T* __restrict__ ent, const u32* __restrict__ ids, u64 n, T* __restrict__ out)
+// Every entity type is three units of 4, 8 or 16 bytes (FP32 points; FP64 points and FP32 boxes; FP64
+// boxes). Consecutive threads take consecutive units, so three lanes read one entity and the writes are
+// whole lines; every thread issues the loads of G units before storing any of them. One lane per entity
+// read its record in 3 to 6 instructions that touch 32 lines each, and the load unit was the bound where
+// the entities sit in L2: 65.8M FP32 boxes of 4096 trees 1.19 ms, now 1.00; 8M FP64 boxes beside their emission 0.353 ms, now 0.297.
+template<int BYTES>
+struct GatherUnit;
+template<>
+struct GatherUnit<4>
 {
-  constexpr int kGatherPerThread = G;
+  using Type = u32;
+};
+template<>
+struct GatherUnit<8>
+{
+  using Type = uint2;
+};
+template<>
+struct GatherUnit<16>
+{
+  using Type = uint4;
+};
+constexpr int kGatherPerThread = 8;
+
+// vec: both arrays start on a multiple of the unit (the tree's always does; a caller's may not)
+template<typename T, int W, int G>
+__global__ void __launch_bounds__(256) gather_kernel(const T* __restrict__ ent, const u32* __restrict__ ids, u64 n, T* __restrict__ out, bool vec)
+{
+  using Unit = typename GatherUnit<int(sizeof(T)) * W / 3>::Type;
+  constexpr int S = W / 3; // scalars per unit
+  constexpr u32 kNone = 0xffffffffu;
+  const Unit* src = reinterpret_cast<const Unit*>(ent);
+  Unit* dst = reinterpret_cast<Unit*>(out);
   const u64 stride = u64(gridDim.x) * blockDim.x;
-  for (u64 i0 = blockIdx.x * u64(blockDim.x) + threadIdx.x; i0 < n; i0 += stride * kGatherPerThread)
+  const u64 units = n * 3;
+  for (u64 i0 = blockIdx.x * u64(blockDim.x) + threadIdx.x; i0 < units; i0 += stride * G)
   {
-    T v[kGatherPerThread][W];
-    u32 id[kGatherPerThread];
+    Unit v[G];
+    u32 from[G]; // (entities are below 2^30, so units fit 32 bits)
 #pragma unroll
-    for (int k = 0; k < kGatherPerThread; ++k)
+    for (int k = 0; k < G; ++k)
     {
       const u64 i = i0 + k * stride;
-      id[k] = i < n ? ids[i] : 0xffffffffu;
+      from[k] = kNone;
+      if (i < units)
+      {
+        const u32 e = u32(i) / 3u;
+        const u32 id = ids[e];
+        if (id < n)
+          from[k] = id * 3u + (u32(i) - e * 3u);
+      }
     }
 #pragma unroll
-    for (int k = 0; k < kGatherPerThread; ++k)
-      if (id[k] < n)
+    for (int k = 0; k < G; ++k)
+      if (from[k] != kNone)
+      {
+        if (vec)
+          v[k] = src[from[k]];
+        else
+        {
+          T x[S];
 #pragma unroll
-        for (int c = 0; c < W; ++c)
-          v[k][c] = ent[u64(id[k]) * W + c];
+          for (int c = 0; c < S; ++c)
+            x[c] = ent[u64(from[k]) * S + c];
+          memcpy(&v[k], x, sizeof(Unit));
+        }
+      }
 #pragma unroll
-    for (int k = 0; k < kGatherPerThread; ++k)
-    {
-      const u64 i = i0 + k * stride;
-      if (i < n && id[k] < n)
-#pragma unroll
-        for (int c = 0; c < W; ++c)
-          out[i * W + c] = v[k][c];
-    }
+    for (int k = 0; k < G; ++k)
+      if (from[k] != kNone)
+        dst[i0 + k * stride] = v[k];
   }
+}
+template<typename T, int W>
+static bool gather_aligned(const T* ent)
+{
+  return reinterpret_cast<uintptr_t>(ent) % (sizeof(T) * W / 3) == 0;
 }
 
 // ---------------------------------------------------------------- 6. node emission
@@ -1452,15 +1493,12 @@ static int build_impl(TreeState& t, const T* ent, const void* box, u64 n, cudaSt
   if ((e = cudaEventRecord(t.fork, st)) || (e = cudaStreamWaitEvent(es, t.fork, 0)))
     return cuda_status(e, "ordering the emission stream");
   prof.mark("gather+emit", st);
-  // Two gather blocks per SM, 8 independent entity loads per thread, leave the rest of each SM to the
-  // emission. A full-occupancy gather holds every SM until it ends. Measured beside the emission
-  // (16M points): 0.512 ms for this shape, 0.573 ms for one block per SM with 4 loads, 0.587 ms at
-  // full occupancy (sweep of 152-2432 blocks and 2-16 loads per thread).
-  // Box trees (entities twice as wide): one block per SM with 2 loads per thread, 2.5% faster for the
-  // 8M-box rebuild than 4 loads (sweep of 152-608 blocks and 2-4 loads per thread).
-  constexpr int G = IS_BOX ? 2 : kGatherWide;
-  gather_kernel<T, W, G><<<grid_blocks((n + G - 1) / G, 256, IS_BOX ? 152 : 2 * 152), 256, 0, st>>>(ent, t.sortedIds.as<u32>(), n,
-                                                                                                   t.sortedGeom.as<T>());
+  // A few gather blocks per SM leave the rest of each SM to the emission: a full-occupancy gather holds
+  // every SM until it ends. Build and static export of 16M points: 1.880 ms with 3 blocks per SM and 8 units
+  // per thread, 1.914 with 2, 1.904 with 4, 1.955 with 6, 1.889 with 3 blocks of 4 units, 2.05 with 16 units.
+  // Rebuild of 8M boxes with its collision: 3.762 ms with 2 blocks, 3.764 with 3, 3.857 with 4.
+  gather_kernel<T, W, kGatherPerThread><<<grid_blocks((3 * n + kGatherPerThread - 1) / kGatherPerThread, 256, (IS_BOX ? 2 : 3) * 152), 256, 0, st>>>(
+    ent, t.sortedIds.as<u32>(), n, t.sortedGeom.as<T>(), gather_aligned<T, W>(ent));
 
   u32* parent = IS_BOX ? t.nodeParent.as<u32>() : nullptr;
   const int emitBlocks = grid_blocks(maxNodes, 256, 152 * 16);
@@ -1949,8 +1987,8 @@ static int forest_build_impl(TreeState& t, const T* ent, const T* boxes, cudaStr
   const cudaStream_t es = st;
   prof.mark("gather", st);
   if (n)
-    gather_kernel<T, W, kGatherPerThread><<<grid_blocks((n + kGatherPerThread - 1) / kGatherPerThread, 256, 152 * 16), 256, 0, st>>>(
-      ent, t.sortedIds.as<u32>(), n, t.sortedGeom.as<T>());
+    gather_kernel<T, W, kGatherPerThread><<<grid_blocks((3 * n + kGatherPerThread - 1) / kGatherPerThread, 256, 152 * 16), 256, 0, st>>>(
+      ent, t.sortedIds.as<u32>(), n, t.sortedGeom.as<T>(), gather_aligned<T, W>(ent));
   prof.mark("emit", st);
   u32* parent = IS_BOX ? t.nodeParent.as<u32>() : nullptr;
   // entities that the emission places in no node keep kNoOwner
@@ -2203,20 +2241,24 @@ int set_entities(TreeState& t, const void* entities, u64 n, int mem, cudaStream_
       return cuda_status(e, "copying entities");
     src = t.entities.p;
   }
-  const int blocks = grid_blocks((n + kGatherPerThread - 1) / kGatherPerThread, 256, 152 * 16);
+  const int blocks = grid_blocks((3 * n + kGatherPerThread - 1) / kGatherPerThread, 256, 152 * 16);
   if (t.scalar == OTG_SCALAR_F64)
   {
     if (isBox)
-      gather_kernel<double, 6, kGatherPerThread><<<blocks, 256, 0, st>>>((const double*)src, t.sortedIds.as<u32>(), n, t.sortedGeom.as<double>());
+      gather_kernel<double, 6, kGatherPerThread><<<blocks, 256, 0, st>>>((const double*)src, t.sortedIds.as<u32>(), n, t.sortedGeom.as<double>(),
+                                                                              gather_aligned<double, 6>((const double*)src));
     else
-      gather_kernel<double, 3, kGatherPerThread><<<blocks, 256, 0, st>>>((const double*)src, t.sortedIds.as<u32>(), n, t.sortedGeom.as<double>());
+      gather_kernel<double, 3, kGatherPerThread><<<blocks, 256, 0, st>>>((const double*)src, t.sortedIds.as<u32>(), n, t.sortedGeom.as<double>(),
+                                                                              gather_aligned<double, 3>((const double*)src));
   }
   else
   {
     if (isBox)
-      gather_kernel<float, 6, kGatherPerThread><<<blocks, 256, 0, st>>>((const float*)src, t.sortedIds.as<u32>(), n, t.sortedGeom.as<float>());
+      gather_kernel<float, 6, kGatherPerThread><<<blocks, 256, 0, st>>>((const float*)src, t.sortedIds.as<u32>(), n, t.sortedGeom.as<float>(),
+                                                                              gather_aligned<float, 6>((const float*)src));
     else
-      gather_kernel<float, 3, kGatherPerThread><<<blocks, 256, 0, st>>>((const float*)src, t.sortedIds.as<u32>(), n, t.sortedGeom.as<float>());
+      gather_kernel<float, 3, kGatherPerThread><<<blocks, 256, 0, st>>>((const float*)src, t.sortedIds.as<u32>(), n, t.sortedGeom.as<float>(),
+                                                                              gather_aligned<float, 3>((const float*)src));
   }
   t.image32 = t.boxImage32 = false; // the FP32 filter images follow the geometry
   t.respanned = true;
