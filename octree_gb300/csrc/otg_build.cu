@@ -1241,56 +1241,130 @@ __global__ void __launch_bounds__(256) emit_split_kernel(u32 d, u32 D, const K* 
 }
 
 // ---------------------------------------------------------------- 7. node boxes
-// ot_dynamic_hash_core.h:1425-1450 (children first, then own entities), one depth per launch
+// Minimum and maximum of node geometry: NaN is passed over, as by std::min / std::max of a number and NaN.
+// FP64 values are kept as ordered bits and compared in 32-bit halves: an FP64 compare occupies this GPU's FP64
+// pipe for 16 cycles of an SM, and those would set the time of mbr_level_kernel (8M boxes: 0.32 ms against 0.13).
+template<typename T>
+struct MinMax
+{
+  T v;
+  __device__ __forceinline__ explicit MinMax(T x) : v(x) {}
+  __device__ __forceinline__ void low(T x) { v = smin(v, x); }
+  __device__ __forceinline__ void high(T x) { v = smax(v, x); }
+  __device__ __forceinline__ void low_lane(int o) { v = smin(v, __shfl_xor_sync(0xffffffffu, v, o)); }
+  __device__ __forceinline__ void high_lane(int o) { v = smax(v, __shfl_xor_sync(0xffffffffu, v, o)); }
+  __device__ __forceinline__ T get() const { return v; }
+};
+template<>
+struct MinMax<double>
+{
+  u32 hi, lo; // ordered bits
+  __device__ __forceinline__ explicit MinMax(double x)
+  {
+    const unsigned long long o = ord_bits(x);
+    hi = u32(o >> 32);
+    lo = u32(o);
+  }
+  static __device__ __forceinline__ bool is_nan(double x)
+  {
+    const u32 h = u32(__double2hiint(x)) & 0x7fffffffu;
+    return h > 0x7ff00000u || (h == 0x7ff00000u && __double2loint(x) != 0);
+  }
+  __device__ __forceinline__ void take(u32 h, u32 l, bool yes)
+  {
+    hi = yes ? h : hi;
+    lo = yes ? l : lo;
+  }
+  __device__ __forceinline__ void low(double x)
+  {
+    const MinMax o(x);
+    take(o.hi, o.lo, (o.hi < hi || (o.hi == hi && o.lo < lo)) && !is_nan(x));
+  }
+  __device__ __forceinline__ void high(double x)
+  {
+    const MinMax o(x);
+    take(o.hi, o.lo, (o.hi > hi || (o.hi == hi && o.lo > lo)) && !is_nan(x));
+  }
+  __device__ __forceinline__ void low_lane(int o)
+  {
+    const u32 h = __shfl_xor_sync(0xffffffffu, hi, o), l = __shfl_xor_sync(0xffffffffu, lo, o);
+    take(h, l, h < hi || (h == hi && l < lo));
+  }
+  __device__ __forceinline__ void high_lane(int o)
+  {
+    const u32 h = __shfl_xor_sync(0xffffffffu, hi, o), l = __shfl_xor_sync(0xffffffffu, lo, o);
+    take(h, l, h > hi || (h == hi && l > lo));
+  }
+  __device__ __forceinline__ double get() const { return Ord<double>::val((u64(hi) << 32) | lo); }
+};
+
+// ot_dynamic_hash_core.h:1425-1450 (children first, then own entities), one depth per launch. Eight
+// lanes per node: lane k takes child k and every eighth entity, so that neighbouring lanes read
+// neighbouring boxes, and the eight partial boxes are combined by shuffles (min and max are exact, in
+// any order). One lane per node read its entities one after another, 32 lines per load: 0.70 ms for the 65.8M
+// FP32 boxes of 4096 trees, 0.22 ms for 8M FP64 boxes.
 template<typename T>
 __global__ void __launch_bounds__(256) mbr_level_kernel(u32 d, const u32* __restrict__ levelCount, const uint4* __restrict__ link,
                                                         const T* __restrict__ sortedGeom, T* __restrict__ nodeBox, T* __restrict__ nodeMax)
 {
   u32 begin, cnt;
   level_range(levelCount, d, begin, cnt);
-  for (u32 i = blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += gridDim.x * blockDim.x)
+  const u32 lane8 = threadIdx.x & 7;
+  const u32 groups = (gridDim.x * blockDim.x) >> 3;
+  // whole warps run the same number of rounds: the shuffles below take every lane
+  const u32 rounds = (cnt + groups - 1) / groups;
+  for (u32 r = 0; r < rounds; ++r)
   {
+    const u32 i = r * groups + ((blockIdx.x * blockDim.x + threadIdx.x) >> 3);
     const u32 node = begin + i;
-    const uint4 L = link[node];
-    T mn[3], mx[3];
-#pragma unroll
-    for (int c = 0; c < 3; ++c)
-    {
-      mn[c] = Lim<T>::max();
-      mx[c] = -Lim<T>::max();
-    }
+    bool ok = i < cnt;
+    uint4 L = make_uint4(0u, 0u, 0u, 0u);
+    if (ok)
+      L = link[node];
+    MinMax<T> mn[3] = { MinMax<T>(Lim<T>::max()), MinMax<T>(Lim<T>::max()), MinMax<T>(Lim<T>::max()) };
+    MinMax<T> mx[3] = { MinMax<T>(-Lim<T>::max()), MinMax<T>(-Lim<T>::max()), MinMax<T>(-Lim<T>::max()) };
     const u32 fc = L.x & kFirstChildMask, cc = L.x >> kChildShift;
     if (L.z > L.w || (cc && fc <= node))
-      continue; // malformed link: emission reports capacity errors separately
-    for (u32 k = 0; k < cc; ++k)
+      ok = false; // malformed link: emission reports capacity errors separately
+    if (ok)
     {
-      const T* cb = nodeBox + u64(fc + k) * 6;
-      const T* cm = nodeMax + u64(fc + k) * 3;
+      if (lane8 < cc)
+      {
+        const T* cb = nodeBox + u64(fc + lane8) * 6;
+        const T* cm = nodeMax + u64(fc + lane8) * 3;
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+        {
+          mn[c].low(cb[c]);
+          mx[c].high(cm[c]);
+        }
+      }
+      for (u32 e = L.y + lane8; e < L.z; e += 8)
+      {
+        const T* g = sortedGeom + u64(e) * 6;
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+        {
+          mn[c].low(g[c]);
+          mx[c].high(g[3 + c]);
+        }
+      }
+    }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1)
 #pragma unroll
       for (int c = 0; c < 3; ++c)
       {
-        mn[c] = smin(mn[c], cb[c]);
-        mx[c] = smax(mx[c], cm[c]);
+        mn[c].low_lane(o);
+        mx[c].high_lane(o);
       }
-    }
-    for (u32 e = L.y; e < L.z; ++e)
+    if (ok && lane8 < 3)
     {
-      const T* g = sortedGeom + u64(e) * 6;
-#pragma unroll
-      for (int c = 0; c < 3; ++c)
-      {
-        mn[c] = smin(mn[c], g[c]);
-        mx[c] = smax(mx[c], g[3 + c]);
-      }
-    }
-    T* nb = nodeBox + u64(node) * 6;
-    T* nm = nodeMax + u64(node) * 3;
-#pragma unroll
-    for (int c = 0; c < 3; ++c)
-    {
-      nb[c] = mn[c];
-      nb[3 + c] = mx[c] - mn[c];
-      nm[c] = mx[c];
+      const T lo = lane8 == 0 ? mn[0].get() : lane8 == 1 ? mn[1].get() : mn[2].get();
+      const T hi = lane8 == 0 ? mx[0].get() : lane8 == 1 ? mx[1].get() : mx[2].get();
+      nodeBox[u64(node) * 6 + lane8] = lo;
+      nodeBox[u64(node) * 6 + 3 + lane8] = hi - lo;
+      nodeMax[u64(node) * 3 + lane8] = hi;
     }
   }
 }
@@ -1589,7 +1663,7 @@ static int build_impl(TreeState& t, const T* ent, const void* box, u64 n, cudaSt
   if constexpr (IS_BOX)
   {
     for (int d = int(D); d >= 0; --d)
-      mbr_level_kernel<T><<<emit_blocks(u32(d), 1, emitBlocks, ~u64(0), 256), 256, 0, st>>>(u32(d), t.levelCount.as<u32>(), t.nodeLink.as<uint4>(), t.sortedGeom.as<T>(), t.nodeBox.as<T>(),
+      mbr_level_kernel<T><<<emit_blocks(u32(d), 1, emitBlocks, ~u64(0), 32), 256, 0, st>>>(u32(d), t.levelCount.as<u32>(), t.nodeLink.as<uint4>(), t.sortedGeom.as<T>(), t.nodeBox.as<T>(),
                                                       t.nodeMax.as<T>());
   }
   else
@@ -2081,7 +2155,7 @@ static int forest_build_impl(TreeState& t, const T* ent, const T* boxes, cudaStr
   if constexpr (IS_BOX)
   {
     for (int d = int(Dmax); d >= 0; --d)
-      mbr_level_kernel<T><<<emit_blocks(u32(d), trees, emitBlocks, ~u64(0), 256), 256, 0, st>>>(u32(d), levelCount, t.nodeLink.as<uint4>(), t.sortedGeom.as<T>(), t.nodeBox.as<T>(),
+      mbr_level_kernel<T><<<emit_blocks(u32(d), trees, emitBlocks, ~u64(0), 32), 256, 0, st>>>(u32(d), levelCount, t.nodeLink.as<uint4>(), t.sortedGeom.as<T>(), t.nodeBox.as<T>(),
                                                       t.nodeMax.as<T>());
   }
   else if (boxes)
