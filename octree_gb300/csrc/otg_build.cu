@@ -1376,7 +1376,7 @@ template<typename T>
 __global__ void __launch_bounds__(256) root_box_kernel(const uint4* __restrict__ link, const T* __restrict__ sortedGeom, T* __restrict__ nodeBox,
                                                        Space<T>* spAll)
 {
-  __shared__ T smn[3][256], smx[3][256];
+  __shared__ T smn[3][8], smx[3][8];
   const u32 root = blockIdx.x;
   Space<T>* sp = spAll + root;
   nodeBox += u64(root) * 6;
@@ -1398,33 +1398,35 @@ __global__ void __launch_bounds__(256) root_box_kernel(const uint4* __restrict__
       mx[c] = smax(mx[c], p[c]);
     }
   }
+  // (one thread over 256 partial boxes took 87 us)
 #pragma unroll
   for (int c = 0; c < 3; ++c)
   {
-    smn[c][threadIdx.x] = mn[c];
-    smx[c][threadIdx.x] = mx[c];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+    {
+      mn[c] = smin(mn[c], __shfl_xor_sync(0xffffffffu, mn[c], o));
+      mx[c] = smax(mx[c], __shfl_xor_sync(0xffffffffu, mx[c], o));
+    }
+    if ((threadIdx.x & 31) == 0)
+    {
+      smn[c][threadIdx.x >> 5] = mn[c];
+      smx[c][threadIdx.x >> 5] = mx[c];
+    }
   }
   __syncthreads();
-  if (threadIdx.x == 0)
+  if (threadIdx.x < 3)
   {
-    T bmin[3], bmax[3];
-    for (int c = 0; c < 3; ++c)
+    const int c = threadIdx.x;
+    T bmin = nodeBox[c], bmax = nodeBox[c] + nodeBox[3 + c];
+    for (int w = 0; w < 8; ++w)
     {
-      bmin[c] = nodeBox[c];
-      bmax[c] = nodeBox[c] + nodeBox[3 + c];
+      bmin = smin(bmin, smn[c][w]);
+      bmax = smax(bmax, smx[c][w]);
     }
-    for (int t = 0; t < blockDim.x; ++t)
-      for (int c = 0; c < 3; ++c)
-      {
-        bmin[c] = smin(bmin[c], smn[c][t]);
-        bmax[c] = smax(bmax[c], smx[c][t]);
-      }
-    for (int c = 0; c < 3; ++c)
-    {
-      nodeBox[c] = bmin[c];
-      nodeBox[3 + c] = bmax[c] - bmin[c];
-      sp->nodeSize[0][c] = nodeBox[3 + c];
-    }
+    nodeBox[c] = bmin;
+    nodeBox[3 + c] = bmax - bmin;
+    sp->nodeSize[0][c] = bmax - bmin;
   }
 }
 
@@ -3382,10 +3384,12 @@ static int insert_impl(TreeState& t, const T* pts, u64 n2, cudaStream_t st)
 
   // 6. the new tree
   prof.mark("write", st);
+  // (at least as large as the arrays they replace: a Create sizes its node arrays by a bound, and one that
+  // follows on this tree then finds room and pays no cudaMalloc / cudaFree, 0.67 ms for 4M points)
   DevBuf ids, geom, link, key, box, depth;
-  if ((e = ids.ensure_pooled(sizeof(u32) * nt, st)) || (e = geom.ensure_pooled(sizeof(T) * 3 * nt, st)) ||
-      (e = link.ensure_pooled(sizeof(uint4) * F, st)) || (e = key.ensure_pooled(sizeof(u64) * F, st)) ||
-      (e = box.ensure_pooled(sizeof(T) * 6 * F, st)) || (e = depth.ensure_pooled(F, st)))
+  if ((e = ids.ensure_pooled(std::max(sizeof(u32) * nt, t.sortedIds.bytes), st)) || (e = geom.ensure_pooled(std::max(sizeof(T) * 3 * nt, t.sortedGeom.bytes), st)) ||
+      (e = link.ensure_pooled(std::max(sizeof(uint4) * F, t.nodeLink.bytes), st)) || (e = key.ensure_pooled(std::max(sizeof(u64) * F, t.nodeKey.bytes), st)) ||
+      (e = box.ensure_pooled(std::max(sizeof(T) * 6 * F, t.nodeBox.bytes), st)) || (e = depth.ensure_pooled(std::max(size_t(F), t.nodeDepth.bytes), st)))
     return cuda_status(e, "allocating the inserted tree");
   insert_old_entities_kernel<T><<<blocks_for(n), 256, 0, st>>>(oldOwner.as<u32>(), u32(n), startNew.as<u32>(), t.sortedIds.as<u32>(), t.sortedGeom.as<T>(),
                                                                ids.as<u32>(), geom.as<T>());
