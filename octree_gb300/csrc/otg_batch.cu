@@ -350,8 +350,11 @@ struct BatchArgs
 
 constexpr u32 kCandBuf = 64;
 
+// Rays on FP64 trees take 94 registers by themselves, which leaves 16 warps per SM; 32 are asked for (64 registers, a
+// few spills on the exact path): 30k rays through 1M FP64 boxes 0.53 ms, now 0.44; 40 warps give 0.52. The other
+// kinds take what they need: bounds of 8, 40 or 48 warps made them 3 to 30% slower.
 template<typename T, int KIND, int WARPS>
-__global__ void __launch_bounds__(WARPS * 32) batch_query_kernel(BatchArgs<T, KIND> a)
+__global__ void __launch_bounds__(WARPS * 32, KIND == kRayAll && sizeof(T) == 8 ? 32 / WARPS : 0) batch_query_kernel(BatchArgs<T, KIND> a)
 {
   static_assert(KIND >= kRange && KIND <= kPick, "every query kind has its own setup, node test and entity test below");
   using G = GeoD<T>;
@@ -364,6 +367,7 @@ __global__ void __launch_bounds__(WARPS * 32) batch_query_kernel(BatchArgs<T, KI
   __shared__ RayF32 rayF[kRayPre ? WARPS : 1];
   __shared__ u32 candMem[kRayPre ? WARPS : 1][kRayPre ? kCandBuf : 1];
   __shared__ RangeF32 rangeF[kRangeF32 ? WARPS : 1];
+  __shared__ u32 runMem[WARPS][3][32]; // flat runs: entity bases, child bases, child runs' lanes
   __shared__ u32 stackMem[WARPS][kWideStack];
   __shared__ u64 itemMem[WARPS][kItemBuf];
   __shared__ double distMem[KIND == kRayAll ? WARPS : 1][KIND == kRayAll ? kItemBuf : 1];
@@ -776,10 +780,15 @@ __global__ void __launch_bounds__(WARPS * 32) batch_query_kernel(BatchArgs<T, KI
         }
       }
       const bool tests = act && !whole;
-      // entities of the popped nodes
+      // The entities and the children of the popped nodes as flat runs: the items of the lanes before (excl),
+      // of both kinds from one scan where the counts fit one word (23 and 9 bits), and for the r-th lane
+      // that has any, its first item minus its place in the flat order, in shared memory.
+      const u32 cntE = tests ? L.z - L.y : 0u;
+      const u32 cntC = (tests || expand) ? (L.x >> kChildShift) : 0u;
+      u32 inclE = cntE, inclC = cntC;
+      if (!__any_sync(~0u, cntE >= (1u << 17)))
       {
-        const u32 cnt = tests ? L.z - L.y : 0u;
-        u32 incl = cnt;
+        u32 incl = cntE | (cntC << 23);
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1)
         {
@@ -787,14 +796,58 @@ __global__ void __launch_bounds__(WARPS * 32) batch_query_kernel(BatchArgs<T, KI
           if (lane >= u32(o))
             incl += y;
         }
-        const u32 total = __shfl_sync(~0u, incl, 31);
+        inclE = incl & ((1u << 23) - 1);
+        inclC = incl >> 23;
+      }
+      else
+      {
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1)
+        {
+          const u32 y = __shfl_up_sync(~0u, inclE, o), z = __shfl_up_sync(~0u, inclC, o);
+          if (lane >= u32(o))
+          {
+            inclE += y;
+            inclC += z;
+          }
+        }
+      }
+      const u32 totalE = __shfl_sync(~0u, inclE, 31), totalC = __shfl_sync(~0u, inclC, 31);
+      const u32 exclE = inclE - cntE, exclC = inclC - cntC;
+      const u32 lt = (1u << lane) - 1u;
+      {
+        const u32 nzE = __ballot_sync(~0u, cntE != 0u), nzC = __ballot_sync(~0u, cntC != 0u);
+        if (cntE)
+          runMem[w][0][__popc(nzE & lt)] = L.y - exclE;
+        if (cntC)
+        {
+          runMem[w][1][__popc(nzC & lt)] = (L.x & kFirstChildMask) - exclC;
+          runMem[w][2][__popc(nzC & lt)] = lane;
+        }
+        __syncwarp();
+      }
+      // The run of item f0 + lane (`before`: the runs that start before f0): the runs that start in the window
+      // of 32 items up to it, by one reduction and a population count. A binary search over the lanes'
+      // sums takes five dependent shuffles: 10k ranges on 1M FP64 points 54 us, now 48; 1M ranges and 1M rays
+      // on 4096 FP32 trees 1.49 and 2.12 ms, now 1.38 and 1.95.
+      auto flat_run = [&](u32 excl, u32 cnt, u32 f0, u32& before) -> u32 {
+        const u32 at = excl - f0;
+        const u32 starts = __reduce_or_sync(~0u, (cnt && at < 32u) ? 1u << at : 0u);
+        const u32 run = before + __popc(starts & (lt | (1u << lane))) - 1u;
+        before += __popc(starts);
+        return run;
+      };
+      const u32 expandMask = kWhole ? __ballot_sync(~0u, expand) : 0u;
+      // entities of the popped nodes
+      {
+        const u32 total = totalE;
+        u32 before = 0;
         for (u32 f0 = 0; f0 < total; f0 += 32)
         {
           const u32 f = f0 + lane;
-          const u32 o = owner(incl, min(f, total - 1));
-          const u32 oy = __shfl_sync(~0u, L.y, o), oex = __shfl_sync(~0u, incl - cnt, o);
+          const u32 run = flat_run(exclE, cntE, f0, before);
+          const u32 e = runMem[w][0][run] + f;
           const bool v = f < total;
-          const u32 e = oy + (f - oex);
           bool hit = false;
           double d = 0.0;
           if constexpr (kRayPre)
@@ -901,26 +954,18 @@ __global__ void __launch_bounds__(WARPS * 32) batch_query_kernel(BatchArgs<T, KI
       }
       // children of the popped nodes, tested before they are pushed
       {
-        const u32 cnt = (tests || expand) ? (L.x >> kChildShift) : 0u;
-        u32 incl = cnt;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1)
-        {
-          const u32 y = __shfl_up_sync(~0u, incl, o);
-          if (lane >= u32(o))
-            incl += y;
-        }
-        const u32 total = __shfl_sync(~0u, incl, 31);
+        const u32 total = totalC;
+        u32 before = 0;
         for (u32 f0 = 0; f0 < total; f0 += 32)
         {
           const u32 f = f0 + lane;
-          const u32 o = owner(incl, min(f, total - 1));
-          const u32 ofc = __shfl_sync(~0u, L.x & kFirstChildMask, o), oex = __shfl_sync(~0u, incl - cnt, o);
+          const u32 run = flat_run(exclC, cntC, f0, before);
           bool keep = false, contained = false;
-          const u32 child = ofc + (f - oex);
+          const u32 child = runMem[w][1][run] + f;
           bool free = false; // a contained node's child
           if constexpr (kWhole)
-            free = __shfl_sync(~0u, expand, o);
+            if (expandMask)
+              free = (expandMask >> runMem[w][2][run]) & 1u;
           if (f < total)
           {
             keep = contained = free;
