@@ -100,12 +100,25 @@ constexpr int kRange = 0, kFrustum = 1, kRayAll = 2, kPlane = 3, kPlanePositive 
 //     and the root box's coordinates, so also every node's). RN is monotone, so maxL + tol <= nmin
 //     gives maxL <= RN(nmin - tol); and nmin + g/2 < maxL + tol gives RN(nmin - tol) < maxL.
 // Undecided tests run in FP64, so every answer is the FP64 answer.
+//
+// Box trees. A node's image holds the exact MBR max where the tests use maxR = RN(nmin + nsize), within the
+// slack g of it: their P and Q thresholds are widened by g. An entity's image holds lo = rd(bmin) and
+// hi = ru(bmax), so bmin lies in [lo, succ(lo)) and bmax in (pred(hi), hi], and its test is decided by four
+// thresholds per dimension (e0 .. e3, boxes that lie in the root box, tol >= 0):
+//   inside (rmin <= bmin, bmax <= rmax and both on the other side too, contains_box_no_tol), with
+//     e0 = rd(rmin), e1 = ru(rmin), e2 = rd(rmax), e3 = ru(rmax):
+//     in  if e1 <= lo < e2 and e1 < hi <= e2 in every dimension; out if lo or hi < e0 or > e3 in some dimension
+//   overlap (GetBoxRelation == Overlapped), with e0 = rd(rmin - tol - g), e1 = ru(rmin + tol),
+//     e2 = rd(rmax - tol - g), e3 = ru(rmax + tol + g):
+//     in  if hi > e1 and lo < e2 in every dimension (its "overlapped" branch); out if hi < e0 or lo > e3 in some
+//     dimension (then "separated" or "adjacent")
 struct RangeF32
 {
   float w[3], s[3], plo[3], phi[3], qlo[3], qhi[3];
+  float e0[3], e1[3], e2[3], e3[3]; // box entities
 };
 
-__device__ __forceinline__ void range_thresholds(const double* r, const double* rsize, const double* rootBox, double tol, RangeF32& f)
+__device__ __forceinline__ void range_thresholds(const double* r, const double* rsize, const double* rootBox, double tol, bool isBox, int mode, RangeF32& f)
 {
   double M = 0.0;
 #pragma unroll
@@ -123,10 +136,16 @@ __device__ __forceinline__ void range_thresholds(const double* r, const double* 
     const double W = maxL + tol;
     f.w[d] = __double2float_ru(W + g);
     f.s[d] = __double2float_rd(W - g);
-    f.plo[d] = __double2float_rd(P);
-    f.phi[d] = __double2float_ru(P);
-    f.qlo[d] = __double2float_rd(Q);
-    f.qhi[d] = __double2float_ru(Q);
+    const double wide = isBox ? g : 0.0;
+    f.plo[d] = __double2float_rd(P - wide);
+    f.phi[d] = __double2float_ru(P + wide);
+    f.qlo[d] = __double2float_rd(Q - wide);
+    f.qhi[d] = __double2float_ru(Q + wide);
+    const bool over = mode == OTG_RANGE_OVERLAP;
+    f.e0[d] = __double2float_rd(over ? r[d] - tol - g : r[d]);
+    f.e1[d] = __double2float_ru(over ? r[d] + tol : r[d]);
+    f.e2[d] = __double2float_rd(over ? r[3 + d] - tol - g : r[3 + d]);
+    f.e3[d] = __double2float_ru(over ? r[3 + d] + tol + g : r[3 + d]);
   }
 }
 
@@ -170,9 +189,10 @@ struct RangeQ
   RangeF32 f;
   u32 flags, pad;
 };
-static_assert(sizeof(RangeQ) == 80, "RangeQ: 20 words");
+constexpr u32 kRangeWords = 30; // of the thresholds
+static_assert(sizeof(RangeQ) == 128, "RangeQ: 32 words");
 
-__global__ void __launch_bounds__(128) range_prepare_kernel(TreeView<double> tv, const double* __restrict__ ranges, u32 nq, double tol,
+__global__ void __launch_bounds__(128) range_prepare_kernel(TreeView<double> tv, const double* __restrict__ ranges, u32 nq, int mode, double tol,
                                                             RangeQ* __restrict__ out)
 {
   using G = GeoD<double>;
@@ -196,7 +216,7 @@ __global__ void __launch_bounds__(128) range_prepare_kernel(TreeView<double> tv,
       vol *= rsize[c];
     if (vol <= 0.0)
       o.flags |= kRangeEmpty;
-    range_thresholds(r, rsize, nb, tol, o.f);
+    range_thresholds(r, rsize, nb, tol, tv.isBox != 0, mode, o.f);
     o.pad = 0;
     out[q] = o;
   }
@@ -218,6 +238,103 @@ __device__ __forceinline__ void range_node_f32(const float4* __restrict__ img, u
   }
   enter = anyPrune ? 0 : (allKeep ? 1 : 2);
   inside = anyOut ? 0 : (allIn ? 1 : 2);
+}
+
+// box entity: 0 out, 1 in, 2 undecided
+__device__ __forceinline__ int range_box_f32(const float4* __restrict__ img, u32 e, const RangeF32& f, bool over)
+{
+  const float4 mn = img[2 * size_t(e)], mx = img[2 * size_t(e) + 1];
+  const float lo[3] = { mn.x, mn.y, mn.z }, hi[3] = { mx.x, mx.y, mx.z };
+  bool allIn = true, anyOut = false;
+#pragma unroll
+  for (int d = 0; d < 3; ++d)
+  {
+    if (over)
+    {
+      allIn &= (hi[d] > f.e1[d]) & (lo[d] < f.e2[d]);
+      anyOut |= (hi[d] < f.e0[d]) | (lo[d] > f.e3[d]);
+    }
+    else
+    {
+      allIn &= (f.e1[d] <= lo[d]) & (lo[d] < f.e2[d]) & (f.e1[d] < hi[d]) & (hi[d] <= f.e2[d]);
+      anyOut |= (lo[d] < f.e0[d]) | (hi[d] < f.e0[d]) | (lo[d] > f.e3[d]) | (hi[d] > f.e3[d]);
+    }
+  }
+  return anyOut ? 0 : (allIn ? 1 : 2);
+}
+__device__ __noinline__ bool range_box_fp64(const double* q, const double* box, int mode, double tol)
+{
+  double r[6], rsize[3], b[6];
+  range_load(q, r, rsize);
+  load_box(box, b);
+  return mode == OTG_RANGE_OVERLAP ? GeoD<double>::box_relation(r, b, tol) == -1 : GeoD<double>::contains_box_no_tol(r, b);
+}
+
+// ---- FP32 pre-tests of PickSearch on FP64 trees. A node or box holds the point p if
+// min - tol < p < max + tol in every dimension (node_contains_point compares |p - min - half| with half + tol,
+// box_contains_point the two sides; with tol = 0 the sides belong to it), up to roundings far below
+// g = 2^-46 (M + tol), M bounding the point's and the root box's coordinates:
+//   in  if lo < rd(p + tol - g) and hi > ru(p - tol + g) in every dimension
+//   out if lo > ru(p + tol + g) or hi < rd(p - tol - g) in some dimension
+// A point entity equals p within tol only if it is not out (lo = hi = its image, RN).
+struct PickF32
+{
+  float inLo[3], inHi[3], outLo[3], outHi[3];
+};
+struct PickQ
+{
+  PickF32 f;
+  u32 skip, pad[3]; // skip: outside the tree's box (:430-431)
+};
+static_assert(sizeof(PickQ) == 64, "PickQ: 16 words");
+
+__global__ void __launch_bounds__(128) pick_prepare_kernel(TreeView<double> tv, const double* __restrict__ pts, u32 nq, double tol, PickQ* __restrict__ out)
+{
+  for (u32 q = blockIdx.x * blockDim.x + threadIdx.x; q < nq; q += gridDim.x * blockDim.x)
+  {
+    const double* nb = tv.nodeBox + u64(query_root(tv, q)) * 6;
+    double rb[6], p[3];
+    double M = 0.0;
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+    {
+      rb[c] = nb[c];
+      rb[3 + c] = nb[c] + nb[3 + c];
+      p[c] = pts[u64(q) * 3 + c];
+      M = fmax(M, fmax(fabs(p[c]), fmax(fabs(rb[c]), fabs(rb[3 + c]))));
+    }
+    const double g = (M + fabs(tol)) * 0x1p-46;
+    PickQ o;
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+    {
+      o.f.inLo[c] = __double2float_rd(p[c] + tol - g);
+      o.f.inHi[c] = __double2float_ru(p[c] - tol + g);
+      o.f.outLo[c] = __double2float_ru(p[c] + tol + g);
+      o.f.outHi[c] = __double2float_rd(p[c] - tol - g);
+    }
+    o.skip = GeoD<double>::box_contains_point(rb, p, tol) ? 0u : 1u;
+    o.pad[0] = o.pad[1] = o.pad[2] = 0;
+    out[q] = o;
+  }
+}
+// 0 out, 1 in, 2 undecided
+__device__ __forceinline__ int pick_f32(float4 mn, float4 mx, const PickF32& f)
+{
+  const float lo[3] = { mn.x, mn.y, mn.z }, hi[3] = { mx.x, mx.y, mx.z };
+  bool allIn = true, anyOut = false;
+#pragma unroll
+  for (int d = 0; d < 3; ++d)
+  {
+    allIn &= (lo[d] < f.inLo[d]) & (hi[d] > f.inHi[d]);
+    anyOut |= (lo[d] > f.outLo[d]) | (hi[d] < f.outHi[d]);
+  }
+  return anyOut ? 0 : (allIn ? 1 : 2);
+}
+__device__ __noinline__ bool pick_node_fp64(const double* nb, const double* p, double tol) { return GeoD<double>::node_contains_point(nb, nb + 3, p, tol); }
+__device__ __noinline__ bool pick_entity_fp64(const double* g, int isBox, const double* p, double tol)
+{
+  return isBox ? GeoD<double>::box_contains_point(g, p, tol) : GeoD<double>::points_equal(g, p, tol);
 }
 
 // point: 0 outside, 1 inside, 2 undecided (also for a point without a finite image)
@@ -340,9 +457,9 @@ struct BatchArgs
   int phase;          // 0: whole queries; 1: top levels, deeper subtrees become items; 2: the items
   u32 splitCap;       // item capacity of the work buffer
   u32 splitDepth;     // depth of the subtrees that become items
-  // range on FP64 point trees: one RangeQ per query (FP32 pre-tests); set only where out.count has
-  // three slots (the item count, then the pre-tests and the undecided ones, added at the end).
-  // Rays on FP64 box trees with FP32 images: one RayPrep per query.
+  // FP64 trees with FP32 images, one record per query of its setup. Ranges: RangeQ; set only where
+  // out.count has three slots (the item count, then the pre-tests and the undecided ones, added at the
+  // end). Rays on box trees: RayPrep. Picks: PickQ.
   const void* prep = nullptr;
   float tolUp = 0.f, tolIncUp = 0.f; // tol and tolInc rounded up (rays)
   bool planeF32 = false;             // FP32 plane tests: images (FP64 trees), entities in their nodes
@@ -360,6 +477,8 @@ __global__ void __launch_bounds__(WARPS * 32, KIND == kRayAll && sizeof(T) == 8 
   using G = GeoD<T>;
   constexpr bool kRangeF32 = KIND == kRange && sizeof(T) == 8;
   constexpr bool kRayPre = KIND == kRayAll && sizeof(T) == 8;
+  constexpr bool kPickPre = KIND == kPick && sizeof(T) == 8;
+  __shared__ PickF32 pickF[kPickPre ? WARPS : 1];
   constexpr bool kPlanes = KIND == kFrustum || KIND == kPlane || KIND == kPlanePositive;
   // kinds that take whole subtrees untested
   constexpr bool kWhole = KIND == kRange || KIND == kPlanePositive || KIND == kFrustum;
@@ -418,9 +537,9 @@ __global__ void __launch_bounds__(WARPS * 32, KIND == kRayAll && sizeof(T) == 8 
         // the query's prepared thresholds into the warp's shared copy, its flags to every lane
         const u32* src = reinterpret_cast<const u32*>(static_cast<const RangeQ*>(a.prep) + q);
         __syncwarp(); // the previous query's thresholds are read by every lane before they change
-        if (lane < 18)
+        if (lane < kRangeWords)
           reinterpret_cast<u32*>(&rangeF[w])[lane] = src[lane];
-        const u32 flags = src[18];
+        const u32 flags = src[kRangeWords];
         __syncwarp();
         useF32 = true;
         if (a.phase != 2 && (flags & kRangeAll))
@@ -485,7 +604,19 @@ __global__ void __launch_bounds__(WARPS * 32, KIND == kRayAll && sizeof(T) == 8 
     else if constexpr (KIND == kPick)
     {
       pl = a.q + u64(q) * 3; // the point
-      if (a.phase != 2)
+      bool made = false;
+      if constexpr (kPickPre)
+        if (a.prep)
+        {
+          const u32* src = reinterpret_cast<const u32*>(static_cast<const PickQ*>(a.prep) + q);
+          __syncwarp(); // the previous query's thresholds are read by every lane before they change
+          if (lane < 12)
+            reinterpret_cast<u32*>(&pickF[w])[lane] = src[lane];
+          skip = a.phase != 2 && src[12] != 0;
+          __syncwarp();
+          made = true;
+        }
+      if (!made && a.phase != 2)
       {
         T rb[6];
 #pragma unroll
@@ -654,7 +785,19 @@ __global__ void __launch_bounds__(WARPS * 32, KIND == kRayAll && sizeof(T) == 8 
       else if constexpr (KIND == kQuery)
         return cond_combine(a.qp, q, a.err, [&](const QueryCond& c) { return cond_node(a.qp, c, nb, a.tol); });
       else if constexpr (KIND == kPick)
+      {
+        if constexpr (kPickPre)
+        {
+          if (a.prep)
+          {
+            const int dec = pick_f32(tv.nodeImg[2 * size_t(node)], tv.nodeImg[2 * size_t(node) + 1], pickF[w]);
+            if (dec != 2)
+              return dec == 1;
+          }
+          return pick_node_fp64(nb, pl, a.tol);
+        }
         return G::node_contains_point(nb, nb + 3, pl, a.tol);
+      }
       else if constexpr (KIND == kRayAll)
       {
         T en, ex;
@@ -886,6 +1029,20 @@ __global__ void __launch_bounds__(WARPS * 32, KIND == kRayAll && sizeof(T) == 8 
                     hit = G::box_contains_point(r, tv.geom + u64(e) * 3, a.tol);
                 }
               }
+              else if (kRangeF32)
+              {
+                if constexpr (kRangeF32)
+                {
+                  int dec = 2;
+                  if (useF32)
+                  {
+                    dec = range_box_f32(tv.boxImg, e, rangeF[w], a.mode == OTG_RANGE_OVERLAP);
+                    ++f32Tests;
+                    f32Undecided += dec == 2 ? 1u : 0u;
+                  }
+                  hit = dec == 2 ? range_box_fp64(a.q + u64(q) * 6, tv.geom + u64(e) * 6, a.mode, a.tol) : dec == 1;
+                }
+              }
               else
               {
                 T bx[6];
@@ -938,6 +1095,25 @@ __global__ void __launch_bounds__(WARPS * 32, KIND == kRayAll && sizeof(T) == 8 
             {
               const T* g = tv.geom + u64(e) * (tv.isBox ? 6 : 3);
               hit = cond_combine(a.qp, q, a.err, [&](const QueryCond& c) { return cond_entity(a.qp, c, g, tv.isBox != 0, a.tol); });
+            }
+            else if constexpr (kPickPre)
+            {
+              int dec = 2;
+              if (a.prep)
+              {
+                float4 lo, hi;
+                if (tv.isBox)
+                {
+                  lo = tv.boxImg[2 * size_t(e)];
+                  hi = tv.boxImg[2 * size_t(e) + 1];
+                }
+                else
+                  lo = hi = tv.pointImg[e];
+                dec = pick_f32(lo, hi, pickF[w]);
+                if (!tv.isBox) // a point within reach is tested exactly, and so is one without a finite image
+                  dec = dec != 0 || !(lo.w < INFINITY) ? 2 : 0;
+              }
+              hit = dec == 2 ? pick_entity_fp64(tv.geom + u64(e) * (tv.isBox ? 6 : 3), tv.isBox, pl, a.tol) : dec == 1;
             }
             else if constexpr (KIND == kPick)
               hit = tv.isBox ? G::box_contains_point(tv.geom + u64(e) * 6, pl, a.tol) : G::points_equal(tv.geom + u64(e) * 3, pl, a.tol);
@@ -1096,12 +1272,12 @@ int batch_range(const TreeView<T>& tv, const T* ranges, u32 nq, int mode, T tol,
   TmpBuf prep;
   if constexpr (sizeof(T) == 8)
   {
-    // FP64 point trees with FP32 images: the per-query setup by one thread per query
-    if (tv.nodeImg && tv.pointImg && !tv.isBox && nq)
+    // FP64 trees with FP32 images: the per-query setup by one thread per query
+    if (tv.nodeImg && (tv.isBox ? tv.boxImg && tv.inNodes && tol >= T(0) : tv.pointImg != nullptr) && nq)
     {
       if (cudaError_t e = prep.ensure(sizeof(RangeQ) * nq, st))
         return cuda_status(e, "allocating the range setup");
-      range_prepare_kernel<<<u32((nq + 127) / 128), 128, 0, st>>>(tv, ranges, nq, double(tol), prep.as<RangeQ>());
+      range_prepare_kernel<<<u32((nq + 127) / 128), 128, 0, st>>>(tv, ranges, nq, mode, double(tol), prep.as<RangeQ>());
       a.prep = prep.p;
     }
   }
@@ -1145,7 +1321,19 @@ int batch_query_program(const TreeView<T>& tv, const QueryProgram<T>& qp, u32 nq
 template<typename T>
 int batch_pick(const TreeView<T>& tv, const T* pts, u32 nq, T tol, Appender out, u32* work, u32* err, cudaStream_t st, int shape, size_t workBytes)
 {
-  return launch_batch<T, kPick>(BatchArgs<T, kPick>{ tv, pts, 0, nq, 0, tol, T(0), T(0), out, work, err }, shape, st, workBytes);
+  BatchArgs<T, kPick> a{ tv, pts, 0, nq, 0, tol, T(0), T(0), out, work, err };
+  TmpBuf prep;
+  if constexpr (sizeof(T) == 8)
+  {
+    if (tv.nodeImg && (tv.isBox ? tv.boxImg : tv.pointImg) && tv.inNodes && tol >= T(0) && nq)
+    {
+      if (cudaError_t e = prep.ensure(sizeof(PickQ) * nq, st))
+        return cuda_status(e, "allocating the pick setup");
+      pick_prepare_kernel<<<u32((nq + 127) / 128), 128, 0, st>>>(tv, pts, nq, double(tol), prep.as<PickQ>());
+      a.prep = prep.p;
+    }
+  }
+  return launch_batch<T, kPick>(a, shape, st, workBytes);
 }
 template<typename T>
 int batch_ray_all(const TreeView<T>& tv, const T* rays, u32 nq, T tol, T tolInc, T maxDist, Appender out, u32* work, u32* err, cudaStream_t st,

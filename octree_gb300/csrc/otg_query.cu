@@ -1474,6 +1474,10 @@ static int range_impl(const TreeState& t, const void* ranges, u64 nq, int mode, 
     tv.nodeImg = t.nodeBox32.as<float4>();
     tv.pointImg = t.geom32.as<float4>();
   }
+  if constexpr (sizeof(T) == 8)
+    if (algo != OTG_ALGO_PLAIN_FP64 && tv.isBox)
+      if (int rci = use_images(const_cast<TreeState&>(t), tv, nq * 128, st))
+        return rci;
   TmpBuf work;
   if (cudaError_t e = work.ensure(batch_work_bytes(nq), st))
     return cuda_status(e, "allocating the work counter");
@@ -1517,6 +1521,10 @@ static int pick_impl(const TreeState& t, const void* pts, u64 nq, double tol, in
   Collected c;
   auto tv = view<T>(t, qTree);
   T tl = tol_of<T>(tol);
+  if constexpr (sizeof(T) == 8)
+    if (algo != OTG_ALGO_PLAIN_FP64)
+      if (int rci = use_images(const_cast<TreeState&>(t), tv, nq * 64, st))
+        return rci;
   TmpBuf work;
   if (cudaError_t e = work.ensure(batch_work_bytes(nq), st))
     return cuda_status(e, "allocating the work counter");
