@@ -1221,7 +1221,7 @@ static int launch_batch_w(const BatchArgs<T, KIND>& a, cudaStream_t st)
     e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (!e)
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, batch_query_kernel<T, KIND, WARPS>, WARPS * 32, 0);
-  if (!e)
+  if (!e && !a.out.cleared)
     e = cudaMemsetAsync(a.work, 0, 16, st);
   if (e)
     return cuda_status(e, "configuring the batched query kernel");

@@ -2318,11 +2318,24 @@ int finish_build(TreeState& t, cudaStream_t st)
     return OTG_OK;
   u32 hostErr = 0;
   std::vector<u32> lc(32, 0);
-  cudaError_t e = cudaMemcpyAsync(&hostErr, t.err.p, sizeof(u32), cudaMemcpyDeviceToHost, st);
-  if (!e && (t.n || t.trees))
-    e = cudaMemcpyAsync(lc.data(), t.levelCount.p, sizeof(u32) * 32, cudaMemcpyDeviceToHost, st);
-  if (!e)
-    e = cudaStreamSynchronize(st);
+  cudaError_t e;
+  {
+    HostBlock b;
+    u32 plain[33] = {};
+    u32* h = b.p ? static_cast<u32*>(b.p) : plain;
+    e = cudaMemcpyAsync(h, t.err.p, sizeof(u32), cudaMemcpyDeviceToHost, st);
+    if (!e && (t.n || t.trees))
+      e = cudaMemcpyAsync(h + 1, t.levelCount.p, sizeof(u32) * 32, cudaMemcpyDeviceToHost, st);
+    const cudaError_t w = cudaStreamSynchronize(st);
+    if (!e)
+      e = w;
+    if (!e)
+    {
+      hostErr = h[0];
+      if (t.n || t.trees)
+        lc.assign(h + 1, h + 33);
+    }
+  }
   if (e)
     return cuda_status(e, "finishing build");
   if (hostErr & kErrTimeout)
@@ -3176,12 +3189,7 @@ static int insert_impl(TreeState& t, const T* pts, u64 n2, cudaStream_t st)
   cudaError_t e;
   u32 hostErr = 0;
   auto read_err = [&](const char* what) -> int {
-    cudaError_t ce = cudaMemcpyAsync(&hostErr, err, sizeof(u32), cudaMemcpyDeviceToHost, st);
-    if (!ce)
-      ce = cudaStreamSynchronize(st);
-    if (ce)
-      return cuda_status(ce, what);
-    return OTG_OK;
+    return cuda_status(read_back(&hostErr, err, sizeof(u32), st), what);
   };
   // counts read back by the host: [0] clusters, [1] distinct keys, [2] new branch nodes, [3] spare
   u32* hostCounts = nullptr;
@@ -3192,10 +3200,7 @@ static int insert_impl(TreeState& t, const T* pts, u64 n2, cudaStream_t st)
   u32 hc[4] = { 0, 0, 0, 0 };
   (void)hostCounts;
   auto read_count = [&](int i, const char* what) -> int {
-    cudaError_t ce = cudaMemcpyAsync(&hc[i], dCounts + i, sizeof(u32), cudaMemcpyDeviceToHost, st);
-    if (!ce)
-      ce = cudaStreamSynchronize(st);
-    return ce ? cuda_status(ce, what) : OTG_OK;
+    return cuda_status(read_back(&hc[i], dCounts + i, sizeof(u32), st), what);
   };
   Profiler& prof = profiler();
   prof.reset();
@@ -3400,7 +3405,7 @@ static int insert_impl(TreeState& t, const T* pts, u64 n2, cudaStream_t st)
                                                         key.as<u64>(), box.as<T>(), depth.as<unsigned char>());
   prof.mark("end", st);
   std::vector<u32> dc(64);
-  if ((e = cudaGetLastError()) || (e = cudaMemcpyAsync(dc.data(), depthCount.p, sizeof(u32) * 64, cudaMemcpyDeviceToHost, st)))
+  if ((e = cudaGetLastError()) || (e = read_back(dc.data(), depthCount.p, sizeof(u32) * 64, st)))
     return cuda_status(e, "inserting points");
   if (int rc = read_err("inserting points"))
     return rc;
@@ -3468,7 +3473,7 @@ int insert_points(TreeState& t, const void* entities, u64 n2, int mem, cudaStrea
     // a point outside a given space has the location key 0 and sorts first; the reference keeps it
     // in a node that the root does not link
     u64 first = 0;
-    if ((e = cudaMemcpyAsync(&first, t.sortedKeys, t.keys32 ? 4 : 8, cudaMemcpyDeviceToHost, st)) || (e = cudaStreamSynchronize(st)))
+    if ((e = read_back(&first, t.sortedKeys, t.keys32 ? 4 : 8, st)))
       return cuda_status(e, "reading the first location");
     if (first == 0)
     {

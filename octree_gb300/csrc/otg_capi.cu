@@ -41,6 +41,59 @@ void keep_pool_memory(int device)
   done[device] = true;
 }
 
+// blocks not in use (a lost cudaHostAlloc leaves p null: the copies then go to pageable memory)
+static std::mutex g_hostBlocksLock;
+static std::vector<void*>& host_blocks()
+{
+  static auto* v = new std::vector<void*>(); // outlives every thread
+  return *v;
+}
+HostBlock::HostBlock() : p(nullptr)
+{
+  {
+    std::lock_guard<std::mutex> g(g_hostBlocksLock);
+    auto& v = host_blocks();
+    if (!v.empty())
+    {
+      p = v.back();
+      v.pop_back();
+      return;
+    }
+  }
+  if (cudaHostAlloc(&p, kBytes, cudaHostAllocPortable) != cudaSuccess)
+  {
+    cudaGetLastError();
+    p = nullptr;
+  }
+}
+HostBlock::~HostBlock()
+{
+  if (!p)
+    return;
+  {
+    std::lock_guard<std::mutex> g(g_hostBlocksLock);
+    auto& v = host_blocks();
+    if (v.size() < size_t(kKept))
+    {
+      v.push_back(p);
+      return;
+    }
+  }
+  cudaFreeHost(p);
+}
+cudaError_t read_back(void* dst, const void* dev, size_t bytes, cudaStream_t st)
+{
+  HostBlock b;
+  const bool pinned = b.p && bytes <= HostBlock::kBytes;
+  cudaError_t e = cudaMemcpyAsync(pinned ? b.p : dst, dev, bytes, cudaMemcpyDeviceToHost, st);
+  const cudaError_t w = cudaStreamSynchronize(st); // also after an error: the block may still be written
+  if (!e)
+    e = w;
+  if (!e && pinned)
+    std::memcpy(dst, b.p, bytes);
+  return e;
+}
+
 int cuda_status(cudaError_t e, const char* what)
 {
   if (e == cudaSuccess)
@@ -647,13 +700,49 @@ extern "C"
       return OTG_ERR_INVALID_ARGUMENT;
     cudaStream_t st = (cudaStream_t)stream;
     cudaMemcpyKind kind = mem == OTG_MEM_HOST ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice;
+    struct Part
+    {
+      void* dst;
+      const void* src;
+      size_t bytes;
+    };
+    const bool dist = distances && r->s.hasDist;
+    const Part parts[3] = { { offsets, r->s.offsets.p, offsets ? sizeof(uint64_t) * (r->s.nq + 1) : 0 },
+                            { ids, r->s.ids.p, ids ? sizeof(uint32_t) * r->s.nids : 0 },
+                            { distances, r->s.dist.p, dist ? sizeof(double) * r->s.nids : 0 } };
     cudaError_t e = cudaSuccess;
-    if (offsets)
-      e = cudaMemcpyAsync(offsets, r->s.offsets.p, sizeof(uint64_t) * (r->s.nq + 1), kind, st);
-    if (!e && ids && r->s.nids)
-      e = cudaMemcpyAsync(ids, r->s.ids.p, sizeof(uint32_t) * r->s.nids, kind, st);
-    if (!e && distances && r->s.hasDist && r->s.nids)
-      e = cudaMemcpyAsync(distances, r->s.dist.p, sizeof(double) * r->s.nids, kind, st);
+    const size_t total = parts[0].bytes + parts[1].bytes + parts[2].bytes;
+    if (mem == OTG_MEM_HOST && total <= HostBlock::kBytes)
+    {
+      // a small result: its arrays side by side into pinned memory, one wait
+      HostBlock b;
+      if (b.p)
+      {
+        unsigned char* at = static_cast<unsigned char*>(b.p);
+        for (const Part& p : parts)
+          if (p.bytes)
+          {
+            if (!e)
+              e = cudaMemcpyAsync(at, p.src, p.bytes, kind, st);
+            at += p.bytes;
+          }
+        const cudaError_t w = cudaStreamSynchronize(st);
+        if (!e)
+          e = w;
+        at = static_cast<unsigned char*>(b.p);
+        if (!e)
+          for (const Part& p : parts)
+            if (p.bytes)
+            {
+              std::memcpy(p.dst, at, p.bytes);
+              at += p.bytes;
+            }
+        return cuda_status(e, "copying result");
+      }
+    }
+    for (const Part& p : parts)
+      if (p.bytes && !e)
+        e = cudaMemcpyAsync(p.dst, p.src, p.bytes, kind, st);
     if (!e && mem == OTG_MEM_HOST)
       e = cudaStreamSynchronize(st);
     return cuda_status(e, "copying result");

@@ -450,10 +450,7 @@ int collide_search_filtered(TreeState& A, TreeState& B, bool self, double tol, A
 int collide_search_stats(const CollideSearch& s, u64& tests, u64& rechecks, cudaStream_t st)
 {
   CollideCounters h{};
-  cudaError_t e = cudaMemcpyAsync(&h, s.ctr.p, sizeof(h), cudaMemcpyDeviceToHost, st);
-  if (!e)
-    e = cudaStreamSynchronize(st);
-  if (e)
+  if (cudaError_t e = read_back(&h, s.ctr.p, sizeof(h), st))
     return cuda_status(e, "reading collision statistics");
   tests = h.tests;
   rechecks = h.rechecks;

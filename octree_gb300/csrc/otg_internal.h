@@ -182,6 +182,23 @@ struct TmpBuf
   }
 };
 
+// Pinned host memory for the small copies back of a call (counts, error bits, small results): a copy
+// to pageable memory goes through the driver's own buffer and blocks, about 10 us each. Blocks come from a
+// process-wide list (at most kKept of them stay in it) and belong to one call at a time; a call waits for its
+// copies before it gives the block back.
+struct HostBlock
+{
+  static constexpr size_t kBytes = size_t(256) << 10;
+  static constexpr int kKept = 8;
+  void* p;
+  HostBlock();
+  ~HostBlock();
+  HostBlock(const HostBlock&) = delete;
+  HostBlock& operator=(const HostBlock&) = delete;
+};
+// copies `bytes` (at most HostBlock::kBytes) of device memory to dst and waits for the stream
+cudaError_t read_back(void* dst, const void* dev, size_t bytes, cudaStream_t st);
+
 // ownerNode of an entity that no node reachable from the root holds (a location outside the grid:
 // the reference keeps it in a node the root does not link, so no query or collision sees it)
 constexpr u32 kNoOwner = 0xffffffffu;

@@ -65,8 +65,8 @@ struct KnnCounters
   unsigned long long rechecks; // exact distance evaluations
   u32 work;                    // next query to take
   u32 fallbacks;
+  u32 irregular; // queries with other than k results (outside their slots)
   u32 err;
-  u32 irregular; // queries with other than k results (outside their slots), fallbacks among them
 };
 
 template<typename T>
@@ -94,6 +94,7 @@ struct KnnArgs
   u32* count;
   // slots of k results per query: query q's at slot[q], or at q * kAll
   const u64* slot;
+  u64* evenOffsets; // nq + 1 offsets to write, or null
   u32* slotIds;
   double* slotDist;
   // results of the queries that have another number of them
@@ -452,6 +453,12 @@ __global__ void __launch_bounds__(WARPS * 32) knn_filtered_kernel(KnnArgs<T> a)
       break;
     const u32 q = a.order ? a.order[item] : item;
     const u32 k = a.kArr ? a.kArr[q] : a.kAll;
+    if (a.evenOffsets && lane == 0)
+    {
+      a.evenOffsets[q] = u64(q) * k;
+      if (q == a.nq - 1)
+        a.evenOffsets[a.nq] = u64(a.nq) * k;
+    }
     if (k == 0) // ot_query.h:1217-1219: no neighbour requested -> empty result
     {
       if (lane == 0)
@@ -880,12 +887,6 @@ __global__ void csr_move_kernel(const u64* __restrict__ start, const u32* __rest
   }
 }
 
-__global__ void even_offsets_kernel(u64* __restrict__ off, u64 nq, u32 k)
-{
-  for (u64 q = blockIdx.x * u64(blockDim.x) + threadIdx.x; q <= nq; q += u64(gridDim.x) * blockDim.x)
-    off[q] = q * k;
-}
-
 // ---------------------------------------------------------------- host
 static void host_bounds(double v, float& lo, float& hi)
 {
@@ -1010,10 +1011,7 @@ static int knn_filtered_impl(TreeState& t, const T* pts, const u32* dk, u64 nq, 
     cudaMemsetAsync(stats.p, 0, 16, st);
     k_stats_kernel<<<blocks_for(nq), 256, 0, st>>>(dk, nq, stats.as<u32>(), reinterpret_cast<unsigned long long*>(stats.as<unsigned char>() + 8));
     unsigned long long h[2] = { 0, 0 };
-    e = cudaMemcpyAsync(h, stats.p, 16, cudaMemcpyDeviceToHost, st);
-    if (!e)
-      e = cudaStreamSynchronize(st);
-    if (e)
+    if ((e = read_back(h, stats.p, 16, st)))
       return cuda_status(e, "reading k statistics");
     kmax = u32(h[0]);
     ksum = h[1];
@@ -1030,14 +1028,21 @@ static int knn_filtered_impl(TreeState& t, const T* pts, const u32* dk, u64 nq, 
       return cuda_status(e, "allocating the query order");
     query_key_kernel<T><<<blocks_for(nq), 256, 0, st>>>(pts, nq, t.space.as<Space<T>>(), qkeys.as<u32>(), order.as<u32>());
   }
-  TmpBuf ctr, fb, start, cnt, oIds, oDist;
-  if ((e = ctr.ensure(sizeof(KnnCounters), st)) || (e = fb.ensure(sizeof(u32) * nq, st)) || (e = start.ensure(sizeof(u64) * nq, st)) ||
-      (e = cnt.ensure(sizeof(u32) * nq, st)))
+  // one block: the counters, the queries' starts and counts, the list of fallbacks
+  TmpBuf perQuery, irregular;
+  if ((e = perQuery.ensure(64 + (sizeof(u64) + 2 * sizeof(u32)) * nq, st)))
     return cuda_status(e, "allocating kNN buffers");
-  cudaMemsetAsync(ctr.p, 0, sizeof(KnnCounters), st);
+  static_assert(sizeof(KnnCounters) <= 64, "the starts follow the counters");
+  KnnCounters* ctr = perQuery.as<KnnCounters>();
+  u64* start = reinterpret_cast<u64*>(perQuery.as<unsigned char>() + 64);
+  u32* cnt = reinterpret_cast<u32*>(start + nq);
+  u32* fb = cnt + nq;
   if (sortQueries)
-    if (int rc = sort_pairs_u32(qkeys.as<u32>(), order.as<u32>(), nq, 30, st, &ctr.as<KnnCounters>()->err))
+  {
+    cudaMemsetAsync(ctr, 0, sizeof(KnnCounters), st); // (the sort's error bits)
+    if (int rc = sort_pairs_u32(qkeys.as<u32>(), order.as<u32>(), nq, 30, st, &ctr->err))
       return rc;
+  }
   qkeys.release();
   KnnArgs<T> a{};
   a.link = t.nodeLink.as<uint4>();
@@ -1071,17 +1076,17 @@ static int knn_filtered_impl(TreeState& t, const T* pts, const u32* dk, u64 nq, 
   a.widenLo = sizeof(T) == 8 ? 1.f - 0x1p-18f : 1.f - 0x1p-16f;
   a.widenHi = sizeof(T) == 8 ? 1.f + 0x1p-18f : 1.f + 0x1p-16f;
   a.kLimit = big ? 240u : 112u;
-  a.ctr = ctr.as<KnnCounters>();
-  a.fallback = fb.as<u32>();
-  a.start = start.as<u64>();
-  a.count = cnt.as<u32>();
+  a.ctr = ctr;
+  a.fallback = fb;
+  a.start = start;
+  a.count = cnt;
   a.direct = t.respanned ? 0u : kDirectPoints; // (points may lie outside their nodes)
   a.stackCap = (7 * (t.D + 1) + 9 + 3) & ~3u; // depth first: at most 7 entries per level beside the current node's 8 children
   // a slot of k per query: the result itself if every query has k (no ties within the tolerance, enough
   // points in reach); then nothing is moved and the call waits for the GPU once
   const u64 tiles = (nq + kScanTile - 1) / kScanTile;
   TmpBuf tileSums;
-  if ((e = tileSums.ensure(sizeof(u64) * (tiles + 1), st)) ||
+  if ((dk && (e = tileSums.ensure(sizeof(u64) * (tiles + 1), st))) ||
       (e = result_alloc(r, sizeof(u64) * (nq + 1), sizeof(u32) * std::max<u64>(ksum, 1), sizeof(double) * std::max<u64>(ksum, 1), st)))
     return cuda_status(e, "allocating the kNN result");
   if (dk)
@@ -1092,30 +1097,27 @@ static int knn_filtered_impl(TreeState& t, const T* pts, const u32* dk, u64 nq, 
     a.slot = r.offsets.as<u64>();
   }
   else
-    even_offsets_kernel<<<blocks_for(nq + 1), 256, 0, st>>>(r.offsets.as<u64>(), nq, kAll);
+    a.evenOffsets = r.offsets.as<u64>(); // written by the search
   a.slotIds = r.ids.as<u32>();
   a.slotDist = r.dist.as<double>();
   u64 cap = ksum / 8 + 4096;
   KnnCounters h{};
   for (int attempt = 0; attempt < 2; ++attempt)
   {
-    if ((e = oIds.ensure(sizeof(u32) * cap, st)) || (e = oDist.ensure(sizeof(double) * cap, st)))
+    if ((e = irregular.ensure((sizeof(u32) + sizeof(double)) * cap, st)))
       return cuda_status(e, "allocating the kNN output");
-    a.outIds = oIds.as<u32>();
-    a.outDist = oDist.as<double>();
+    a.outDist = irregular.as<double>();
+    a.outIds = reinterpret_cast<u32*>(a.outDist + cap);
     a.outCap = cap;
     int rc = tune_run(tune_key("knn", sizeof(T) == 8, int(t.kind), t.n, nq), { { 2, "warp x2" }, { 4, "warp x4" }, { 8, "warp x8" } }, 4, st,
                       [&](int shape) {
-                        cudaMemsetAsync(ctr.p, 0, offsetof(KnnCounters, err), st); // keeps the sort's error bits
-                        cudaMemsetAsync(&ctr.as<KnnCounters>()->irregular, 0, sizeof(u32), st);
+                        // (keeps the sort's error bits, the last word)
+                        cudaMemsetAsync(ctr, 0, sortQueries ? offsetof(KnnCounters, err) : sizeof(KnnCounters), st);
                         return big ? launch_filtered<T, 512>(a, shape, st) : launch_filtered<T, 256>(a, shape, st);
                       });
     if (rc)
       return rc;
-    e = cudaMemcpyAsync(&h, ctr.p, sizeof(h), cudaMemcpyDeviceToHost, st);
-    if (!e)
-      e = cudaStreamSynchronize(st);
-    if (e)
+    if ((e = read_back(&h, ctr, sizeof(h), st)))
       return cuda_status(e, "running the kNN kernel");
     if (h.out <= cap)
       break;
@@ -1145,24 +1147,26 @@ static int knn_filtered_impl(TreeState& t, const T* pts, const u32* dk, u64 nq, 
     TmpBuf fpts, fk;
     if ((e = fpts.ensure(sizeof(T) * 3 * h.fallbacks, st)) || (e = fk.ensure(sizeof(u32) * h.fallbacks, st)))
       return cuda_status(e, "allocating fallback queries");
-    fallback_points_kernel<<<blocks_for(h.fallbacks), 256, 0, st>>>(fb.as<u32>(), h.fallbacks, pts, u32(sizeof(T) * 3), dk, kAll,
+    fallback_points_kernel<<<blocks_for(h.fallbacks), 256, 0, st>>>(fb, h.fallbacks, pts, u32(sizeof(T) * 3), dk, kAll,
                                                                    fpts.as<unsigned char>(), fk.as<u32>());
     if (int rc = query_knn(t, fpts.p, h.fallbacks, fk.as<u32>(), 0, maxDist, tol, OTG_ALGO_PLAIN_FP64, fbr, OTG_MEM_DEVICE, st))
       return rc;
-    fallback_slots_kernel<<<blocks_for(h.fallbacks), 256, 0, st>>>(fb.as<u32>(), h.fallbacks, fbr.offsets.as<u64>(), start.as<u64>(), cnt.as<u32>());
+    fallback_slots_kernel<<<blocks_for(h.fallbacks), 256, 0, st>>>(fb, h.fallbacks, fbr.offsets.as<u64>(), start, cnt);
   }
   // CSR: offsets by scan of the counts, then entries moved into query order
   u64 total = 0;
-  scan_reduce_kernel<<<u32(tiles), kScanThreads, 0, st>>>(cnt.as<u32>(), nq, tileSums.as<u64>());
+  if ((e = tileSums.ensure(sizeof(u64) * (tiles + 1), st)))
+    return cuda_status(e, "allocating the kNN result");
+  scan_reduce_kernel<<<u32(tiles), kScanThreads, 0, st>>>(cnt, nq, tileSums.as<u64>());
   scan_tiles_kernel<<<1, kScanThreads, 0, st>>>(tileSums.as<u64>(), tiles);
-  scan_apply_kernel<<<u32(tiles), kScanThreads, 0, st>>>(cnt.as<u32>(), nq, tileSums.as<u64>(), r.offsets.as<u64>());
-  if ((e = cudaMemcpyAsync(&total, tileSums.as<u64>() + tiles, sizeof(u64), cudaMemcpyDeviceToHost, st)) || (e = cudaStreamSynchronize(st)))
+  scan_apply_kernel<<<u32(tiles), kScanThreads, 0, st>>>(cnt, nq, tileSums.as<u64>(), r.offsets.as<u64>());
+  if ((e = read_back(&total, tileSums.as<u64>() + tiles, sizeof(u64), st)))
     return cuda_status(e, "counting the kNN result");
   ResultState moved;
   if ((e = result_alloc(moved, 0, sizeof(u32) * std::max<u64>(total, 1), sizeof(double) * std::max<u64>(total, 1), st)))
     return cuda_status(e, "allocating the result");
-  csr_move_kernel<<<blocks_for(nq * 32), 256, 0, st>>>(start.as<u64>(), cnt.as<u32>(), r.offsets.as<u64>(), nq, r.ids.as<u32>(), r.dist.as<double>(),
-                                                        oIds.as<u32>(), oDist.as<double>(), fbr.ids.as<u32>(), fbr.dist.as<double>(), moved.ids.as<u32>(),
+  csr_move_kernel<<<blocks_for(nq * 32), 256, 0, st>>>(start, cnt, r.offsets.as<u64>(), nq, r.ids.as<u32>(), r.dist.as<double>(),
+                                                        a.outIds, a.outDist, fbr.ids.as<u32>(), fbr.dist.as<double>(), moved.ids.as<u32>(),
                                                         moved.dist.as<double>());
   std::swap(r.ids.p, moved.ids.p);
   std::swap(r.ids.bytes, moved.ids.bytes);

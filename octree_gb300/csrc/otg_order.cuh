@@ -47,6 +47,41 @@ __global__ void query_scatter_kernel(const u64* __restrict__ items, const double
   }
 }
 
+// offsets (nq + 1 of them) from the counts in one block: up to kScanOneBlock queries this is one launch where
+// the scan over tiles takes three
+constexpr u64 kScanOneBlock = 16384;
+__global__ void __launch_bounds__(1024) scan_one_block_kernel(const u32* __restrict__ cnt, u32 nq, u64* __restrict__ off)
+{
+  __shared__ u64 warpSums[32];
+  const u32 lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const u32 per = (nq + 1023) / 1024; // counts per thread
+  const u32 b = min(nq, threadIdx.x * per), e = min(nq, b + per);
+  u64 sum = 0;
+  for (u32 i = b; i < e; ++i)
+    sum += cnt[i];
+  u64 incl = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1)
+  {
+    const u64 y = __shfl_up_sync(~0u, incl, o);
+    if (lane >= u32(o))
+      incl += y;
+  }
+  if (lane == 31)
+    warpSums[w] = incl;
+  __syncthreads();
+  u64 at = incl - sum;
+  for (u32 i = 0; i < w; ++i)
+    at += warpSums[i];
+  for (u32 i = b; i < e; ++i)
+  {
+    off[i] = at;
+    at += cnt[i];
+  }
+  if (threadIdx.x == 1023)
+    off[nq] = at;
+}
+
 // sort key of an item: the distance's bits (distances are >= 0, so bit order is value order), then
 // the id; without distances the id alone
 template<bool DIST>
@@ -87,13 +122,13 @@ __device__ __forceinline__ void run_sort_lanes(RunKey<DIST>& v, u32 lane)
 
 // One warp per query sorts its run in place: each 32 items in registers, then every item's place is
 // its place among its 32 plus the counts of smaller items in the other sorted groups (binary
-// searches in shared memory). Runs above kRunSortMax go to the list longRuns[2 ...] (longRuns[0]
-// counts them) for run_sort_block_kernel. A bitonic network over 128 items takes twice the steps.
+// searches in shared memory). Runs above kRunSortMax go to the list longRuns (longCount[0] counts them)
+// for run_sort_block_kernel. A bitonic network over 128 items takes twice the steps.
 constexpr u32 kRunSortMax = 256;
 constexpr int kRunSortWarps = 8;
 template<bool DIST>
 __global__ void __launch_bounds__(kRunSortWarps * 32) run_sort_kernel(const u64* __restrict__ off, u64 nq, u32* __restrict__ ids, double* __restrict__ dist,
-                                                                    u32* __restrict__ longRuns, u32 longCap)
+                                                                    u32* __restrict__ longCount, u32* __restrict__ longRuns, u32 longCap)
 {
   __shared__ u64 sd[DIST ? kRunSortWarps : 1][DIST ? kRunSortMax : 1];
   __shared__ u32 si[kRunSortWarps][kRunSortMax];
@@ -109,9 +144,9 @@ __global__ void __launch_bounds__(kRunSortWarps * 32) run_sort_kernel(const u64*
     {
       if (lane == 0)
       {
-        const u32 at = atomicAdd(longRuns, 1u);
+        const u32 at = atomicAdd(longCount, 1u);
         if (at < longCap)
-          longRuns[2 + at] = u32(q);
+          longRuns[at] = u32(q);
       }
       continue;
     }
@@ -175,26 +210,26 @@ __global__ void __launch_bounds__(kRunSortWarps * 32) run_sort_kernel(const u64*
 }
 
 // One block per listed run sorts it in place with a bitonic network in shared memory (dynamic: 12 or
-// 4 bytes per item); runs above kBlockRunMax are only counted, in longRuns[1].
+// 4 bytes per item); runs above kBlockRunMax are only counted, in longCount[1].
 constexpr u32 kBlockRunMax = 8192;
 constexpr int kBlockSortThreads = 512;
 template<bool DIST>
 __global__ void __launch_bounds__(kBlockSortThreads) run_sort_block_kernel(const u64* __restrict__ off, u32* __restrict__ ids, double* __restrict__ dist,
-                                                                         u32* __restrict__ longRuns, u32 longCap)
+                                                                         u32* __restrict__ longCount, const u32* __restrict__ longRuns, u32 longCap)
 {
   extern __shared__ u64 runMem[];
   u64* sd = runMem;
   u32* si = reinterpret_cast<u32*>(runMem + (DIST ? kBlockRunMax : 0));
-  const u32 n = min(longRuns[0], longCap);
+  const u32 n = min(longCount[0], longCap);
   for (u32 r = blockIdx.x; r < n; r += gridDim.x)
   {
-    const u32 q = longRuns[2 + r];
+    const u32 q = longRuns[r];
     const u64 b = off[q];
     const u64 len64 = off[q + 1] - b;
     if (len64 > kBlockRunMax)
     {
       if (threadIdx.x == 0)
-        atomicAdd(longRuns + 1, 1u);
+        atomicAdd(longCount + 1, 1u);
       continue;
     }
     const u32 len = u32(len64);

@@ -1090,8 +1090,13 @@ __global__ void item_ids_kernel(const u64* __restrict__ items, u64 m, u32* __res
 struct Collected
 {
   // count: four words read back together: the item count, the filter's tests, the undecided tests,
-  // and the error bits (the low half of the fourth)
+  // and the error bits (the low half of the fourth); then the work buffer of the batched kernels,
+  // which starts with its own 16 bytes of counters
   TmpBuf items, dist, count;
+  size_t workBytes = 0;
+  u32* work() const { return reinterpret_cast<u32*>(count.as<unsigned char>() + 32); }
+  // zeroes the words and the work buffer's counters
+  void clear(cudaStream_t st) const { cudaMemsetAsync(count.p, 0, 32 + std::min<size_t>(workBytes, 16), st); }
   u64 m = 0;
   u64 tests = 0, rechecks = 0;
   u32* errp() const { return reinterpret_cast<u32*>(count.as<unsigned long long>() + 3); }
@@ -1122,32 +1127,32 @@ static int status_of(u32 h)
   return OTG_OK;
 }
 
-// Runs launch(appender) until the append buffer was large enough; items end in c.items. `most` bounds
+// Runs launch(appender, err) until the append buffer was large enough; items end in c.items. `most` bounds
 // the items (queries times entities): below kItemFloor of them the buffer holds that bound, as a
 // second run costs the whole search again and a larger pooled buffer costs nothing (rays through 1M
 // boxes have 75 hits each where the guess was 16: their search ran twice, 2 x 3.4 ms).
+// workBytes: size of the batched kernels' work buffer (c.work()). launch clears the counters (c.clear)
+// before each search that it runs.
 constexpr u64 kItemFloor = u64(8) << 20;
 template<typename F>
-static int collect(Collected& c, bool withDist, u64 guess, u64 most, F&& launch, cudaStream_t st)
+static int collect(Collected& c, bool withDist, u64 guess, u64 most, size_t workBytes, F&& launch, cudaStream_t st)
 {
   cudaError_t e;
-  if ((e = c.count.ensure(sizeof(unsigned long long) * 4, st)))
+  c.workBytes = workBytes;
+  if ((e = c.count.ensure(32 + workBytes, st)))
     return cuda_status(e, "allocating counters");
   u64 cap = std::max<u64>(std::max<u64>(guess, 1024), std::min(most, kItemFloor));
   for (int attempt = 0; attempt < 3; ++attempt)
   {
     if ((e = c.items.ensure(sizeof(u64) * cap, st)) || (withDist && (e = c.dist.ensure(sizeof(double) * cap, st))))
       return cuda_status(e, "allocating result buffer");
-    cudaMemsetAsync(c.count.p, 0, sizeof(unsigned long long) * 4, st);
-    Appender a{ c.items.as<u64>(), withDist ? c.dist.as<double>() : nullptr, c.count.as<unsigned long long>(), cap };
-    launch(a, c.errp());
+    Appender a{ c.items.as<u64>(), withDist ? c.dist.as<double>() : nullptr, c.count.as<unsigned long long>(), cap, true };
+    if (int rc = launch(a, c.errp()))
+      return rc;
     if ((e = cudaGetLastError()))
       return cuda_status(e, "launching query");
     unsigned long long h[4] = { 0, 0, 0, 0 };
-    e = cudaMemcpyAsync(h, c.count.p, sizeof(h), cudaMemcpyDeviceToHost, st);
-    if (!e)
-      e = cudaStreamSynchronize(st);
-    if (e)
+    if ((e = read_back(h, c.count.p, sizeof(h), st)))
       return cuda_status(e, "running query");
     const unsigned long long m = h[0];
     c.tests = h[1];
@@ -1176,47 +1181,58 @@ static int order_by_runs(Collected& c, u64 nq, ResultState& r, bool withDist, cu
   // put every item's atomic on a few counters)
   if (m >= (u64(1) << 32) || nq >= (u64(1) << 31) || m > u64(kBlockRunMax) * nq)
     return OTG_OK;
-  TmpBuf cnt, slot, tileSums, longRuns;
+  // one block: the long runs' two counters, the counts, then (8-byte aligned) the tile sums, the items' slots and the
+  // list of runs above kRunSortMax (at most m / kRunSortMax of them)
   const u64 tiles = (nq + kScanTile - 1) / kScanTile;
-  // the list of runs above kRunSortMax: at most m / kRunSortMax of them, after its two counters
   const u64 longCap = m / kRunSortMax + 1;
+  const size_t zeroed = sizeof(u32) * (2 + nq), sumsAt = (zeroed + 7) & ~size_t(7);
+  TmpBuf buf;
   cudaError_t e;
-  if ((e = cnt.ensure(sizeof(u32) * nq, st)) || (e = slot.ensure(sizeof(u32) * m, st)) || (e = tileSums.ensure(sizeof(u64) * (tiles + 1), st)) ||
-      (e = longRuns.ensure(sizeof(u32) * (2 + longCap), st)))
+  if ((e = buf.ensure(sumsAt + sizeof(u64) * (tiles + 1) + sizeof(u32) * (m + longCap), st)))
     return cuda_status(e, "allocating the result order");
-  cudaMemsetAsync(cnt.p, 0, sizeof(u32) * nq, st);
-  cudaMemsetAsync(longRuns.p, 0, sizeof(u32) * 2, st);
-  query_slots_kernel<<<blocks_for(m), 256, 0, st>>>(c.items.as<u64>(), m, cnt.as<u32>(), slot.as<u32>());
-  scan_reduce_kernel<<<u32(tiles), kScanThreads, 0, st>>>(cnt.as<u32>(), nq, tileSums.as<u64>());
-  scan_tiles_kernel<<<1, kScanThreads, 0, st>>>(tileSums.as<u64>(), tiles);
-  scan_apply_kernel<<<u32(tiles), kScanThreads, 0, st>>>(cnt.as<u32>(), nq, tileSums.as<u64>(), r.offsets.as<u64>());
-  query_scatter_kernel<<<blocks_for(m), 256, 0, st>>>(c.items.as<u64>(), withDist ? c.dist.as<double>() : nullptr, slot.as<u32>(), m, r.offsets.as<u64>(),
+  u32* longCount = buf.as<u32>();
+  u32* cnt = longCount + 2;
+  u64* tileSums = reinterpret_cast<u64*>(buf.as<unsigned char>() + sumsAt);
+  u32* slot = reinterpret_cast<u32*>(tileSums + tiles + 1);
+  u32* longRuns = slot + m;
+  cudaMemsetAsync(buf.p, 0, zeroed, st);
+  query_slots_kernel<<<blocks_for(m), 256, 0, st>>>(c.items.as<u64>(), m, cnt, slot);
+  if (nq <= kScanOneBlock)
+    scan_one_block_kernel<<<1, 1024, 0, st>>>(cnt, u32(nq), r.offsets.as<u64>());
+  else
+  {
+    scan_reduce_kernel<<<u32(tiles), kScanThreads, 0, st>>>(cnt, nq, tileSums);
+    scan_tiles_kernel<<<1, kScanThreads, 0, st>>>(tileSums, tiles);
+    scan_apply_kernel<<<u32(tiles), kScanThreads, 0, st>>>(cnt, nq, tileSums, r.offsets.as<u64>());
+  }
+  query_scatter_kernel<<<blocks_for(m), 256, 0, st>>>(c.items.as<u64>(), withDist ? c.dist.as<double>() : nullptr, slot, m, r.offsets.as<u64>(),
                                                       r.ids.as<u32>(), withDist ? r.dist.as<double>() : nullptr);
   const u32 grid = u32(std::min<u64>((nq + kRunSortWarps - 1) / kRunSortWarps, 152 * 8));
-  const u32 longGrid = u32(std::min<u64>(longCap, 152 * 2));
   const u64* off = r.offsets.as<u64>();
   if (withDist)
+    run_sort_kernel<true><<<grid, kRunSortWarps * 32, 0, st>>>(off, nq, r.ids.as<u32>(), r.dist.as<double>(), longCount, longRuns, u32(longCap));
+  else
+    run_sort_kernel<false><<<grid, kRunSortWarps * 32, 0, st>>>(off, nq, r.ids.as<u32>(), nullptr, longCount, longRuns, u32(longCap));
+  // the long runs, where there are some (the host waits here in any case)
+  u32 h[2] = { 0, 0 };
+  if ((e = cudaGetLastError()) || (e = read_back(h, longCount, sizeof(h), st)))
+    return cuda_status(e, "finishing result");
+  if (h[0])
   {
-    run_sort_kernel<true><<<grid, kRunSortWarps * 32, 0, st>>>(off, nq, r.ids.as<u32>(), r.dist.as<double>(), longRuns.as<u32>(), u32(longCap));
-    if (m > kRunSortMax)
+    const u32 longGrid = std::min<u32>(h[0], 152 * 2);
+    if (withDist)
     {
       if ((e = cudaFuncSetAttribute(run_sort_block_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kBlockRunMax * 12))))
         return cuda_status(e, "configuring the run sort");
-      run_sort_block_kernel<true><<<longGrid, kBlockSortThreads, kBlockRunMax * 12, st>>>(off, r.ids.as<u32>(), r.dist.as<double>(), longRuns.as<u32>(),
+      run_sort_block_kernel<true><<<longGrid, kBlockSortThreads, kBlockRunMax * 12, st>>>(off, r.ids.as<u32>(), r.dist.as<double>(), longCount, longRuns,
                                                                                         u32(longCap));
     }
+    else
+      run_sort_block_kernel<false><<<longGrid, kBlockSortThreads, kBlockRunMax * 4, st>>>(off, r.ids.as<u32>(), nullptr, longCount, longRuns, u32(longCap));
+    if ((e = cudaGetLastError()) || (e = read_back(h, longCount, sizeof(h), st)))
+      return cuda_status(e, "finishing result");
   }
-  else
-  {
-    run_sort_kernel<false><<<grid, kRunSortWarps * 32, 0, st>>>(off, nq, r.ids.as<u32>(), nullptr, longRuns.as<u32>(), u32(longCap));
-    if (m > kRunSortMax)
-      run_sort_block_kernel<false><<<longGrid, kBlockSortThreads, kBlockRunMax * 4, st>>>(off, r.ids.as<u32>(), nullptr, longRuns.as<u32>(), u32(longCap));
-  }
-  u32 tooLong = 0;
-  if ((e = cudaGetLastError()) || (e = cudaMemcpyAsync(&tooLong, longRuns.as<u32>() + 1, sizeof(u32), cudaMemcpyDeviceToHost, st)) ||
-      (e = cudaStreamSynchronize(st)))
-    return cuda_status(e, "finishing result");
-  done = tooLong == 0;
+  done = h[1] == 0;
   return OTG_OK;
 }
 
@@ -1380,7 +1396,7 @@ static int finish_pairs(Collected& c, u64 nA, u64 nB, ResultState& r, cudaStream
     query_scatter_kernel<<<blocks_for(m), 256, 0, st>>>(c.items.as<u64>(), nullptr, slot.as<u32>(), m, off.as<u64>(), bs.as<u32>(), nullptr);
     pair_write_kernel<<<u32(std::min<u64>((nA + 255) / 256, 152 * 8)), 256, 0, st>>>(off.as<u64>(), nA, bs.as<u32>(), r.ids.as<uint2>(), tooLong.as<u32>());
     u32 h = 0;
-    if ((e = cudaGetLastError()) || (e = cudaMemcpyAsync(&h, tooLong.p, sizeof(u32), cudaMemcpyDeviceToHost, st)) || (e = cudaStreamSynchronize(st)))
+    if ((e = cudaGetLastError()) || (e = read_back(&h, tooLong.p, sizeof(u32), st)))
       return cuda_status(e, "ordering pairs");
     done = h == 0;
   }
@@ -1478,30 +1494,26 @@ static int range_impl(const TreeState& t, const void* ranges, u64 nq, int mode, 
     if (algo != OTG_ALGO_PLAIN_FP64 && tv.isBox)
       if (int rci = use_images(const_cast<TreeState&>(t), tv, nq * 128, st))
         return rci;
-  TmpBuf work;
-  if (cudaError_t e = work.ensure(batch_work_bytes(nq), st))
-    return cuda_status(e, "allocating the work counter");
-  int launchRc = OTG_OK;
   int rc = collect(
-    c, false, nq * 32, nq * t.n,
+    c, false, nq * 32, nq * t.n, batch_work_bytes(nq),
     [&](Appender a, u32* err) {
       if (algo == OTG_ALGO_PLAIN_FP64)
+      {
+        c.clear(st);
         range_plain_kernel<T><<<u32((nq + 127) / 128), 128, 0, st>>>(tv, (const T*)d, u32(nq), mode, tl, a, err);
-      else
-        launchRc = tune_run(query_key("range", algo, qTree, sizeof(T) == 8, t.kind, t.n, nq), query_shapes(algo, nq), kDefaultQueryShape, st, [&](int shape) {
-          cudaMemsetAsync(a.count, 0, sizeof(unsigned long long), st);
-          cudaMemsetAsync(err, 0, sizeof(u32), st);
+        return int(OTG_OK);
+      }
+      return tune_run(query_key("range", algo, qTree, sizeof(T) == 8, t.kind, t.n, nq), query_shapes(algo, nq), kDefaultQueryShape, st, [&](int shape) {
+          c.clear(st);
           if (shape == 0)
           {
             range_plain_kernel<T><<<u32((nq + 127) / 128), 128, 0, st>>>(tv, (const T*)d, u32(nq), mode, tl, a, err);
             return cuda_status(cudaGetLastError(), "launching the range search");
           }
-          return batch_range<T>(tv, (const T*)d, u32(nq), mode, tl, a, work.as<u32>(), err, st, shape, work.bytes);
+          return batch_range<T>(tv, (const T*)d, u32(nq), mode, tl, a, c.work(), err, st, shape, c.workBytes);
         });
     },
     st);
-  if (launchRc)
-    return launchRc;
   if (rc)
     return rc;
   r.filterTests = c.tests; // the FP32 pre-tests of the batched kernel and the ones left to FP64
@@ -1525,30 +1537,26 @@ static int pick_impl(const TreeState& t, const void* pts, u64 nq, double tol, in
     if (algo != OTG_ALGO_PLAIN_FP64)
       if (int rci = use_images(const_cast<TreeState&>(t), tv, nq * 64, st))
         return rci;
-  TmpBuf work;
-  if (cudaError_t e = work.ensure(batch_work_bytes(nq), st))
-    return cuda_status(e, "allocating the work counter");
-  int launchRc = OTG_OK;
   int rc = collect(
-    c, false, nq * 8, nq * t.n,
+    c, false, nq * 8, nq * t.n, batch_work_bytes(nq),
     [&](Appender a, u32* err) {
       if (algo == OTG_ALGO_PLAIN_FP64)
+      {
+        c.clear(st);
         pick_plain_kernel<T><<<u32((nq + 127) / 128), 128, 0, st>>>(tv, (const T*)d, u32(nq), tl, a, err);
-      else
-        launchRc = tune_run(query_key("pick", algo, qTree, sizeof(T) == 8, t.kind, t.n, nq), query_shapes(algo, nq), kDefaultQueryShape, st, [&](int shape) {
-          cudaMemsetAsync(a.count, 0, sizeof(unsigned long long), st);
-          cudaMemsetAsync(err, 0, sizeof(u32), st);
+        return int(OTG_OK);
+      }
+      return tune_run(query_key("pick", algo, qTree, sizeof(T) == 8, t.kind, t.n, nq), query_shapes(algo, nq), kDefaultQueryShape, st, [&](int shape) {
+          c.clear(st);
           if (shape == 0)
           {
             pick_plain_kernel<T><<<u32((nq + 127) / 128), 128, 0, st>>>(tv, (const T*)d, u32(nq), tl, a, err);
             return cuda_status(cudaGetLastError(), "launching the pick search");
           }
-          return batch_pick<T>(tv, (const T*)d, u32(nq), tl, a, work.as<u32>(), err, st, shape, work.bytes);
+          return batch_pick<T>(tv, (const T*)d, u32(nq), tl, a, c.work(), err, st, shape, c.workBytes);
         });
     },
     st);
-  if (launchRc)
-    return launchRc;
   if (rc)
     return rc;
   return finish_sorted_ids(c, nq, r, st, t, qTree);
@@ -1571,30 +1579,26 @@ static int frustum_impl(const TreeState& t, const void* planes, u64 np, u64 nq, 
       if (int rci = use_images(const_cast<TreeState&>(t), tv, nq * (t.n / 16 + 1), st))
         return rci;
   T tl = tol_of<T>(tol);
-  TmpBuf work;
-  if (cudaError_t e = work.ensure(batch_work_bytes(nq), st))
-    return cuda_status(e, "allocating the work counter");
-  int launchRc = OTG_OK;
   int rc = collect(
-    c, false, std::max<u64>(nq * 64, t.n / 4), nq * t.n,
+    c, false, std::max<u64>(nq * 64, t.n / 4), nq * t.n, batch_work_bytes(nq),
     [&](Appender a, u32* err) {
       if (algo == OTG_ALGO_PLAIN_FP64)
+      {
+        c.clear(st);
         frustum_plain_kernel<T><<<u32((nq + 127) / 128), 128, 0, st>>>(tv, (const T*)d, u32(np), u32(nq), tl, a, err);
-      else
-        launchRc = tune_run(query_key("frustum", algo, qTree, sizeof(T) == 8, t.kind, t.n, nq), query_shapes(algo, nq), kDefaultQueryShape, st, [&](int shape) {
-          cudaMemsetAsync(a.count, 0, sizeof(unsigned long long), st);
-          cudaMemsetAsync(err, 0, sizeof(u32), st);
+        return int(OTG_OK);
+      }
+      return tune_run(query_key("frustum", algo, qTree, sizeof(T) == 8, t.kind, t.n, nq), query_shapes(algo, nq), kDefaultQueryShape, st, [&](int shape) {
+          c.clear(st);
           if (shape == 0)
           {
             frustum_plain_kernel<T><<<u32((nq + 127) / 128), 128, 0, st>>>(tv, (const T*)d, u32(np), u32(nq), tl, a, err);
             return cuda_status(cudaGetLastError(), "launching the frustum culling");
           }
-          return batch_frustum<T>(tv, (const T*)d, u32(np), u32(nq), tl, a, work.as<u32>(), err, st, shape, work.bytes);
+          return batch_frustum<T>(tv, (const T*)d, u32(np), u32(nq), tl, a, c.work(), err, st, shape, c.workBytes);
         });
     },
     st);
-  if (launchRc)
-    return launchRc;
   if (rc)
     return rc;
   return finish_sorted_ids(c, nq, r, st, t, qTree);
@@ -1620,31 +1624,27 @@ static int plane_impl(const TreeState& t, const void* planes, u64 nq, bool posit
         return rci;
     }
   T tl = tol_of<T>(tol);
-  TmpBuf work;
-  if (cudaError_t e = work.ensure(batch_work_bytes(nq), st))
-    return cuda_status(e, "allocating the work counter");
-  int launchRc = OTG_OK;
   int rc = collect(
-    c, false, std::max<u64>(nq * 64, positive ? t.n : t.n / 16), nq * t.n,
+    c, false, std::max<u64>(nq * 64, positive ? t.n : t.n / 16), nq * t.n, batch_work_bytes(nq),
     [&](Appender a, u32* err) {
       if (algo == OTG_ALGO_PLAIN_FP64)
+      {
+        c.clear(st);
         plane_plain_kernel<T><<<u32((nq + 127) / 128), 128, 0, st>>>(tv, (const T*)d, u32(nq), positive ? 1 : 0, tl, a, err);
-      else
-        launchRc = tune_run(query_key(positive ? "plane positive" : "plane", algo, qTree, sizeof(T) == 8, t.kind, t.n, nq), query_shapes(algo, nq), kDefaultQueryShape, st,
+        return int(OTG_OK);
+      }
+      return tune_run(query_key(positive ? "plane positive" : "plane", algo, qTree, sizeof(T) == 8, t.kind, t.n, nq), query_shapes(algo, nq), kDefaultQueryShape, st,
                             [&](int shape) {
-                              cudaMemsetAsync(a.count, 0, sizeof(unsigned long long), st);
-                              cudaMemsetAsync(err, 0, sizeof(u32), st);
+                              c.clear(st);
                               if (shape == 0)
                               {
                                 plane_plain_kernel<T><<<u32((nq + 127) / 128), 128, 0, st>>>(tv, (const T*)d, u32(nq), positive ? 1 : 0, tl, a, err);
                                 return cuda_status(cudaGetLastError(), "launching the plane search");
                               }
-                              return batch_plane<T>(tv, (const T*)d, u32(nq), positive, tl, a, work.as<u32>(), err, st, shape, work.bytes);
+                              return batch_plane<T>(tv, (const T*)d, u32(nq), positive, tl, a, c.work(), err, st, shape, c.workBytes);
                             });
     },
     st);
-  if (launchRc)
-    return launchRc;
   if (rc)
     return rc;
   return finish_sorted_ids(c, nq, r, st, t, qTree);
@@ -1715,31 +1715,27 @@ static int query_impl(const TreeState& t, const QueryCond* conds, const u64* off
   Collected c;
   auto tv = view<T>(t, nullptr);
   T tl = tol_of<T>(tol);
-  TmpBuf work;
-  if (cudaError_t e = work.ensure(batch_work_bytes(nq), st))
-    return cuda_status(e, "allocating the work counter");
-  int launchRc = OTG_OK;
   int rc = collect(
-    c, false, std::max<u64>(nq * 64, t.n / 4), nq * t.n,
+    c, false, std::max<u64>(nq * 64, t.n / 4), nq * t.n, batch_work_bytes(nq),
     [&](Appender a, u32* err) {
       if (algo == OTG_ALGO_PLAIN_FP64)
+      {
+        c.clear(st);
         query_plain_kernel<T><<<u32((nq + 127) / 128), 128, 0, st>>>(tv, qp, u32(nq), tl, a, err);
-      else
-        launchRc = tune_run(query_key(orOp ? "query or" : "query and", algo, false, sizeof(T) == 8, t.kind, t.n, nq), query_shapes(algo, nq), kDefaultQueryShape, st,
+        return int(OTG_OK);
+      }
+      return tune_run(query_key(orOp ? "query or" : "query and", algo, false, sizeof(T) == 8, t.kind, t.n, nq), query_shapes(algo, nq), kDefaultQueryShape, st,
                             [&](int shape) {
-                              cudaMemsetAsync(a.count, 0, sizeof(unsigned long long), st);
-                              cudaMemsetAsync(err, 0, sizeof(u32), st);
+                              c.clear(st);
                               if (shape == 0)
                               {
                                 query_plain_kernel<T><<<u32((nq + 127) / 128), 128, 0, st>>>(tv, qp, u32(nq), tl, a, err);
                                 return cuda_status(cudaGetLastError(), "launching the combined query");
                               }
-                              return batch_query_program<T>(tv, qp, u32(nq), tl, a, work.as<u32>(), err, st, shape, work.bytes);
+                              return batch_query_program<T>(tv, qp, u32(nq), tl, a, c.work(), err, st, shape, c.workBytes);
                             });
     },
     st);
-  if (launchRc)
-    return launchRc;
   if (rc)
     return rc;
   return finish_sorted_ids(c, nq, r, st, t, nullptr);
@@ -1775,16 +1771,18 @@ static int knn_impl(const TreeState& t, const void* pts, u64 nq, const u32* k, u
     if ((e = m.ensure(sizeof(u32), st)) || (e = cudaMemsetAsync(m.p, 0, sizeof(u32), st)))
       return cuda_status(e, "finding the largest k");
     max_u32_kernel<<<u32(std::min<u64>((nq + 255) / 256, 152 * 8)), 256, 0, st>>>((const u32*)dk, nq, m.as<u32>());
-    if ((e = cudaMemcpyAsync(&kMax, m.p, sizeof(u32), cudaMemcpyDeviceToHost, st)) || (e = cudaStreamSynchronize(st)))
+    if ((e = read_back(&kMax, m.p, sizeof(u32), st)))
       return cuda_status(e, "finding the largest k");
   }
   const int bucket = knn_heap_bucket(kMax);
   Collected c;
   int rc = collect(
-    c, true, nq * 16, nq * t.n,
+    c, true, nq * 16, nq * t.n, 0,
     [&](Appender a, u32* err) {
+      c.clear(st);
       launch_knn_threshold<T>(bucket, u32((nq + 127) / 128), st, tv, (const T*)d, u32(nq), (const u32*)dk, kAll, F0, tl, F.as<T>(), err);
       knn_collect_kernel<T><<<u32((nq + 127) / 128), 128, 0, st>>>(tv, (const T*)d, u32(nq), F.as<T>(), tl, a, err);
+      return int(OTG_OK);
     },
     st);
   if (rc)
@@ -1814,57 +1812,45 @@ static int ray_impl(const TreeState& t, const void* rays, u64 nq, double tol, do
         return rci;
   if (!first)
   {
-    TmpBuf work;
-    if (cudaError_t e = work.ensure(batch_work_bytes(nq), st))
-      return cuda_status(e, "allocating the work counter");
-    int launchRc = OTG_OK;
     rc = collect(
-      c, true, nq * 16, nq * t.n,
+      c, true, nq * 16, nq * t.n, batch_work_bytes(nq),
       [&](Appender a, u32* err) {
         if (algo == OTG_ALGO_PLAIN_FP64)
+        {
+          c.clear(st);
           ray_all_plain_kernel<T><<<u32((nq + 127) / 128), 128, 0, st>>>(tv, (const T*)d, u32(nq), tl, ti, md, a, err);
-        else
-          launchRc = tune_run(query_key("ray all", algo, qTree, sizeof(T) == 8, t.kind, t.n, nq), query_shapes(algo, nq), kDefaultQueryShape, st, [&](int shape) {
-            cudaMemsetAsync(a.count, 0, sizeof(unsigned long long), st);
-            cudaMemsetAsync(err, 0, sizeof(u32), st);
+          return int(OTG_OK);
+        }
+        return tune_run(query_key("ray all", algo, qTree, sizeof(T) == 8, t.kind, t.n, nq), query_shapes(algo, nq), kDefaultQueryShape, st, [&](int shape) {
+            c.clear(st);
             if (shape == 0)
             {
               ray_all_plain_kernel<T><<<u32((nq + 127) / 128), 128, 0, st>>>(tv, (const T*)d, u32(nq), tl, ti, md, a, err);
               return cuda_status(cudaGetLastError(), "launching the ray query");
             }
-            return batch_ray_all<T>(tv, (const T*)d, u32(nq), tl, ti, md, a, work.as<u32>(), err, st, shape, work.bytes);
+            return batch_ray_all<T>(tv, (const T*)d, u32(nq), tl, ti, md, a, c.work(), err, st, shape, c.workBytes);
           });
       },
       st);
-    if (launchRc)
-      return launchRc;
   }
   else
   {
-    TmpBuf work;
-    if (algo == OTG_ALGO_PLAIN_FP64)
-    {
+    const bool plain = algo == OTG_ALGO_PLAIN_FP64;
+    if (plain)
       if (cudaError_t e = M.ensure(sizeof(T) * nq, st))
         return cuda_status(e, "allocating ray thresholds");
-    }
-    else if (cudaError_t e = work.ensure(ray_first_work_bytes(nq), st))
-      return cuda_status(e, "allocating the ray list");
-    int launchRc = OTG_OK;
     rc = collect(
-      c, true, nq * 4, nq * t.n,
+      c, true, nq * 4, nq * t.n, plain ? 0 : ray_first_work_bytes(nq),
       [&](Appender a, u32* err) {
-        if (algo != OTG_ALGO_PLAIN_FP64)
-        {
-          // entities outside their nodes (set_entities) are found in the walk's own order only
-          launchRc = ray_first<T>(tv, tv.isBox && !t.respanned, (const T*)d, u32(nq), tl, ti, md, a, work.as<u32>(), err, st);
-          return;
-        }
+        c.clear(st);
+        // entities outside their nodes (set_entities) are found in the walk's own order only
+        if (!plain)
+          return ray_first<T>(tv, tv.isBox && !t.respanned, (const T*)d, u32(nq), tl, ti, md, a, c.work(), err, st);
         ray_first_threshold_kernel<T><<<u32((nq + 127) / 128), 128, 0, st>>>(tv, (const T*)d, u32(nq), tl, ti, md, M.as<T>(), err);
         ray_first_collect_kernel<T><<<u32((nq + 127) / 128), 128, 0, st>>>(tv, (const T*)d, u32(nq), tl, ti, M.as<T>(), a, err);
+        return int(OTG_OK);
       },
       st);
-    if (launchRc)
-      return launchRc;
   }
   if (rc)
     return rc;
@@ -1895,18 +1881,16 @@ static int collide_impl(const TreeState& a, const TreeState& b, bool self, doubl
   T tl = tol_of<T>(tol);
   const bool filtered = algo != OTG_ALGO_PLAIN_FP64;
   CollideSearch search;
-  int searchRc = OTG_OK;
   int rc = collect(
-    c, false, a.n * 4, 0,
+    c, false, a.n * 4, 0, 0,
     [&](Appender ap, u32* err) {
+      c.clear(st);
       if (filtered)
-        searchRc = collide_search_filtered(const_cast<TreeState&>(a), const_cast<TreeState&>(b), self, tol, ap, err, search, st);
-      else
-        collide_plain_kernel<T><<<u32((a.n + 127) / 128), 128, 0, st>>>(ta, tb, tl, self ? 1 : 0, ap, err);
+        return collide_search_filtered(const_cast<TreeState&>(a), const_cast<TreeState&>(b), self, tol, ap, err, search, st);
+      collide_plain_kernel<T><<<u32((a.n + 127) / 128), 128, 0, st>>>(ta, tb, tl, self ? 1 : 0, ap, err);
+      return int(OTG_OK);
     },
     st);
-  if (searchRc)
-    return searchRc;
   if (rc)
     return rc;
   u64 tests = 0, rechecks = 0;
@@ -1922,10 +1906,7 @@ static int collide_impl(const TreeState& a, const TreeState& b, bool self, doubl
     collide_filter_kernel<T><<<blocks_for(m, 128), 128, 0, st>>>(struct_view<T>(a), struct_view<T>(b), self ? 1 : 0, c.items.as<u64>(), m, tl,
                                                                   keys.as<u64>(), kept.as<unsigned long long>());
   unsigned long long k = 0;
-  e = cudaMemcpyAsync(&k, kept.p, sizeof(k), cudaMemcpyDeviceToHost, st);
-  if (!e)
-    e = cudaStreamSynchronize(st);
-  if (e)
+  if ((e = read_back(&k, kept.p, sizeof(k), st)))
     return cuda_status(e, "filtering pairs");
   swap(c.items, keys);
   c.m = k;

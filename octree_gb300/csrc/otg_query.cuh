@@ -53,6 +53,7 @@ struct Appender
   double* dist;    // optional
   unsigned long long* count;
   u64 capacity;
+  bool cleared = false; // the work buffer's counters were cleared with the count
   __device__ __forceinline__ void put(u32 q, u32 id, double d = 0.0)
   {
     u64 pos = atomicAdd(count, 1ull);

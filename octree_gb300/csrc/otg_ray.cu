@@ -555,7 +555,8 @@ int ray_first(const TreeView<T>& tv, bool near, const T* rays, u32 nq, T tol, T 
     }
     near = near && a.prep;
   }
-  cudaMemsetAsync(work, 0, sizeof(u32) * 4, st);
+  if (!out.cleared)
+    cudaMemsetAsync(work, 0, sizeof(u32) * 4, st);
   u32 grid = 0;
   if (near)
   {

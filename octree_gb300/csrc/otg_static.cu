@@ -357,9 +357,7 @@ int export_static_impl(TreeState& t, otg_static_layout* out, cudaStream_t st)
   StaticCtl h;
   e = cudaGetLastError();
   if (!e)
-    e = cudaMemcpyAsync(&h, ctl, sizeof(StaticCtl), cudaMemcpyDeviceToHost, st);
-  if (!e)
-    e = cudaStreamSynchronize(st);
+    e = read_back(&h, ctl, sizeof(StaticCtl), st);
   if (e)
     return cuda_status(e, "computing the static layout");
   if (h.err)
@@ -430,10 +428,7 @@ int export_static(TreeState& t, otg_static_layout* out, cudaStream_t st)
   {
     // a point outside the space has the root's location and sorts first (key 0)
     u64 first = 0;
-    cudaError_t e = cudaMemcpyAsync(&first, t.sortedKeys, t.keys32 ? 4 : 8, cudaMemcpyDeviceToHost, st);
-    if (!e)
-      e = cudaStreamSynchronize(st);
-    if (e)
+    if (cudaError_t e = read_back(&first, t.sortedKeys, t.keys32 ? 4 : 8, st))
       return cuda_status(e, "reading the first location");
     if (first == 0)
     {

@@ -100,3 +100,21 @@ def test_dense_ids_of_a_forest():
         lists.append(np.flatnonzero((x >= lo[q]) & (x <= hi[q])))
     eo, ei = csr(lists)
     assert np.array_equal(got[0], eo) and np.array_equal(got[1], ei)
+
+
+@pytest.mark.parametrize("nq", [1, 1023, 1024, 1025, 16384, 16385, 40_000])
+def test_query_counts(nq):
+    """Offsets scanned by one block up to 16384 queries, by tiles above; results read back through the pinned block
+    and, above its 256 KiB, directly."""
+    rng = np.random.default_rng(23)
+    x = np.sort(rng.integers(0, 1 << 16, 5000))
+    pts = np.stack([x / 64.0, np.full(len(x), 0.5), np.full(len(x), 0.5)], 1)
+    t = otg.Tree("points").create(pts, max_depth=10, max_elements=8)
+    lo = rng.integers(0, 1 << 16, nq)
+    hi = lo + rng.integers(1, 200, nq)
+    r = np.zeros((nq, 6))
+    r[:, 0], r[:, 3], r[:, 4:] = lo / 64.0 - 1 / 128, hi / 64.0 - 1 / 128, 1
+    off, ids, _ = t.range_search(r, tol=0.0)
+    a, b = np.searchsorted(x, lo), np.searchsorted(x, hi)
+    assert np.array_equal(off, np.concatenate([[0], np.cumsum(b - a)]))
+    assert np.array_equal(ids, np.concatenate([np.arange(i, j) for i, j in zip(a, b)]))
