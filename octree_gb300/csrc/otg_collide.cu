@@ -8,8 +8,8 @@
 // box first and then box by box. Entities of shallow nodes (large boxes, long walks, little in common)
 // come first, one to a packet; packets are taken from a shared counter.
 // Bound by instruction issue and by the latency of the node loads. One entity per warp spends a walk of
-// the upper levels on every box: 4M clustered FP64 boxes with themselves took 6.67 ms and now take 1.90 ms,
-// 8M against 16M 9.39 and 2.24 ms.
+// the upper levels on every box: 4M clustered FP64 boxes with themselves took 6.67 ms and now take 1.55 ms,
+// 8M against 16M 9.39 and 1.89 ms.
 //
 // The test runs on FP32 images of the second tree's boxes, lo = rd(min) and hi = ru(max). With M the
 // largest coordinate of the two root boxes and of the first box, and G = 2^-20 (M + tol), four bounds per dimension of the
@@ -32,6 +32,9 @@ namespace otg
 {
 
 constexpr u32 kPairBuf = 128;
+// Subtrees of at most this many entities are tested without their nodes. 4M clustered boxes of 32 per node with
+// themselves: 1.98 ms at 0, 1.83 at 64, 1.73 at 128 (searches of 16M boxes of 16 per node stay within 1%).
+constexpr u32 kDirectBoxes = 128;
 
 struct CollideCounters
 {
@@ -55,7 +58,9 @@ struct CollideArgs
   const T* geomB;
   const uint4* linkB;
   const float4* nodeB; // per node {min rounded down}, {max rounded up}
+  const u32* ownerB;
   u32 nB, nNodesB;
+  u32 direct;          // subtrees of at most this many entities are tested without their nodes
   u32 stackCap;        // entries of a warp's stack
   T tol;
   int selfMode;
@@ -76,6 +81,7 @@ struct CollideWarpMem
 {
   float4 box[32][4];
   float4 child[8][2];
+  float4 common[2]; // the packet's common bounds
   u64 pairs[kPairBuf];
 };
 static_assert(sizeof(CollideWarpMem) % 16 == 0, "warps' parts start on 16 bytes");
@@ -95,8 +101,11 @@ __device__ __noinline__ bool boxes_overlap_exact(const T* a, const T* b, T tol)
   return GeoD<T>::box_relation(ea, eb, tol) == -1;
 }
 
+// 64 registers and 32 warps per SM, with the children's boxes loaded after the entities and the common box in shared
+// memory: 1.55 and 1.89 ms on the two workloads above. The children on their way during the entities: 1.73 and
+// 2.17 ms; at 80 to 96 registers and 24 warps 1.76 and 2.20; 40 warps spill (1.88 and 2.17).
 template<typename T, int WARPS>
-__global__ void __launch_bounds__(WARPS * 32) collide_packet_kernel(CollideArgs<T> a)
+__global__ void __launch_bounds__(WARPS * 32, 32 / WARPS) collide_packet_kernel(CollideArgs<T> a)
 {
   extern __shared__ __align__(16) unsigned char collideMem[];
   const u32 lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -195,6 +204,11 @@ __global__ void __launch_bounds__(WARPS * 32) collide_packet_kernel(CollideArgs<
     const u32 all = __ballot_sync(~0u, valid);
     if (!all)
       continue;
+    if (lane == 0)
+    {
+      W.common[0] = u0;
+      W.common[1] = u1;
+    }
     u32 sp = 1, visits = 0, nbuf = 0;
     bool bad = false;
     if (lane == 0)
@@ -209,34 +223,27 @@ __global__ void __launch_bounds__(WARPS * 32) collide_packet_kernel(CollideArgs<
       const uint4 L = stackL[sp];
       const u32 mask = stackM[sp];
       __syncwarp();
-      const u32 fc = L.x & kFirstChildMask, cc = L.x >> kChildShift;
-      if (L.z > a.nB || L.y > L.z || ++visits > a.nNodesB || cc > 8u || u64(fc) + cc > a.nNodesB || sp + cc > a.stackCap)
+      // A subtree of few entities is one run of the tree order, tested as it comes instead of by its nodes
+      // (boxes that overlap also overlap each other's nodes, so this adds no pair).
+      const bool whole = L.w - L.y <= a.direct;
+      const u32 end = whole ? L.w : L.z;
+      const u32 fc = L.x & kFirstChildMask, cc = whole ? 0u : L.x >> kChildShift;
+      if (L.z > a.nB || L.y > L.z || L.w > a.nB || ++visits > a.nNodesB || cc > 8u || u64(fc) + cc > a.nNodesB || sp + cc > a.stackCap)
       {
         bad = true;
         break;
       }
-      // the children's boxes and links on their way while the entities are tested
-      float4 cl = make_float4(0.f, 0.f, 0.f, 0.f), ch = cl;
-      uint4 cL = make_uint4(0u, 0u, 0u, 0u);
-      if (lane < cc)
-      {
-        cl = a.nodeB[2 * size_t(fc + lane)];
-        ch = a.nodeB[2 * size_t(fc + lane) + 1];
-        cL = a.linkB[fc + lane];
-        if (!a.sure)
-          ch = make_float4(__fadd_ru(ch.x, a.tolHi), __fadd_ru(ch.y, a.tolHi), __fadd_ru(ch.z, a.tolHi), 0.f);
-      }
       const u32 jb = a.selfMode ? max(L.y, iMin + 1) : L.y;
-      for (u32 base = jb; base < L.z; base += 32)
+      for (u32 base = jb; base < end; base += 32)
       {
         const u32 j = base + lane;
         bool in = false;
         float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
-        if (j < L.z)
+        if (j < end)
         {
           lo = a.imgB[2 * size_t(j)];
           hi = a.imgB[2 * size_t(j) + 1];
-          in = !apart(u0, u1, lo, hi);
+          in = !apart(W.common[0], W.common[1], lo, hi);
         }
         if (!__any_sync(~0u, in))
           continue;
@@ -260,6 +267,9 @@ __global__ void __launch_bounds__(WARPS * 32) collide_packet_kernel(CollideArgs<
               hit = boxes_overlap_exact<T>(a.geomA + u64(il) * 6, a.geomB + u64(j) * 6, a.tol);
               ++rechecks;
             }
+            // a subtree's run may hold entities of no reachable node
+            if (hit && whole)
+              hit = a.ownerB[j] != kNoOwner;
           }
           const u32 bal = __ballot_sync(~0u, hit);
           if (!bal)
@@ -280,8 +290,19 @@ __global__ void __launch_bounds__(WARPS * 32) collide_packet_kernel(CollideArgs<
       }
       if (cc)
       {
+      // the children's boxes and links
+      float4 cl = make_float4(0.f, 0.f, 0.f, 0.f), ch = cl;
+      uint4 cL = make_uint4(0u, 0u, 0u, 0u);
+      if (lane < cc)
+      {
+        cl = a.nodeB[2 * size_t(fc + lane)];
+        ch = a.nodeB[2 * size_t(fc + lane) + 1];
+        cL = a.linkB[fc + lane];
+        if (!a.sure)
+          ch = make_float4(__fadd_ru(ch.x, a.tolHi), __fadd_ru(ch.y, a.tolHi), __fadd_ru(ch.z, a.tolHi), 0.f);
+      }
         // the subtree must reach the packet's box, and in a single tree hold a position after its first
-        const bool ok = lane < cc && !apart(u0, u1, cl, ch) && (!a.selfMode || cL.w > iMin + 1);
+        const bool ok = lane < cc && !apart(W.common[0], W.common[1], cl, ch) && (!a.selfMode || cL.w > iMin + 1);
         u32 bal = __ballot_sync(~0u, ok);
         if (ok)
         {
@@ -420,6 +441,8 @@ static int collide_search_impl(TreeState& A, TreeState& B, bool self, bool swapO
   a.selfMode = self ? 1 : 0;
   a.swapOut = swapOut ? 1 : 0;
   a.sure = !A.respanned && !B.respanned;
+  a.direct = a.sure ? kDirectBoxes : 0u;
+  a.ownerB = B.ownerNode.as<u32>();
   a.tolHi = float(a.tol);
   if (double(a.tolHi) < double(a.tol))
     a.tolHi = std::nextafter(a.tolHi, __builtin_huge_valf());
