@@ -290,17 +290,17 @@ __global__ void __launch_bounds__(WARPS * 32, 32 / WARPS) collide_packet_kernel(
       }
       if (cc)
       {
-      // the children's boxes and links
-      float4 cl = make_float4(0.f, 0.f, 0.f, 0.f), ch = cl;
-      uint4 cL = make_uint4(0u, 0u, 0u, 0u);
-      if (lane < cc)
-      {
-        cl = a.nodeB[2 * size_t(fc + lane)];
-        ch = a.nodeB[2 * size_t(fc + lane) + 1];
-        cL = a.linkB[fc + lane];
-        if (!a.sure)
-          ch = make_float4(__fadd_ru(ch.x, a.tolHi), __fadd_ru(ch.y, a.tolHi), __fadd_ru(ch.z, a.tolHi), 0.f);
-      }
+        // the children's boxes and links
+        float4 cl = make_float4(0.f, 0.f, 0.f, 0.f), ch = cl;
+        uint4 cL = make_uint4(0u, 0u, 0u, 0u);
+        if (lane < cc)
+        {
+          cl = a.nodeB[2 * size_t(fc + lane)];
+          ch = a.nodeB[2 * size_t(fc + lane) + 1];
+          cL = a.linkB[fc + lane];
+          if (!a.sure)
+            ch = make_float4(__fadd_ru(ch.x, a.tolHi), __fadd_ru(ch.y, a.tolHi), __fadd_ru(ch.z, a.tolHi), 0.f);
+        }
         // the subtree must reach the packet's box, and in a single tree hold a position after its first
         const bool ok = lane < cc && !apart(W.common[0], W.common[1], cl, ch) && (!a.selfMode || cL.w > iMin + 1);
         u32 bal = __ballot_sync(~0u, ok);

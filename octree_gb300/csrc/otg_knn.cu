@@ -21,7 +21,8 @@
 // Bound by instruction issue: a query of k = 32 visits about ten subtrees of the tree's lower levels and
 // tests a few hundred points in FP32, then takes k exact distances (FP64 square roots) and orders them.
 // 1M queries, k in 1..64, 16M points: 14.2 ms with leaf-by-leaf tests and shared-memory sorts for the bound and
-// the order, 10.1 ms with bisection and register sorts, 6.8 ms with small subtrees tested whole.
+// the order, 10.1 ms with bisection and register sorts, 6.8 ms with small subtrees tested whole,
+// 6.55 ms with the pivots of knn_kth_bound and 40 warps per SM.
 #include "otg_query.cuh"
 
 #include <cfloat>
@@ -341,45 +342,52 @@ __device__ __forceinline__ void warp_order_pairs(unsigned long long* k, u32* v, 
   }
 }
 
-// An upper bound of the k-th least hi2 in the buffer, infinite with fewer than k below F0lo2: bisection on
-// the float bits (ordered like the values, which are not negative). Stops once exactly k values lie
-// below, or after `steps` halvings; a sort of the buffer took four times the instructions.
-template<typename T, int CAP>
-__device__ __forceinline__ float knn_kth_bound(const KnnWarpMem<CAP>& W, float F0lo2, u32 k, u32 lane, u32 bufN, int steps)
+// An upper bound of the k-th least of the bufN <= C * 32 values that are below F0lo2, infinite with fewer than k of
+// them: bisection on the float bits (ordered like the values, which are not negative). Squared distances of
+// points spread evenly grow with the 2/3 power of their rank, so the first two pivots bracket that
+// estimate. Stops once at most k + 1 values lie below, or after `steps` pivots.
+template<int C>
+__device__ __forceinline__ float knn_kth_bound(const float* hi2, float F0lo2, u32 k, u32 lane, u32 bufN, int steps)
 {
-  u32 h[CAP / 32];
+  u32 h[C];
   u32 lo = 0x7f800000u, hi = 0, finite = 0;
 #pragma unroll
-  for (int c = 0; c < CAP / 32; ++c)
+  for (int c = 0; c < C; ++c)
   {
     h[c] = 0x7f800000u;
-    if (u32(c) * 32 < bufN)
+    const u32 i = c * 32 + lane;
+    if (i < bufN)
     {
-      const u32 i = c * 32 + lane;
-      if (i < bufN && W.hi2[i] < F0lo2)
+      const float v = hi2[i];
+      if (v < F0lo2)
       {
-        h[c] = __float_as_uint(W.hi2[i]);
+        h[c] = __float_as_uint(v);
         lo = min(lo, h[c]);
         if (h[c] < 0x7f800000u)
           hi = max(hi, h[c]);
       }
-      finite += __popc(__ballot_sync(~0u, h[c] < 0x7f800000u));
     }
+    finite += __popc(__ballot_sync(~0u, h[c] < 0x7f800000u));
   }
   if (finite < k)
     return kInf;
   lo = __reduce_min_sync(~0u, lo);
   hi = __reduce_max_sync(~0u, hi);
+  const float guess = __uint_as_float(hi) * exp2f(log2f(float(k) / float(finite)) * (2.f / 3.f));
   // count(<= hi) >= k throughout
   u32 above = finite;
-  while (steps-- > 0 && above > k && lo < hi)
+  for (int s = 0; s < steps && above > k + 1 && lo < hi; ++s)
   {
-    const u32 mid = lo + ((hi - lo) >> 1);
+    u32 mid = lo + ((hi - lo) >> 1);
+    if (s < 2)
+    {
+      const u32 g = __float_as_uint(guess * (s == 0 ? 1.1f : 0.9f));
+      mid = g > lo && g < hi ? g : mid;
+    }
     u32 n = 0;
 #pragma unroll
-    for (int c = 0; c < CAP / 32; ++c)
-      if (u32(c) * 32 < bufN)
-        n += __popc(__ballot_sync(~0u, h[c] <= mid));
+    for (int c = 0; c < C; ++c)
+      n += __popc(__ballot_sync(~0u, h[c] <= mid));
     if (n >= k)
     {
       hi = mid;
@@ -397,7 +405,10 @@ __device__ __forceinline__ void knn_flush(KnnWarpMem<CAP>& W, const KnnArgs<T>& 
 {
   __syncwarp();
   // round-to-nearest with a 2^-20 margin per step keeps every value an upper bound
-  const float R2 = knn_kth_bound<T, CAP>(W, a.F0lo2, k, lane, bufN, steps);
+  // (the buffer's size picks the count of values per lane: 2 or 4 in most queries)
+  const float R2 = bufN <= 64    ? knn_kth_bound<2>(W.hi2, a.F0lo2, k, lane, bufN, steps)
+                   : bufN <= 128 ? knn_kth_bound<4>(W.hi2, a.F0lo2, k, lane, bufN, steps)
+                                 : knn_kth_bound<CAP / 32>(W.hi2, a.F0lo2, k, lane, bufN, steps);
   const float Rhi = sqrtf(R2) * (1.f + 0x1p-20f);
   const float Fc = fmaxf(a.tolHi, fminf(Rhi, a.F0hi) * a.onePlusTolHi);
   const float nFc2 = (Fc * Fc) * (1.f + 0x1p-20f);
@@ -432,8 +443,10 @@ __device__ __forceinline__ void knn_flush(KnnWarpMem<CAP>& W, const KnnArgs<T>& 
   bufN = kept;
 }
 
+// 40 warps per SM (48 registers, some spills): 1M queries, k in 1..64, 16M points 6.55 ms; 7.22 at 64 to 80 registers and
+// 24 to 32 warps, 7.03 with 48 warps.
 template<typename T, int CAP, int WARPS>
-__global__ void __launch_bounds__(WARPS * 32) knn_filtered_kernel(KnnArgs<T> a)
+__global__ void __launch_bounds__(WARPS * 32, 40 / WARPS) knn_filtered_kernel(KnnArgs<T> a)
 {
   extern __shared__ __align__(16) unsigned char smem[];
   const u32 lane = threadIdx.x & 31;
