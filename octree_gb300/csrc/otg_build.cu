@@ -602,6 +602,38 @@ __device__ __forceinline__ u64 entity_key(const T* e, const typename Ord<T>::U* 
   }
 }
 
+// The digits that a build sorts its keys by: `bits` key bits, of a box key without the depth bits that a
+// tree of depth D leaves zero. A box larger than its space by rounding has the depth -1: all bits above the depth
+// are ones then, and the 32-bit key is above every other's with or without them. In a 64-bit key those
+// ones are those of a cell, where the depth's upper bits order it after the cell's own; such keys keep all bits.
+template<typename K, bool IS_BOX>
+static RadixPlan build_radix_plan(u32 bits, u32 D)
+{
+  if (!IS_BOX || sizeof(K) == 8)
+    return radix_plan(bits, 0, 0, sizeof(K) == 4);
+  u32 low = 1;
+  while ((D >> low) != 0)
+    ++low;
+  return radix_plan(bits, low, 5 - low, true);
+}
+constexpr u32 kHistWords = kMaxPasses * kRadix; // at most eight narrow passes, or four wide ones
+
+// one count for each pass's digit of a key (the plan's numbers at constant indexes: uniform registers)
+template<typename K, bool IS_BOX>
+__device__ __forceinline__ void count_digits(u32* sh, const RadixPlan& plan, K k)
+{
+#pragma unroll
+  for (u32 p = 0; p < (sizeof(K) == 4 ? 4u : kMaxPasses); ++p)
+    if (p < plan.passes)
+    {
+      const SortDigit& g = plan.digit[p];
+      u32 d = u32(k >> g.shift) & (plan.radix - 1);
+      if (IS_BOX && sizeof(K) == 4 && p == 0)
+        d = (u32(k) & g.keep) | (d & ~g.keep);
+      atomicAdd(&sh[p * plan.radix + d], 1u);
+    }
+}
+
 // STAGED (16-byte aligned entities): whole tiles of 256 chunks (12 KB) arrive in shared memory by
 // bulk copies (cp.async.bulk, completion on an mbarrier), two buffers deep, while the previous tile
 // is coded; each thread reads its 48-byte chunk from shared memory. The chunks after the last whole
@@ -611,21 +643,21 @@ constexpr u32 kCodegenTileBytes = kCodegenTileChunks * 48;
 template<typename T, typename R, typename K, bool IS_BOX, bool STAGED = false>
 __global__ void __launch_bounds__(256) codegen_kernel(const T* __restrict__ ent, u64 n, bool vec, const Space<T>* __restrict__ spg,
                                                       const typename Ord<T>::U* __restrict__ tabG, u32 cells, int tabInSmem,
-                                                      K* __restrict__ keys, u32* __restrict__ hist, u32 passes, bool regular, u32* __restrict__ err,
-                                                      u32 stageOff = 0)
+                                                      K* __restrict__ keys, u32* __restrict__ hist, RadixPlan plan, bool regular,
+                                                      u32* __restrict__ err, u32 stageOff = 0)
 {
   using O = Ord<T>;
   using U = typename O::U;
   constexpr int W = IS_BOX ? 6 : 3;
   constexpr int E = Chunk<T, W>::E;
   extern __shared__ __align__(16) unsigned char s_dyn[];
-  __shared__ u32 sh[8][kRadix];
+  __shared__ u32 sh[kHistWords];
   __shared__ float minF[3], rastF[3], margF[3];
   __shared__ u32 sD;
   const size_t perDim = RasterLayout<T>::per_dim(cells);
   U* stab = reinterpret_cast<U*>(s_dyn);
-  for (int i = threadIdx.x; i < 8 * kRadix; i += blockDim.x)
-    (&sh[0][0])[i] = 0;
+  for (u32 i = threadIdx.x; i < plan.passes * plan.radix; i += blockDim.x)
+    sh[i] = 0;
   if (tabInSmem)
     for (size_t i = threadIdx.x; i < 3 * perDim; i += blockDim.x)
       stab[i] = tabG[i];
@@ -662,8 +694,7 @@ __global__ void __launch_bounds__(256) codegen_kernel(const T* __restrict__ ent,
       else
         kk = K(entity_key<T, IS_BOX, sizeof(K) == 4>(v + k * W, tab, perDim, cells, minF, rastF, D, margF));
       keys[c * E + k] = kk;
-      for (u32 p = 0; p < passes; ++p)
-        atomicAdd(&sh[p][(kk >> (kRadixBits * p)) & (kRadix - 1)], 1u);
+      count_digits<K, IS_BOX>(sh, plan, kk);
     }
   };
   u64 firstDirect = 0;
@@ -749,10 +780,9 @@ __global__ void __launch_bounds__(256) codegen_kernel(const T* __restrict__ ent,
     code(v, c, cnt);
   }
   __syncthreads();
-  for (u32 p = 0; p < passes; ++p)
-    for (int d = threadIdx.x; d < kRadix; d += blockDim.x)
-      if (sh[p][d])
-        atomicAdd(&hist[p * kRadix + d], sh[p][d]);
+  for (u32 i = threadIdx.x; i < plan.passes * plan.radix; i += blockDim.x)
+    if (sh[i])
+      atomicAdd(&hist[i], sh[i]);
 }
 
 // per-entity location keys in input order, reference layout (loc << 5 | depth), computed with the
@@ -1509,7 +1539,7 @@ static int build_impl(TreeState& t, const T* ent, const void* box, u64 n, cudaSt
   // sorted key bits: a loose box centred on the max face of its space has the out-of-grid cell 2^D
   // in up to three dimensions, so its key can hold three bits above 3D + 5
   const u32 sortBits = IS_BOX ? std::min(3 * D + 8, u32(8 * sizeof(K))) : bits;
-  const u32 passes = chunked ? 0u : (sortBits + kRadixBits - 1) / kRadixBits;
+  const RadixPlan plan = chunked ? RadixPlan{} : build_radix_plan<K, IS_BOX>(sortBits, D);
   const u32 cells = IS_BOX ? (1u << D) + 2 : (1u << D);
   const size_t tabBytes = RasterLayout<T>::bytes(cells);
   const u64 minTabEntries = IS_BOX ? 1 : 3 * ((u64(2) << D) - 1);
@@ -1523,7 +1553,7 @@ static int build_impl(TreeState& t, const T* ent, const void* box, u64 n, cudaSt
       (e = t.nodeKey.ensure(sizeof(u64) * maxNodes)) || (e = t.nodeBox.ensure(sizeof(T) * 6 * maxNodes)) ||
       (e = t.nodeDepth.ensure(maxNodes)) || (e = t.levelCount.ensure(sizeof(u32) * 64)) ||
       (e = t.splitQueue.ensure(2 * sizeof(u32) * (n / (t.maxElem + 1) + 2))) || (e = t.space.ensure(sizeof(Space<T>))) ||
-      (e = t.sortScratch.ensure(chunked ? ChunkScratch::bytes() : SortScratch::bytes(n, passes))) || (e = t.bboxBits.ensure(sizeof(U) * 6)) ||
+      (e = t.sortScratch.ensure(chunked ? ChunkScratch::bytes() : SortScratch::bytes(n, plan.passes, plan.radix))) || (e = t.bboxBits.ensure(sizeof(U) * 6)) ||
       (e = t.rasterTab.ensure(tabBytes)) || (e = t.minTab.ensure(sizeof(T) * minTabEntries)) ||
       (IS_BOX && ((e = t.nodeMax.ensure(sizeof(T) * 3 * maxNodes)) || (e = t.ownerNode.ensure(sizeof(u32) * n)) ||
                   (e = t.nodeParent.ensure(sizeof(u32) * maxNodes)))))
@@ -1541,8 +1571,8 @@ static int build_impl(TreeState& t, const T* ent, const void* box, u64 n, cudaSt
   }
   else
   {
-    ss.carve(t.sortScratch.p, n, passes);
-    cudaMemsetAsync(t.sortScratch.p, 0, SortScratch::bytes(n, passes), st);
+    ss.carve(t.sortScratch.p, n, plan.passes, plan.radix);
+    cudaMemsetAsync(t.sortScratch.p, 0, SortScratch::bytes(n, plan.passes, plan.radix), st);
   }
   cudaMemsetAsync(t.levelCount.p, 0, sizeof(u32) * 64, st);
 
@@ -1600,7 +1630,7 @@ static int build_impl(TreeState& t, const T* ent, const void* box, u64 n, cudaSt
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kfn, 256, cgSmem);
     cgBlocks = std::max(1, std::min(cgBlocks, std::max(perSm, 1) * std::max(sms, 1)));
   }
-  kfn<<<cgBlocks, 256, cgSmem, st>>>(ent, n, vec, sp, tab, cells, tabInSmem, t.keysA.as<K>(), ss.hist, passes, regular, t.err.as<u32>(), stageOff);
+  kfn<<<cgBlocks, 256, cgSmem, st>>>(ent, n, vec, sp, tab, cells, tabInSmem, t.keysA.as<K>(), ss.hist, plan, regular, t.err.as<u32>(), stageOff);
 
   prof.mark("sort", st);
   bool inB = false;
@@ -1611,7 +1641,7 @@ static int build_impl(TreeState& t, const T* ent, const void* box, u64 n, cudaSt
       return rc;
   }
   else
-    inB = onesweep_passes<K>(t.keysA.as<K>(), t.sortedIds.as<u32>(), t.keysB.as<K>(), t.valsB.as<u32>(), n, 0, passes, true, ss, t.err.as<u32>(), st);
+    inB = onesweep_passes<K>(t.keysA.as<K>(), t.sortedIds.as<u32>(), t.keysB.as<K>(), t.valsB.as<u32>(), n, plan, true, ss, t.err.as<u32>(), st);
   if (inB)
   {
     std::swap(t.sortedIds, t.valsB);
@@ -1940,12 +1970,12 @@ template<typename T, typename K, bool IS_BOX>
 __global__ void __launch_bounds__(256) forest_codegen_kernel(const T* __restrict__ ent, const uint2* __restrict__ segTiles, const u64* __restrict__ off,
                                                              const Space<T>* __restrict__ sp, const typename Ord<T>::U* __restrict__ tabG,
                                                              const u64* __restrict__ tabOff, int tabInSmem, K* __restrict__ keys, u32* __restrict__ hist,
-                                                             u32 trees, u32 passes, bool regular, u32* __restrict__ err)
+                                                             u32 trees, RadixPlan plan, bool regular, u32* __restrict__ err)
 {
   using U = typename Ord<T>::U;
   constexpr int W = IS_BOX ? 6 : 3;
   extern __shared__ __align__(16) unsigned char s_dyn[];
-  __shared__ u32 sh[8][kRadix];
+  __shared__ u32 sh[kHistWords];
   __shared__ float minF[3], rastF[3], margF[3];
   const uint2 st = segTiles[blockIdx.x];
   const u32 tr = st.x;
@@ -1955,8 +1985,8 @@ __global__ void __launch_bounds__(256) forest_codegen_kernel(const T* __restrict
   const size_t perDim = RasterLayout<T>::per_dim(cells);
   const U* tab = tabG + tabOff[tr];
   U* stab = reinterpret_cast<U*>(s_dyn);
-  for (int i = threadIdx.x; i < 8 * kRadix; i += blockDim.x)
-    (&sh[0][0])[i] = 0;
+  for (u32 i = threadIdx.x; i < plan.passes * plan.radix; i += blockDim.x)
+    sh[i] = 0;
   if (tabInSmem)
     for (size_t i = threadIdx.x; i < 3 * perDim; i += blockDim.x)
       stab[i] = tab[i];
@@ -1992,14 +2022,13 @@ __global__ void __launch_bounds__(256) forest_codegen_kernel(const T* __restrict
     else
       kk = K(entity_key<T, IS_BOX, sizeof(K) == 4>(v, tab, perDim, cells, minF, rastF, D, margF));
     keys[i] = kk;
-    for (u32 p = 0; p < passes; ++p)
-      atomicAdd(&sh[p][(kk >> (kRadixBits * p)) & (kRadix - 1)], 1u);
+    count_digits<K, IS_BOX>(sh, plan, kk);
   }
   __syncthreads();
-  for (u32 p = 0; p < passes; ++p)
-    for (int d = threadIdx.x; d < kRadix; d += blockDim.x)
-      if (sh[p][d])
-        atomicAdd(&hist[(u64(p) * trees + tr) * kRadix + d], sh[p][d]);
+  for (u32 p = 0; p < plan.passes; ++p)
+    for (u32 d = threadIdx.x; d < plan.radix; d += blockDim.x)
+      if (const u32 c = sh[p * plan.radix + d])
+        atomicAdd(&hist[(u64(p) * trees + tr) * plan.radix + d], c);
 }
 
 __global__ void forest_root_init_kernel(uint4* link, u64* nodeKey, unsigned char* nodeDepth, u32* levelCount, const u64* __restrict__ off, u32 trees,
@@ -2031,7 +2060,8 @@ static int forest_build_impl(TreeState& t, const T* ent, const T* boxes, cudaStr
   const u32 Dmax = t.D;
   // sorted key bits (out-of-grid loose-box locations: three bits above 3D + 5)
   const u32 bits = IS_BOX ? std::min(3 * Dmax + 8, u32(8 * sizeof(K))) : 3 * Dmax + 1;
-  const u32 passes = (bits + kRadixBits - 1) / kRadixBits;
+  const RadixPlan plan = build_radix_plan<K, IS_BOX>(bits, Dmax);
+  const u32 passes = plan.passes;
   const u32 tiles = u32(t.segTilesHost.size());
   const u64 tabEntries = t.tabOffHost.back();
   const u64 minEntries = IS_BOX ? 1 : t.minOffHost.back();
@@ -2041,8 +2071,8 @@ static int forest_build_impl(TreeState& t, const T* ent, const T* boxes, cudaStr
   const size_t maxTabBytes = sizeof(U) * maxTab;
   const u64 maxNodes = n + trees + u64(Dmax) * (n / (t.maxElem + 1) + 1) + 2;
   t.maxNodes = maxNodes;
-  const size_t histWords = size_t(passes) * trees * kRadix;
-  const size_t scratchWords = histWords + size_t(passes) * std::max<u32>(tiles, 1) * kRadix + passes + 8;
+  const size_t histWords = size_t(passes) * trees * plan.radix;
+  const size_t scratchWords = histWords + size_t(passes) * std::max<u32>(tiles, 1) * plan.radix + passes + 8;
   cudaError_t e;
   if (!launchOnly)
   {
@@ -2097,19 +2127,19 @@ static int forest_build_impl(TreeState& t, const T* ent, const T* boxes, cudaStr
   u32* scratch = t.sortScratch.as<u32>();
   u32* hist = scratch;
   u32* status = scratch + histWords;
-  u32* counters = status + size_t(passes) * std::max<u32>(tiles, 1) * kRadix;
+  u32* counters = status + size_t(passes) * std::max<u32>(tiles, 1) * plan.radix;
   const int tabInSmem = maxTabBytes <= 64 * 1024 ? 1 : 0;
   const size_t cgSmem = tabInSmem ? maxTabBytes : 0;
   if (tiles)
   {
     auto kfn = forest_codegen_kernel<T, K, IS_BOX>;
     cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(cgSmem));
-    kfn<<<tiles, 256, cgSmem, st>>>(ent, segTiles, off, sp, t.rasterTab.as<U>(), t.tabOff.as<u64>(), tabInSmem, t.keysA.as<K>(), hist, trees, passes,
+    kfn<<<tiles, 256, cgSmem, st>>>(ent, segTiles, off, sp, t.rasterTab.as<U>(), t.tabOff.as<u64>(), tabInSmem, t.keysA.as<K>(), hist, trees, plan,
                                     regular, t.err.as<u32>());
   }
 
   prof.mark("sort", st);
-  const bool inB = onesweep_passes_segmented<K>(t.keysA.as<K>(), t.sortedIds.as<u32>(), t.keysB.as<K>(), t.valsB.as<u32>(), n, passes, true, segTiles,
+  const bool inB = onesweep_passes_segmented<K>(t.keysA.as<K>(), t.sortedIds.as<u32>(), t.keysB.as<K>(), t.valsB.as<u32>(), n, plan, true, segTiles,
                                                 tiles, off, trees, hist, status, counters, t.err.as<u32>(), st);
   if (inB)
   {

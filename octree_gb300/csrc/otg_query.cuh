@@ -262,7 +262,7 @@ static inline int sort_pairs_u64(u64* keys, u32* vals, u64 m, u32 bits, cudaStre
   SortScratch ss;
   ss.carve(scratch.p, m, passes);
   radix_histogram_kernel<u64><<<blocks_for(m), 256, 0, st>>>(keys, m, 0, passes, ss.hist);
-  bool inB = onesweep_passes<u64>(keys, vals, k1.as<u64>(), v1.as<u32>(), m, 0, passes, false, ss, err, st);
+  bool inB = onesweep_passes<u64>(keys, vals, k1.as<u64>(), v1.as<u32>(), m, passes, false, ss, err, st);
   if (inB)
   {
     cudaMemcpyAsync(keys, k1.p, sizeof(u64) * m, cudaMemcpyDeviceToDevice, st);
@@ -285,7 +285,7 @@ static inline int sort_pairs_u32(u32* keys, u32* vals, u64 m, u32 bits, cudaStre
   SortScratch ss;
   ss.carve(scratch.p, m, passes);
   radix_histogram_kernel<u32><<<blocks_for(m), 256, 0, st>>>(keys, m, 0, passes, ss.hist);
-  bool inB = onesweep_passes<u32>(keys, vals, k1.as<u32>(), v1.as<u32>(), m, 0, passes, false, ss, err, st);
+  bool inB = onesweep_passes<u32>(keys, vals, k1.as<u32>(), v1.as<u32>(), m, passes, false, ss, err, st);
   if (inB)
   {
     cudaMemcpyAsync(keys, k1.p, sizeof(u32) * m, cudaMemcpyDeviceToDevice, st);
