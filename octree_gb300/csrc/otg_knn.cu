@@ -533,12 +533,18 @@ __global__ void __launch_bounds__(WARPS * 32, 40 / WARPS) knn_filtered_kernel(Kn
     u32 visits = 0;
     while (sp > 0)
     {
-      --sp;
-      const u32 node = stackNode[sp];
-      const float w2 = stackW[sp];
-      __syncwarp();
-      if (w2 > Fc2)
+      // The topmost of the last 32 nodes that the bound has not passed since they were pushed. The walk is bound
+      // by issue: taking the stack's nodes one by one, and weighing children with two compares each, 6.92 ms for the
+      // 1M queries below, now 6.64; keeping the link of the next node at hand instead cost 15% (more registers).
+      const u32 open = __ballot_sync(~0u, lane < sp && !(stackW[sp - 1 - lane] > Fc2));
+      if (!open)
+      {
+        sp -= min(sp, 32u);
         continue;
+      }
+      sp -= u32(__ffs(int(open)));
+      const u32 node = stackNode[sp];
+      __syncwarp();
       if (++visits > a.nNodes)
       {
         overflow = true;
@@ -607,14 +613,12 @@ __global__ void __launch_bounds__(WARPS * 32, 40 / WARPS) knn_filtered_kernel(Kn
           ok = cw <= Fc2;
         }
         const u32 bal = __ballot_sync(~0u, ok);
+        // farthest first: a child's place is the number of open children farther away (ties: the higher lane); the bits
+        // of a weight order as it does, with the lane in the lowest three
+        const u32 wk = (__float_as_uint(cw) & ~7u) | lane;
         u32 rank = 0;
         for (u32 left = bal; left; left &= left - 1)
-        {
-          const u32 j = u32(__ffs(int(left))) - 1;
-          const float wj = __shfl_sync(~0u, cw, j);
-          if (wj > cw || (wj == cw && j > lane))
-            ++rank;
-        }
+          rank += __shfl_sync(~0u, wk, __ffs(int(left)) - 1) > wk;
         if (ok)
         {
           stackNode[sp + rank] = fc + lane;
