@@ -120,18 +120,201 @@ __device__ __forceinline__ void run_sort_lanes(RunKey<DIST>& v, u32 lane)
     }
 }
 
-// One warp per query sorts its run in place: each 32 items in registers, then every item's place is
-// its place among its 32 plus the counts of smaller items in the other sorted groups (binary
-// searches in shared memory). Runs above kRunSortMax go to the list longRuns (longCount[0] counts them)
-// for run_sort_block_kernel. A bitonic network over 128 items takes twice the steps.
+// ascending bitonic sort of R words per lane, word r of a lane at r * 32 + lane, of which the first n are not ~0
+template<int R>
+__device__ __forceinline__ void run_sort_words(u32 (&x)[R], u32 n, u32 lane)
+{
+#pragma unroll
+  for (u32 size = 2; size <= u32(R) * 32; size <<= 1)
+  {
+    if (R == 1 && size >= 2 * n)
+      break;
+#pragma unroll
+    for (u32 stride = size >> 1; stride > 0; stride >>= 1)
+    {
+      if (stride >= 32)
+      {
+#pragma unroll
+        for (u32 r = 0; r < u32(R); ++r)
+        {
+          const u32 o = r ^ (stride >> 5);
+          if (o > r)
+          {
+            const bool up = ((r * 32) & size) == 0;
+            const u32 a = min(x[r], x[o]), b = max(x[r], x[o]);
+            x[r] = up ? a : b;
+            x[o] = up ? b : a;
+          }
+        }
+      }
+      else
+      {
+#pragma unroll
+        for (u32 r = 0; r < u32(R); ++r)
+        {
+          const u32 o = __shfl_xor_sync(~0u, x[r], stride);
+          const bool up = ((r * 32 + lane) & size) == 0, lower = (lane & stride) == 0;
+          x[r] = (lower == up) ? min(x[r], o) : max(x[r], o);
+        }
+      }
+    }
+  }
+}
+// ascending order of n (at most R * 32) ids
+template<int R>
+__device__ __forceinline__ void run_order_ids(u32* ids, u32 n, u32 lane)
+{
+  u32 x[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+    x[r] = r * 32 + lane < n ? ids[r * 32 + lane] : ~0u;
+  run_sort_words<R>(x, n, lane);
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+    if (r * 32 + lane < n)
+      ids[r * 32 + lane] = x[r];
+}
+
+// (distance, id) order of n (2 to R * 32) items in shared memory by one warp; false if they need the general
+// order (run_order_general). Distances first become 24 bits, their place between the least and the greatest, with
+// their index below, and are sorted as one 32-bit word each: a bitonic step takes 4 instructions, on the 96-bit
+// items about 25. What the 24 bits leave in the wrong order (ties, of which a ray that starts inside several
+// boxes has a few at zero) shows when neighbours are compared, and a few odd-even rounds mend it.
+constexpr u32 kRunFixRounds = 6;
+template<int R>
+__device__ __forceinline__ bool run_order_packed(u64* sd, u32* si, u32 n, u32 lane)
+{
+  float f[R];
+  u32 mn = 0x7f800000u, mx = 0;
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+  {
+    const u32 i = r * 32 + lane;
+    f[r] = i < n ? __double2float_rn(__longlong_as_double((long long)sd[i])) : 0.f;
+    if (i < n)
+    {
+      mn = min(mn, __float_as_uint(f[r]));
+      mx = max(mx, __float_as_uint(f[r]));
+    }
+  }
+  mn = __reduce_min_sync(~0u, mn);
+  mx = __reduce_max_sync(~0u, mx);
+  const float f0 = __uint_as_float(mn), scale = 16777215.f / fmaxf(__uint_as_float(mx) - f0, 0x1p-100f);
+  u32 x[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+  {
+    const u32 i = r * 32 + lane;
+    x[r] = i < n ? (min(u32((f[r] - f0) * scale), 0xffffffu) << 8) | i : ~0u;
+  }
+  run_sort_words<R>(x, n, lane);
+  u64 d[R];
+  u32 id[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+  {
+    const u32 i = r * 32 + lane, from = x[r] & 255u;
+    d[r] = i < n ? sd[from] : 0;
+    id[r] = i < n ? si[from] : 0;
+  }
+  __syncwarp();
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+  {
+    const u32 i = r * 32 + lane;
+    if (i < n)
+    {
+      sd[i] = d[r];
+      si[i] = id[r];
+    }
+  }
+  __syncwarp();
+  for (u32 round = 0; round < kRunFixRounds; ++round)
+  {
+    u32 wrong = 0;
+    for (u32 i = lane; i + 1 < n; i += 32)
+    {
+      const RunKey<true> a{ sd[i], si[i] }, b{ sd[i + 1], si[i + 1] };
+      wrong += b.less(a);
+    }
+    wrong = __reduce_add_sync(~0u, wrong);
+    if (!wrong)
+      return true;
+    if (wrong > 2 * kRunFixRounds) // more ties than the rounds are likely to mend
+      return false;
+    for (u32 parity = 0; parity < 2; ++parity)
+    {
+      for (u32 i = 2 * lane + parity; i + 1 < n; i += 64)
+      {
+        const RunKey<true> a{ sd[i], si[i] }, b{ sd[i + 1], si[i + 1] };
+        if (b.less(a))
+        {
+          sd[i] = b.d;
+          si[i] = b.id;
+          sd[i + 1] = a.d;
+          si[i + 1] = a.id;
+        }
+      }
+      __syncwarp();
+    }
+  }
+  return false;
+}
+
 constexpr u32 kRunSortMax = 256;
 constexpr int kRunSortWarps = 8;
+// The general order of a run of at most kRunSortMax items: each 32 items in registers, then every item's place is
+// its place among its 32 plus the counts of smaller items in the other sorted groups (binary searches in shared memory).
+__device__ __forceinline__ void run_order_general(u32* ids, double* dist, u64* sd, u32* si, u32 len, u32 lane)
+{
+  const u32 groups = (len + 31) >> 5;
+  for (u32 g = 0; g < groups; ++g)
+  {
+    const u32 i = g * 32 + lane;
+    RunKey<true> v{ ~0ull, ~0u };
+    if (i < len)
+      v = run_load<true>(ids, dist, i);
+    run_sort_lanes<true>(v, lane);
+    si[i] = v.id;
+    sd[i] = v.d;
+  }
+  __syncwarp();
+  for (u32 i = lane; i < len; i += 32) // the padding of the last group sorts last in it
+  {
+    const RunKey<true> v{ sd[i], si[i] };
+    u32 rank = lane;
+    for (u32 h = 0; h < groups; ++h)
+    {
+      if (h == i >> 5)
+        continue;
+      u32 lo = 0;
+#pragma unroll
+      for (u32 s = 16; s > 0; s >>= 1)
+      {
+        const u32 j = h * 32 + lo + s - 1;
+        const RunKey<true> o{ sd[j], si[j] };
+        if (o.less(v))
+          lo += s;
+      }
+      const RunKey<true> o{ sd[h * 32 + lo], si[h * 32 + lo] };
+      rank += lo + (o.less(v) ? 1u : 0u);
+    }
+    ids[rank] = v.id;
+    dist[rank] = __longlong_as_double((long long)v.d);
+  }
+}
+
+// One warp per query sorts its run in place: ids as words in registers, distances by packed words, or by the general
+// order where those give up. Runs above kRunSortMax go to the list longRuns (longCount[0] counts them)
+// for run_sort_block_kernel. Bound by issue: the general order for every run took 0.149 ms for the distances of 60k rays
+// (now 0.050), 8.1 us for the ids of 10k ranges of about 60 points (now 4.0) and 38.6 us for those of a forest's 1M ranges
+// of a few boxes (33.9; 60 at the occupancy that the compiler's choice of registers for 256 ids left).
 template<bool DIST>
-__global__ void __launch_bounds__(kRunSortWarps * 32) run_sort_kernel(const u64* __restrict__ off, u64 nq, u32* __restrict__ ids, double* __restrict__ dist,
+__global__ void __launch_bounds__(kRunSortWarps * 32, DIST ? 0 : 8) run_sort_kernel(const u64* __restrict__ off, u64 nq, u32* __restrict__ ids, double* __restrict__ dist,
                                                                     u32* __restrict__ longCount, u32* __restrict__ longRuns, u32 longCap)
 {
   __shared__ u64 sd[DIST ? kRunSortWarps : 1][DIST ? kRunSortMax : 1];
-  __shared__ u32 si[kRunSortWarps][kRunSortMax];
+  __shared__ u32 si[DIST ? kRunSortWarps : 1][DIST ? kRunSortMax : 1];
   const u32 lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const u64 warps = u64(gridDim.x) * kRunSortWarps;
   for (u64 q = u64(blockIdx.x) * kRunSortWarps + w; q < nq; q += warps)
@@ -151,61 +334,39 @@ __global__ void __launch_bounds__(kRunSortWarps * 32) run_sort_kernel(const u64*
       continue;
     }
     const u32 len = u32(len64);
-    if (len <= 32)
+    if constexpr (!DIST)
     {
-      RunKey<DIST> v{ ~0ull, ~0u };
-      if (lane < len)
-        v = run_load<DIST>(ids, dist, b + lane);
-      run_sort_lanes<DIST>(v, lane);
-      if (lane < len)
+      if (len <= 32)
+        run_order_ids<1>(ids + b, len, lane);
+      else if (len <= 64)
+        run_order_ids<2>(ids + b, len, lane);
+      else if (len <= 128)
+        run_order_ids<4>(ids + b, len, lane);
+      else
+        run_order_ids<8>(ids + b, len, lane);
+    }
+    else
+    {
+      for (u32 i = lane; i < len; i += 32)
       {
-        ids[b + lane] = v.id;
-        if (DIST)
-          dist[b + lane] = __longlong_as_double((long long)v.d);
+        si[w][i] = ids[b + i];
+        sd[w][i] = u64(__double_as_longlong(dist[b + i]));
       }
-      continue;
-    }
-    const u32 groups = (len + 31) >> 5;
-    for (u32 g = 0; g < groups; ++g)
-    {
-      const u32 i = g * 32 + lane;
-      RunKey<DIST> v{ ~0ull, ~0u };
-      if (i < len)
-        v = run_load<DIST>(ids, dist, b + i);
-      run_sort_lanes<DIST>(v, lane);
-      si[w][i] = v.id;
-      if (DIST)
-        sd[w][i] = v.d;
-    }
-    __syncwarp();
-    for (u32 g = 0; g < groups; ++g)
-    {
-      const u32 i = g * 32 + lane;
-      if (i >= len) // the padding of the last group sorts last in it
-        continue;
-      const RunKey<DIST> v{ DIST ? sd[w][i] : 0, si[w][i] };
-      u32 rank = lane;
-      for (u32 h = 0; h < groups; ++h)
-      {
-        if (h == g)
-          continue;
-        u32 lo = 0;
-#pragma unroll
-        for (u32 s = 16; s > 0; s >>= 1)
+      __syncwarp();
+      const bool done = len <= 32    ? run_order_packed<1>(sd[w], si[w], len, lane)
+                        : len <= 64  ? run_order_packed<2>(sd[w], si[w], len, lane)
+                        : len <= 128 ? run_order_packed<4>(sd[w], si[w], len, lane)
+                                     : run_order_packed<8>(sd[w], si[w], len, lane);
+      if (done)
+        for (u32 i = lane; i < len; i += 32)
         {
-          const u32 j = h * 32 + lo + s - 1;
-          const RunKey<DIST> o{ DIST ? sd[w][j] : 0, si[w][j] };
-          if (o.less(v))
-            lo += s;
+          ids[b + i] = si[w][i];
+          dist[b + i] = __longlong_as_double((long long)sd[w][i]);
         }
-        const RunKey<DIST> o{ DIST ? sd[w][h * 32 + lo] : 0, si[w][h * 32 + lo] };
-        rank += lo + (o.less(v) ? 1u : 0u);
-      }
-      ids[b + rank] = v.id;
-      if (DIST)
-        dist[b + rank] = __longlong_as_double((long long)v.d);
+      else
+        run_order_general(ids + b, dist + b, sd[w], si[w], len, lane);
+      __syncwarp();
     }
-    __syncwarp();
   }
 }
 

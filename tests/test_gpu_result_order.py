@@ -65,6 +65,27 @@ def test_distance_runs(runs, dtype):
     assert np.array_equal(dist, x[ei])
 
 
+@pytest.mark.parametrize("step", [0.0, 2.0**-44, 2.0**-20, 2.0**40], ids=["equal", "near", "close", "wide"])
+@pytest.mark.parametrize("distinct", [1, 2, 9, 1000])
+def test_distance_ties(distinct, step):
+    """Runs of equal distances and of distances that agree in their leading bits: 1 + step j, `distinct` of them."""
+    rng = np.random.default_rng(23)
+    runs = [2, 3, 12, 13, 31, 32, 33, 64, 65, 128, 129, 255, 256]
+    row = rng.permutation(np.repeat(np.arange(len(runs)), runs))
+    x = 1.0 + step * rng.integers(0, distinct, len(row))
+    b = np.zeros((len(row), 6))
+    b[:, 0], b[:, 3] = x, x + 1.0
+    b[:, 1], b[:, 4] = 4.0 * row, 4.0 * row + 1
+    b[:, 2], b[:, 5] = 0, 1
+    t = otg.Tree("boxes").create(b, max_depth=6, max_elements=16)
+    rays = np.zeros((len(runs), 6))
+    rays[:, 1], rays[:, 2], rays[:, 3] = 4.0 * np.arange(len(runs)) + 0.5, 0.5, 1.0
+    off, ids, dist = t.ray_all(rays, tol=0.0)
+    lists = [np.flatnonzero(row == i) for i in range(len(runs))]
+    eo, ei = csr([l[np.lexsort((l, x[l]))] for l in lists])
+    assert np.array_equal(off, eo) and np.array_equal(ids, ei) and np.array_equal(dist, x[ei])
+
+
 @pytest.mark.parametrize("n", [300, 8191, 8192, 8193, 70_001])
 @pytest.mark.parametrize("nq", [1, 7])
 def test_dense_ids(n, nq):
