@@ -813,7 +813,7 @@ __global__ void location_export_kernel(const T* __restrict__ geom, const u32* __
 // boxes). Consecutive threads take consecutive units, so three lanes read one entity and the writes are
 // whole lines; every thread issues the loads of G units before storing any of them. One lane per entity
 // read its record in 3 to 6 instructions that touch 32 lines each, and the load unit was the bound where
-// the entities sit in L2: 65.8M FP32 boxes of 4096 trees 1.19 ms, now 1.00; 8M FP64 boxes beside their emission 0.353 ms, now 0.297.
+// the entities sit in L2: 65.8M FP32 boxes of 4096 trees 1.19 ms, then 1.00; 8M FP64 boxes beside their emission 0.353 ms, now 0.297.
 template<int BYTES>
 struct GatherUnit;
 template<>
@@ -834,7 +834,28 @@ struct GatherUnit<16>
 constexpr int kGatherPerThread = 8;
 
 // vec: both arrays start on a multiple of the unit (the tree's always does; a caller's may not)
-template<typename T, int W, int G>
+// a load that brings its 256 bytes into L2
+template<typename U>
+__device__ __forceinline__ U load_near(const U* p)
+{
+  U v;
+  if constexpr (sizeof(U) == 4)
+    asm volatile("ld.global.nc.L2::256B.u32 %0, [%1];" : "=r"(v) : "l"(p));
+  else if constexpr (sizeof(U) == 8)
+    asm volatile("ld.global.nc.L2::256B.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+  else
+    asm volatile("ld.global.nc.L2::256B.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+// A block of a single tree's gather takes units a grid apart (its points are read at random, and few blocks leave
+// room for the emission). A forest's block (kGatherRuns) takes G * 256 consecutive units, so that the blocks in
+// flight read a few tens of trees: 65.8M boxes of 4096 trees 0.76 ms, 1.01 with units a grid apart; four trees
+// of 4M 0.237 against 0.316. Where the largest tree takes no more than half of L2 (kGatherNear), every load also
+// brings its 256 bytes into L2, whose other boxes are read soon: 0.70 ms; 1M boxes per tree 0.191 against 0.196, 4M (96 MB)
+// the same, 16M (384 MB) 0.377 against 0.346, so not there.
+constexpr int kGatherStrided = 0, kGatherRuns = 1, kGatherNear = 2;
+constexpr u64 kGatherNearBytes = u64(64) << 20;
+template<typename T, int W, int G, int MODE = kGatherStrided>
 __global__ void __launch_bounds__(256) gather_kernel(const T* __restrict__ ent, const u32* __restrict__ ids, u64 n, T* __restrict__ out, bool vec)
 {
   using Unit = typename GatherUnit<int(sizeof(T)) * W / 3>::Type;
@@ -842,9 +863,10 @@ __global__ void __launch_bounds__(256) gather_kernel(const T* __restrict__ ent, 
   constexpr u32 kNone = 0xffffffffu;
   const Unit* src = reinterpret_cast<const Unit*>(ent);
   Unit* dst = reinterpret_cast<Unit*>(out);
-  const u64 stride = u64(gridDim.x) * blockDim.x;
+  constexpr bool RUNS = MODE != kGatherStrided;
+  const u64 stride = RUNS ? u64(blockDim.x) : u64(gridDim.x) * blockDim.x;
   const u64 units = n * 3;
-  for (u64 i0 = blockIdx.x * u64(blockDim.x) + threadIdx.x; i0 < units; i0 += stride * G)
+  for (u64 i0 = blockIdx.x * u64(blockDim.x) * (RUNS ? G : 1) + threadIdx.x; i0 < units; i0 += u64(gridDim.x) * blockDim.x * G)
   {
     Unit v[G];
     u32 from[G]; // (entities are below 2^30, so units fit 32 bits)
@@ -866,7 +888,7 @@ __global__ void __launch_bounds__(256) gather_kernel(const T* __restrict__ ent, 
       if (from[k] != kNone)
       {
         if (vec)
-          v[k] = src[from[k]];
+          v[k] = MODE == kGatherNear ? load_near(src + from[k]) : src[from[k]];
         else
         {
           T x[S];
@@ -2065,9 +2087,12 @@ static int forest_build_impl(TreeState& t, const T* ent, const T* boxes, cudaStr
   const u32 tiles = u32(t.segTilesHost.size());
   const u64 tabEntries = t.tabOffHost.back();
   const u64 minEntries = IS_BOX ? 1 : t.minOffHost.back();
-  u64 maxTab = 0;
+  u64 maxTab = 0, maxTree = 0;
   for (u32 i = 0; i < trees; ++i)
+  {
     maxTab = std::max(maxTab, t.tabOffHost[i + 1] - t.tabOffHost[i]);
+    maxTree = std::max(maxTree, t.treeOffHost[i + 1] - t.treeOffHost[i]);
+  }
   const size_t maxTabBytes = sizeof(U) * maxTab;
   const u64 maxNodes = n + trees + u64(Dmax) * (n / (t.maxElem + 1) + 1) + 2;
   t.maxNodes = maxNodes;
@@ -2156,8 +2181,12 @@ static int forest_build_impl(TreeState& t, const T* ent, const T* boxes, cudaStr
   const cudaStream_t es = st;
   prof.mark("gather", st);
   if (n)
-    gather_kernel<T, W, kGatherPerThread><<<grid_blocks((3 * n + kGatherPerThread - 1) / kGatherPerThread, 256, 152 * 16), 256, 0, st>>>(
-      ent, t.sortedIds.as<u32>(), n, t.sortedGeom.as<T>(), gather_aligned<T, W>(ent));
+  {
+    auto gfn = maxTree * W * sizeof(T) <= kGatherNearBytes ? gather_kernel<T, W, kGatherPerThread, kGatherNear>
+                                                           : gather_kernel<T, W, kGatherPerThread, kGatherRuns>;
+    gfn<<<grid_blocks((3 * n + kGatherPerThread - 1) / kGatherPerThread, 256, 1 << 20), 256, 0, st>>>(ent, t.sortedIds.as<u32>(), n, t.sortedGeom.as<T>(),
+                                                                                                    gather_aligned<T, W>(ent));
+  }
   prof.mark("emit", st);
   u32* parent = IS_BOX ? t.nodeParent.as<u32>() : nullptr;
   // entities that the emission places in no node keep kNoOwner
