@@ -873,18 +873,7 @@ __global__ void __launch_bounds__(WARPS * 32, KIND == kRayAll && sizeof(T) == 8 
         const bool cont = act && (entry & kContained);
         if (__any_sync(~0u, cont))
         {
-          if (cont && a.phase == 1 && (L.x >> kChildShift) != 0u && L.w - L.y > 1024u)
-          {
-            // only where the children hold the rest of the run: a run may also hold entities of no
-            // reachable node (locations outside the grid)
-            u32 held = L.z - L.y;
-            for (u32 c = 0; c < (L.x >> kChildShift); ++c)
-            {
-              const uint4 C = tv.link[(L.x & kFirstChildMask) + c];
-              held += C.w - C.y;
-            }
-            expand = held == L.w - L.y;
-          }
+          expand = cont && a.phase == 1 && (L.x >> kChildShift) != 0u && L.w - L.y > 1024u;
           whole = cont;
           const u32 len = cont ? (expand ? L.z : L.w) - L.y : 0u;
           u32 incl = len;

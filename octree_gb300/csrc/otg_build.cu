@@ -1001,7 +1001,8 @@ __device__ __forceinline__ void write_node_min(T* nodeBox, u32 node, u64 key, u3
 // (CreateProcessingData's partition_point, :695-711) at the same time, so the dependent-load
 // chain of a node is one binary search deep. Below the root every key of a node's range shares
 // its prefix, so child 7 ends where the range ends; at the root lane 0 also searches that end
-// (locations outside the 3*D-bit grid sort after every child range and belong to no child).
+// (locations outside the 3*D-bit grid sort after every child range and belong to no child). The
+// root's run ends there too: a run that is taken whole holds the entities of its nodes and no others.
 // Per-tree parameters of a forest build (several independent trees emitted together: node t is
 // the root of tree t). All null for a single tree.
 struct ForestNodes
@@ -1263,7 +1264,7 @@ __global__ void __launch_bounds__(256) emit_split_kernel(u32 d, u32 D, const K* 
         if (overflow)
           atomicOr(err, kErrCapacity);
         const u32 nc = overflow ? 0u : nchild;
-        link[node] = make_uint4((nc ? (firstChild & kFirstChildMask) : 0u) | (nc << kChildShift), b, ownEnd, e);
+        link[node] = make_uint4((nc ? (firstChild & kFirstChildMask) : 0u) | (nc << kChildShift), b, ownEnd, end8);
       }
       if (ownerNode)
         for (u32 q = b + gl; q < ownEnd; q += 8)

@@ -58,7 +58,6 @@ struct CollideArgs
   const T* geomB;
   const uint4* linkB;
   const float4* nodeB; // per node {min rounded down}, {max rounded up}
-  const u32* ownerB;
   u32 nB, nNodesB;
   u32 direct;          // subtrees of at most this many entities are tested without their nodes
   u32 stackCap;        // entries of a warp's stack
@@ -267,9 +266,6 @@ __global__ void __launch_bounds__(WARPS * 32, 32 / WARPS) collide_packet_kernel(
               hit = boxes_overlap_exact<T>(a.geomA + u64(il) * 6, a.geomB + u64(j) * 6, a.tol);
               ++rechecks;
             }
-            // a subtree's run may hold entities of no reachable node
-            if (hit && whole)
-              hit = a.ownerB[j] != kNoOwner;
           }
           const u32 bal = __ballot_sync(~0u, hit);
           if (!bal)
@@ -442,7 +438,6 @@ static int collide_search_impl(TreeState& A, TreeState& B, bool self, bool swapO
   a.swapOut = swapOut ? 1 : 0;
   a.sure = !A.respanned && !B.respanned;
   a.direct = a.sure ? kDirectBoxes : 0u;
-  a.ownerB = B.ownerNode.as<u32>();
   a.tolHi = float(a.tol);
   if (double(a.tolHi) < double(a.tol))
     a.tolHi = std::nextafter(a.tolHi, __builtin_huge_valf());

@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(kStaticThreads) static_assign_kernel(StaticCtl
                                                                       const unsigned char* __restrict__ nodeDepth, const K* __restrict__ keys,
                                                                       u32* __restrict__ order, u32 orderCap, u32* __restrict__ childBegin,
                                                                       uint2* __restrict__ seg, unsigned char* __restrict__ depthOut,
-                                                                      T* __restrict__ geom, const T* __restrict__ minTab, u32 D, u64 maxElem)
+                                                                      T* __restrict__ geom, const T* __restrict__ minTab, u32 D, u64 maxElem, u32 n)
 {
   u32 start, b, e;
   level_chunk(c, l, orderCap, start, b, e);
@@ -196,7 +196,9 @@ __global__ void __launch_bounds__(kStaticThreads) static_assign_kernel(StaticCtl
     const u32 cc = active ? child_count(L) : 0u;
     u32 total;
     const u32 excl = block_exclusive_scan(cc, total);
-    if (active && L.w <= L.y)
+    // (the root's run leaves out the entities of locations outside the grid)
+    const u32 end = x ? L.w : n;
+    if (active && end <= L.y)
     {
       atomicOr(&c->err, kErrOrder); // every node of a tree with entities holds some
     }
@@ -207,7 +209,7 @@ __global__ void __launch_bounds__(kStaticThreads) static_assign_kernel(StaticCtl
       childBegin[id] = cb;
       // CreateNode (:383-414): a node that splits keeps the entities of its own depth (the stuck
       // run at the front of its range); a leaf keeps its whole range
-      const u32 own = cc ? L.z - L.y : L.w - L.y;
+      const u32 own = cc ? L.z - L.y : end - L.y;
       seg[id] = make_uint2(L.y, own);
       covered += own;
       // depth: the root stays at 0; a node that splits is at the lowest common ancestor already
@@ -369,7 +371,7 @@ int export_static_impl(TreeState& t, otg_static_layout* out, cudaStream_t st)
     static_scan_kernel<<<1, kScanThreadsStatic, 0, st>>>(ctl, l);
     static_assign_kernel<T, K, IS_BOX><<<kStaticBlocks, kStaticThreads, 0, st>>>(
       ctl, l, t.nodeLink.as<uint4>(), t.nodeDepth.as<unsigned char>(), keys, t.stOrder.as<u32>(), u32(mDyn), t.stChildBegin.as<u32>(),
-      t.stSeg.as<uint2>(), t.stDepth.as<unsigned char>(), IS_BOX ? nullptr : t.stGeom.as<T>(), t.minTab.as<T>(), t.D, t.maxElem);
+      t.stSeg.as<uint2>(), t.stDepth.as<unsigned char>(), IS_BOX ? nullptr : t.stGeom.as<T>(), t.minTab.as<T>(), t.D, t.maxElem, u32(t.n));
   }
   static_finish_kernel<<<1, 32, 0, st>>>(ctl, t.stChildBegin.as<u32>(), u32(mDyn));
   if constexpr (IS_BOX)
