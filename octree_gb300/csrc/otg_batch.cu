@@ -372,7 +372,8 @@ struct PlaneF32
 {
   float n[3], a, b, c, d, pad;
 };
-constexpr u32 kMaxPlanes = 8; // planes per query that the FP32 tests take
+// planes per query that the FP32 tests take, one made by each lane; the ones after them are tested exactly
+constexpr u32 kMaxPlanes = 32;
 
 __device__ __forceinline__ void plane_f32(const PlaneF32& p, const float lo[3], const float hi[3], float& smin, float& smax)
 {
@@ -386,7 +387,25 @@ __device__ __forceinline__ void plane_f32(const PlaneF32& p, const float lo[3], 
   }
 }
 
-// planes {dist, n} of one query, lanes 0 .. np - 1 (np <= kMaxPlanes); rootBox: {min, size}
+// An entity against more than eight planes: 0 negative for some, 1 for none, 2 undecided. Leaving at the first negative
+// one gains with many planes (16 views of 36 on 500k regular FP32 boxes 1.96 ms, now 1.22) and costs with
+// the six of a view (96 views 1.33 ms, 1.43 with it), whose loop stands in the kernel without it.
+__device__ __noinline__ u32 planes_many_f32(const PlaneF32* planes, u32 n, float3 l, float3 h)
+{
+  const float lo[3] = { l.x, l.y, l.z }, hi[3] = { h.x, h.y, h.z };
+  bool sure = true;
+  for (u32 i = 0; i < n; ++i)
+  {
+    float smin, smax;
+    plane_f32(planes[i], lo, hi, smin, smax);
+    if (smax < planes[i].a)
+      return 0;
+    sure &= smax > planes[i].b;
+  }
+  return sure ? 1 : 2;
+}
+
+// planes {dist, n} of one query, lanes 0 .. np - 1; rootBox: {min, size}
 template<typename T>
 __device__ __forceinline__ void plane_thresholds(const T* pl, u32 np, const T* rootBox, T tol, u32 lane, PlaneF32* out)
 {
@@ -424,6 +443,26 @@ __device__ __noinline__ bool frustum_node_exact(const T* nb, const T* pl, u32 np
     if (rel == 0)
       return false;
   }
+  return true;
+}
+// an entity passes unless it is negative for some plane. All planes in one call: 64 frusta of 9 planes on 500k FP32
+// boxes, tested exactly, 0.66 ms with a call for each and 0.45 this way (with the FP32 tests 0.37).
+template<typename T>
+__device__ __noinline__ bool frustum_entity_exact(const T* g, int isBox, const T* pl, u32 np, T tol)
+{
+  if (!isBox)
+  {
+    for (u32 i = 0; i < np; ++i)
+      if (GeoD<T>::point_plane(g, pl[4 * i], pl + 4 * i + 1, tol) == 0)
+        return false;
+    return true;
+  }
+  T b[6];
+  load_box(g, b);
+  const T bsize[3] = { T(b[3] - b[0]), T(b[4] - b[1]), T(b[5] - b[2]) };
+  for (u32 i = 0; i < np; ++i)
+    if (GeoD<T>::box_plane(b, bsize, pl[4 * i], pl + 4 * i + 1, tol) == 0)
+      return false;
   return true;
 }
 // GetEntityPlaneRelation (ot_query.h:586-602) of a point or box
@@ -482,7 +521,7 @@ __global__ void __launch_bounds__(WARPS * 32, KIND == kRayAll && sizeof(T) == 8 
   constexpr bool kPlanes = KIND == kFrustum || KIND == kPlane || KIND == kPlanePositive;
   // kinds that take whole subtrees untested
   constexpr bool kWhole = KIND == kRange || KIND == kPlanePositive || KIND == kFrustum;
-  __shared__ PlaneF32 planeF[kPlanes ? WARPS : 1][kPlanes ? kMaxPlanes : 1];
+  __shared__ PlaneF32 planeF[kPlanes ? WARPS : 1][KIND == kFrustum ? kMaxPlanes : 1];
   __shared__ RayF32 rayF[kRayPre ? WARPS : 1];
   __shared__ u32 candMem[kRayPre ? WARPS : 1][kRayPre ? kCandBuf : 1];
   __shared__ RangeF32 rangeF[kRangeF32 ? WARPS : 1];
@@ -654,11 +693,11 @@ __global__ void __launch_bounds__(WARPS * 32, KIND == kRayAll && sizeof(T) == 8 
       continue;
     bool planeTests = false;
     if constexpr (kPlanes)
-      if (a.planeF32 && a.np <= kMaxPlanes)
+      if (a.planeF32)
       {
         planeTests = true;
         __syncwarp(); // the previous query's planes are read by every lane before they change
-        plane_thresholds<T>(pl, a.np, tv.nodeBox + u64(root) * 6, a.tol, lane, planeF[w]);
+        plane_thresholds<T>(pl, min(a.np, kMaxPlanes), tv.nodeBox + u64(root) * 6, a.tol, lane, planeF[w]);
         __syncwarp();
       }
     // the FP32 corners of a node or entity for the plane tests
@@ -754,8 +793,9 @@ __global__ void __launch_bounds__(WARPS * 32, KIND == kRayAll && sizeof(T) == 8 
         {
           float lo[3], hi[3];
           corners(true, node, lo, hi);
-          bool decided = true, positive = true;
-          for (u32 i = 0; i < np; ++i)
+          const u32 nf = min(np, kMaxPlanes);
+          bool decided = nf == np, positive = true;
+          for (u32 i = 0; i < nf; ++i)
           {
             const PlaneF32& p = planeF[w][i];
             float smin, smax;
@@ -1044,35 +1084,41 @@ __global__ void __launch_bounds__(WARPS * 32, KIND == kRayAll && sizeof(T) == 8 
               const u32 np = KIND == kFrustum ? a.np : 1u;
               const T* g = tv.geom + u64(e) * (tv.isBox ? 6 : 3);
               bool decided = false;
+              u32 passed = 0; // leading planes that the entity is certainly not negative for
               if (planeTests)
               {
                 float lo[3], hi[3];
                 corners(false, e, lo, hi);
                 bool neg = false, sure = true, cut = true;
-                for (u32 i = 0; i < np; ++i)
+                const u32 nf = min(np, kMaxPlanes);
+                if (KIND == kFrustum && nf > 8u)
                 {
-                  const PlaneF32& p = planeF[w][i];
-                  float smin, smax;
-                  plane_f32(p, lo, hi, smin, smax);
-                  neg |= smax < p.a;
-                  sure &= smax > p.b;
-                  if (KIND == kPlane)
-                  {
-                    cut = smin < p.d;
-                    neg |= smin > p.c; // not hit
-                  }
+                  const u32 rel = planes_many_f32(planeF[w], nf, make_float3(lo[0], lo[1], lo[2]), make_float3(hi[0], hi[1], hi[2]));
+                  neg = rel == 0;
+                  sure = rel == 1;
                 }
-                decided = neg | (sure & cut);
+                else
+                  for (u32 i = 0; i < nf; ++i)
+                  {
+                    const PlaneF32& p = planeF[w][i];
+                    float smin, smax;
+                    plane_f32(p, lo, hi, smin, smax);
+                    neg |= smax < p.a;
+                    sure &= smax > p.b;
+                    if (KIND == kPlane)
+                    {
+                      cut = smin < p.d;
+                      neg |= smin > p.c; // not hit
+                    }
+                  }
+                decided = neg | (sure & cut & (nf == np));
                 hit = !neg;
+                passed = sure ? nf : 0u;
               }
               if (!decided)
               {
                 if constexpr (KIND == kFrustum)
-                {
-                  hit = true;
-                  for (u32 i = 0; i < np && hit; ++i)
-                    hit = entity_plane_exact<T>(g, tv.isBox, pl + 4 * i, a.tol) != 0;
-                }
+                  hit = frustum_entity_exact<T>(g, tv.isBox, pl + 4 * passed, np - passed, a.tol);
                 else
                 {
                   const int rel = entity_plane_exact<T>(g, tv.isBox, pl, a.tol);
