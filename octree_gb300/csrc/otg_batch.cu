@@ -707,7 +707,8 @@ __global__ void __launch_bounds__(WARPS * 32, KIND == kRayAll && sizeof(T) == 8 
         if (!isNode && !tv.isBox)
         {
           const float4 p = tv.pointImg[i];
-          lo[0] = hi[0] = p.x, lo[1] = hi[1] = p.y, lo[2] = hi[2] = p.z;
+          lo[0] = hi[0] = p.w < INFINITY ? p.x : NAN; // a point without a finite image decides nothing
+          lo[1] = hi[1] = p.y, lo[2] = hi[2] = p.z;
           return;
         }
         const float4* img = isNode ? tv.nodeImg : tv.boxImg;
@@ -1090,6 +1091,8 @@ __global__ void __launch_bounds__(WARPS * 32, KIND == kRayAll && sizeof(T) == 8 
                 float lo[3], hi[3];
                 corners(false, e, lo, hi);
                 bool neg = false, sure = true, cut = true;
+                // an entity with a NaN (the root may hold some) takes the exact test: the corners' sums pass a NaN over
+                const bool plain = (lo[0] <= hi[0]) & (lo[1] <= hi[1]) & (lo[2] <= hi[2]);
                 const u32 nf = min(np, kMaxPlanes);
                 if (KIND == kFrustum && nf > 8u)
                 {
@@ -1111,9 +1114,9 @@ __global__ void __launch_bounds__(WARPS * 32, KIND == kRayAll && sizeof(T) == 8 
                       neg |= smin > p.c; // not hit
                     }
                   }
-                decided = neg | (sure & cut & (nf == np));
+                decided = plain & (neg | (sure & cut & (nf == np)));
                 hit = !neg;
-                passed = sure ? nf : 0u;
+                passed = plain && sure ? nf : 0u;
               }
               if (!decided)
               {
