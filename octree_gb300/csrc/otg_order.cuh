@@ -551,12 +551,27 @@ __global__ void bit_write_kernel(const u32* __restrict__ bits, const u64* __rest
   }
 }
 
-// ---- pairs: one warp per 32 neighbouring a's sorts their runs of b's by rank (the count of smaller b's in
-// the run: runs average a few items) and writes (a, b); a run above kPairRunMax is only counted.
-constexpr u32 kPairRunMax = 1024;
+// ---- pairs: one warp per 32 neighbouring a's sorts their runs of b's and writes (a, b): runs up to kPairRankMax by
+// rank (the count of smaller b's in the run: runs average a few items), longer ones up to kRunSortMax as words in
+// registers; runs above go to the list longRuns, for run_sort_block_kernel and pair_long_write_kernel. Ranks cost a run's
+// length per item: 60k boxes of 178 and 739 pairs each, whole call, 1.90 and 9.97 ms with ranks up to 1024, 1.40 and 5.6 this way.
+constexpr u32 kPairRankMax = 64;
 constexpr u32 kPairTile = 512;
+template<int R>
+__device__ __forceinline__ void pair_order_run(const u32* bs, u32 a, u32 n, u32 lane, uint2* out)
+{
+  u32 x[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+    x[r] = r * 32 + lane < n ? bs[r * 32 + lane] : ~0u;
+  run_sort_words<R>(x, n, lane);
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+    if (r * 32 + lane < n)
+      out[r * 32 + lane] = make_uint2(a, x[r]);
+}
 __global__ void __launch_bounds__(256) pair_write_kernel(const u64* __restrict__ off, u64 nA, const u32* __restrict__ bs, uint2* __restrict__ out,
-                                                         u32* __restrict__ tooLong)
+                                                         u32* __restrict__ longCount, u32* __restrict__ longRuns, u32 longCap)
 {
   __shared__ u32 sb[8][kPairTile];
   __shared__ u32 so[8][33];
@@ -571,14 +586,25 @@ __global__ void __launch_bounds__(256) pair_write_kernel(const u64* __restrict__
     if (total == 0)
       continue;
     const u64 prev = __shfl_up_sync(~0u, at, 1);
-    const u64 len = at - (lane ? prev : base);
-    if (__any_sync(~0u, len > kPairRunMax))
+    const u32 first = u32((lane ? prev : base) - base), len = u32(at - base) - first;
+    if (len > kRunSortMax)
     {
-      if (lane == 0)
-        atomicAdd(tooLong, 1u);
-      continue;
+      const u32 to = atomicAdd(longCount, 1u);
+      if (to < longCap)
+        longRuns[to] = u32(a0) + lane;
     }
-    const u32 T = u32(total); // at most 32 * kPairRunMax
+    for (u32 mid = __ballot_sync(~0u, len > kPairRankMax && len <= kRunSortMax); mid; mid &= mid - 1)
+    {
+      const u32 r = u32(__ffs(int(mid))) - 1;
+      const u32 b0 = __shfl_sync(~0u, first, r), n = __shfl_sync(~0u, len, r);
+      if (n <= 128)
+        pair_order_run<4>(bs + base + b0, u32(a0) + r, n, lane, out + base + b0);
+      else
+        pair_order_run<8>(bs + base + b0, u32(a0) + r, n, lane, out + base + b0);
+    }
+    if (!__any_sync(~0u, len > 0 && len <= kPairRankMax))
+      continue;
+    const u32 T = u32(total); // (below 2^32: all pairs are)
     so[w][lane + 1] = u32(at - base);
     if (lane == 0)
       so[w][0] = 0;
@@ -595,6 +621,8 @@ __global__ void __launch_bounds__(256) pair_write_kernel(const u64* __restrict__
         if (so[w][r + s] <= t)
           r += s;
       const u32 b0 = so[w][r], b1 = so[w][r + 1];
+      if (b1 - b0 > kPairRankMax)
+        continue;
       u32 rank = 0;
       u32 v;
       if (tile)
@@ -612,6 +640,19 @@ __global__ void __launch_bounds__(256) pair_write_kernel(const u64* __restrict__
       out[base + b0 + rank] = make_uint2(u32(a0) + r, v);
     }
     __syncwarp();
+  }
+}
+// the listed runs, once they are sorted in place
+__global__ void __launch_bounds__(256) pair_long_write_kernel(const u64* __restrict__ off, const u32* __restrict__ bs, uint2* __restrict__ out,
+                                                              const u32* __restrict__ longCount, const u32* __restrict__ longRuns, u32 longCap)
+{
+  const u32 n = min(longCount[0], longCap);
+  for (u32 l = blockIdx.x; l < n; l += gridDim.x)
+  {
+    const u32 a = longRuns[l];
+    const u64 e = off[a + 1];
+    for (u64 i = off[a] + threadIdx.x; i < e; i += blockDim.x)
+      out[i] = make_uint2(a, bs[i]);
   }
 }
 // (a << bBits | b) into (a, b)

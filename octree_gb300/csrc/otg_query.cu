@@ -1404,7 +1404,10 @@ static int finish_by_distance(Collected& c, u64 nq, u64 nEntities, ResultState& 
 // Pairs (a << 32 | b) ascending, one "query" holding 2 m ids. Where the pairs are many (at least one per
 // four entities) by counting: the pairs of each a, their offsets, the b's into their runs, and the runs of
 // 32 neighbouring a's sorted and written by one warp (9.7M pairs of 4M boxes: 0.79 ms by 8 radix passes,
-// a copy and a swap, 0.30 ms this way). Fewer pairs, or a run above kPairRunMax, by a radix sort over the bits in use.
+// a copy and a swap, 0.30 ms this way). Fewer pairs, more than kPairRadixFrom per entity, or a run above kBlockRunMax,
+// by a radix sort over the bits in use (60k boxes, whole call: 178 pairs each 1.40 ms by counting and 1.46 by the radix sort,
+// 502 each 3.9 and 3.7, 739 each 5.6 and 5.2).
+constexpr u64 kPairRadixFrom = 192;
 static int finish_pairs(Collected& c, u64 nA, u64 nB, ResultState& r, cudaStream_t st)
 {
   const u64 m = c.m;
@@ -1418,25 +1421,38 @@ static int finish_pairs(Collected& c, u64 nA, u64 nB, ResultState& r, cudaStream
   if ((e = cudaMemcpyAsync(r.offsets.p, offs, sizeof(offs), cudaMemcpyHostToDevice, st)))
     return cuda_status(e, "result offsets");
   bool done = m == 0;
-  if (m >= nA / 4 && m < (u64(1) << 32) && m)
+  if (m >= nA / 4 && m <= kPairRadixFrom * nA && m < (u64(1) << 32) && m)
   {
-    TmpBuf cnt, slot, off, sums, bs, tooLong;
+    TmpBuf cnt, slot, off, sums, bs, longs;
     const u64 tiles = (nA + kScanTile - 1) / kScanTile;
+    const u64 longCap = m / kRunSortMax + 1; // at most this many runs above kRunSortMax
     if ((e = cnt.ensure(sizeof(u32) * nA, st)) || (e = slot.ensure(sizeof(u32) * m, st)) || (e = off.ensure(sizeof(u64) * (nA + 1), st)) ||
-        (e = sums.ensure(sizeof(u64) * (tiles + 1), st)) || (e = bs.ensure(sizeof(u32) * m, st)) || (e = tooLong.ensure(sizeof(u32), st)))
+        (e = sums.ensure(sizeof(u64) * (tiles + 1), st)) || (e = bs.ensure(sizeof(u32) * m, st)) || (e = longs.ensure(sizeof(u32) * (2 + longCap), st)))
       return cuda_status(e, "allocating the pair order");
+    u32* longCount = longs.as<u32>();
+    u32* longRuns = longCount + 2;
     cudaMemsetAsync(cnt.p, 0, sizeof(u32) * nA, st);
-    cudaMemsetAsync(tooLong.p, 0, sizeof(u32), st);
+    cudaMemsetAsync(longCount, 0, sizeof(u32) * 2, st);
     query_slots_kernel<<<blocks_for(m), 256, 0, st>>>(c.items.as<u64>(), m, cnt.as<u32>(), slot.as<u32>());
     scan_reduce_kernel<<<u32(tiles), kScanThreads, 0, st>>>(cnt.as<u32>(), nA, sums.as<u64>());
     scan_tiles_kernel<<<1, kScanThreads, 0, st>>>(sums.as<u64>(), tiles);
     scan_apply_kernel<<<u32(tiles), kScanThreads, 0, st>>>(cnt.as<u32>(), nA, sums.as<u64>(), off.as<u64>());
     query_scatter_kernel<<<blocks_for(m), 256, 0, st>>>(c.items.as<u64>(), nullptr, slot.as<u32>(), m, off.as<u64>(), bs.as<u32>(), nullptr);
-    pair_write_kernel<<<u32(std::min<u64>((nA + 255) / 256, 152 * 8)), 256, 0, st>>>(off.as<u64>(), nA, bs.as<u32>(), r.ids.as<uint2>(), tooLong.as<u32>());
-    u32 h = 0;
-    if ((e = cudaGetLastError()) || (e = read_back(&h, tooLong.p, sizeof(u32), st)))
+    pair_write_kernel<<<u32(std::min<u64>((nA + 255) / 256, 152 * 8)), 256, 0, st>>>(off.as<u64>(), nA, bs.as<u32>(), r.ids.as<uint2>(), longCount, longRuns,
+                                                                                   u32(longCap));
+    u32 h[2] = { 0, 0 };
+    if ((e = cudaGetLastError()) || (e = read_back(h, longCount, sizeof(h), st)))
       return cuda_status(e, "ordering pairs");
-    done = h == 0;
+    if (h[0])
+    {
+      const u32 grid = std::min<u32>(h[0], 152 * 4);
+      run_sort_block_kernel<false><<<grid, kBlockSortThreads, kBlockRunMax * 4, st>>>(off.as<u64>(), bs.as<u32>(), nullptr, longCount, longRuns,
+                                                                                    u32(longCap));
+      pair_long_write_kernel<<<grid, 256, 0, st>>>(off.as<u64>(), bs.as<u32>(), r.ids.as<uint2>(), longCount, longRuns, u32(longCap));
+      if ((e = cudaGetLastError()) || (e = read_back(h, longCount, sizeof(h), st)))
+        return cuda_status(e, "ordering pairs");
+    }
+    done = h[1] == 0;
   }
   if (!done)
   {
