@@ -1,7 +1,7 @@
 // otg_collide.cu — candidate search of CollisionDetection (core/ot_query.h:1308-1497 two trees,
 // :1690-1914 one tree) with an FP32 filter.
 //
-// One warp walks the other tree for a packet of 32 entities of the first tree that follow each other
+// One warp walks the other tree for a packet of up to 32 entities of the first tree that follow each other
 // in it at the same depth, and so lie close together. A stack entry is a node and the mask of the
 // entities whose boxes may meet it. The node's own entities are tested by the lanes in parallel
 // against each box of the mask (read from shared memory), its children against the packet's common
@@ -36,6 +36,11 @@ constexpr u32 kPairBuf = 128;
 // themselves: 1.98 ms at 0, 1.83 at 64, 1.73 at 128 (searches of 16M boxes of 16 per node stay within 1%).
 constexpr u32 kDirectBoxes = 128;
 
+// Entities to a packet: 32 where that gives every resident warp a packet (about 156k entities), else as many
+// as do. 1000, 20k and 60k boxes that overlap most or some 1500 of the others, whole call: 2.57, 3.48 and 5.18 ms with 32
+// always, 0.34, 1.17 and 2.87 this way; 20k, 60k and 150k with 3 each 0.228, 0.257 and 0.255, now 0.210, 0.230 and 0.261.
+constexpr u64 kPacketsWanted = 152 * 32;
+
 struct CollideCounters
 {
   unsigned long long tests;
@@ -61,6 +66,7 @@ struct CollideArgs
   u32 nB, nNodesB;
   u32 direct;          // subtrees of at most this many entities are tested without their nodes
   u32 stackCap;        // entries of a warp's stack
+  u32 packet;          // entities to a packet
   T tol;
   int selfMode;
   int swapOut; // two trees searched from the second tree's entities: emit (walked position, entity position)
@@ -115,7 +121,7 @@ __global__ void __launch_bounds__(WARPS * 32, 32 / WARPS) collide_packet_kernel(
   const u32 lt = (1u << lane) - 1;
   u32 tests = 0, rechecks = 0;
   const u32 singles = min(*a.singles, a.nA);
-  const u32 items = singles + (a.nA - singles + 31) / 32;
+  const u32 items = singles + (a.nA - singles + a.packet - 1) / a.packet;
   float M = 0.f; // of the header comment
 #pragma unroll
   for (int c = 0; c < 3; ++c)
@@ -143,8 +149,8 @@ __global__ void __launch_bounds__(WARPS * 32, 32 / WARPS) collide_packet_kernel(
     item = __shfl_sync(~0u, item, 0);
     if (item >= items)
       break;
-    const u32 first = item < singles ? item : singles + (item - singles) * 32;
-    const u32 count = item < singles ? 1u : min(32u, a.nA - first);
+    const u32 first = item < singles ? item : singles + (item - singles) * a.packet;
+    const u32 count = item < singles ? 1u : min(a.packet, a.nA - first);
     u32 i = 0xffffffffu;
     bool valid = false;
     float4 a0 = make_float4(INFINITY, INFINITY, INFINITY, 0.f), a1 = make_float4(-INFINITY, -INFINITY, -INFINITY, 0.f);
@@ -393,6 +399,14 @@ static int launch_collide(const CollideArgs<T>& a, cudaStream_t st)
   return cuda_status(cudaGetLastError(), "launching the collision kernel");
 }
 
+static u32 collide_packet_size(u64 n)
+{
+  u32 p = 32;
+  while (p > 1 && n / p < kPacketsWanted)
+    p >>= 1;
+  return p;
+}
+
 template<typename T>
 static int collide_search_impl(TreeState& A, TreeState& B, bool self, bool swapOut, double tol, Appender out, u32* err, CollideSearch& s,
                                cudaStream_t st)
@@ -433,6 +447,7 @@ static int collide_search_impl(TreeState& A, TreeState& B, bool self, bool swapO
   a.nNodesB = u32(B.nodeCount);
   // depth first: at most 7 entries per level beside the current node's 8 children
   a.stackCap = (7 * (B.D + 1) + 9 + 3) & ~3u;
+  a.packet = collide_packet_size(A.n);
   a.tol = tol < 0 ? base_tol<T>() : T(tol);
   a.selfMode = self ? 1 : 0;
   a.swapOut = swapOut ? 1 : 0;
