@@ -33,9 +33,9 @@ namespace otg
 {
 
 constexpr float kInf = __builtin_huge_valf();
-// high bits of a query's start: its results are in the plain kernels' result, or in the array of the
-// queries with other than k results
-constexpr u32 kFromFallback = 1u << 31, kFromOut = 1u << 30;
+// High bits of a query's start, which otherwise is its slot: its results are in the plain kernels' result, or it has more
+// than k and those after the first k start here in the array for them.
+constexpr u32 kFromFallback = 1u << 31, kMoreThanK = 1u << 30;
 
 // One warp's part of the shared memory, followed by its stack (stackCap nodes and bounds). The exact
 // distances of the final order take the place of the bounds, which are not needed by then.
@@ -61,12 +61,12 @@ __host__ __device__ constexpr size_t knn_warp_bytes(u32 stackCap)
 
 struct KnnCounters
 {
-  unsigned long long out;      // result entries written
+  unsigned long long out;      // result entries beyond their queries' slots
   unsigned long long tests;    // FP32 filter evaluations
   unsigned long long rechecks; // exact distance evaluations
   u32 work;                    // next query to take
   u32 fallbacks;
-  u32 irregular; // queries with other than k results (outside their slots)
+  u32 irregular; // queries with other than k results
   u32 err;
 };
 
@@ -93,12 +93,12 @@ struct KnnArgs
   u32* fallback;
   u64* start;
   u32* count;
-  // slots of k results per query: query q's at slot[q], or at q * kAll
+  // slots of k results per query, for the first k of them: query q's at slot[q], or at q * kAll
   const u64* slot;
   u64* evenOffsets; // nq + 1 offsets to write, or null
   u32* slotIds;
   double* slotDist;
-  // results of the queries that have another number of them
+  // the results after the first k (ties within the tolerance)
   u32* outIds;
   double* outDist;
   u64 outCap;
@@ -443,6 +443,42 @@ __device__ __forceinline__ void knn_flush(KnnWarpMem<CAP>& W, const KnnArgs<T>& 
   bufN = kept;
 }
 
+// The results of a query that has another number of them than k: the first k to its slot, the rest to the array
+// for them. Queries with fewer than k (far from everything, or with a tight max distance) leave the rest of their slot
+// unused: in that array they would fill it, and an overflow there costs the whole search again (200k queries of k = 16
+// with 4.2 results each 1.46 ms, now 0.71). Out of line, as the kernel is short of registers.
+template<typename T>
+__device__ __noinline__ void knn_other_count(const KnnArgs<T>& a, const u32* ids, const unsigned long long* key, u32 q, u32 k, u32 m, u32 lane)
+{
+  u64 start = a.slot ? a.slot[q] : u64(q) * a.kAll;
+  for (u32 i = lane; i < min(m, k); i += 32)
+  {
+    a.slotIds[start + i] = ids[i];
+    a.slotDist[start + i] = __longlong_as_double((long long)key[i]);
+  }
+  if (lane == 0)
+    atomicAdd(&a.ctr->irregular, 1u);
+  if (m > k)
+  {
+    unsigned long long s0 = 0;
+    if (lane == 0)
+      s0 = atomicAdd(&a.ctr->out, (unsigned long long)(m - k));
+    s0 = __shfl_sync(~0u, s0, 0);
+    if (s0 + (m - k) <= a.outCap)
+      for (u32 i = k + lane; i < m; i += 32)
+      {
+        a.outIds[s0 + (i - k)] = ids[i];
+        a.outDist[s0 + (i - k)] = __longlong_as_double((long long)key[i]);
+      }
+    start = s0 | (u64(kMoreThanK) << 32);
+  }
+  if (lane == 0)
+  {
+    a.start[q] = start;
+    a.count[q] = m;
+  }
+}
+
 // 40 warps per SM (48 registers, some spills): 1M queries, k in 1..64, 16M points 6.55 ms; 7.22 at 64 to 80 registers and
 // 24 to 32 warps, 7.03 with 48 warps.
 template<typename T, int CAP, int WARPS>
@@ -684,29 +720,21 @@ __global__ void __launch_bounds__(WARPS * 32, 40 / WARPS) knn_filtered_kernel(Kn
       m += __popc(__ballot_sync(~0u, i < bufN && W.key[i] < Fbits));
     }
     // k results go to the query's slot, which is their place in the result if every query has k
-    const bool regular = m == k;
-    unsigned long long s0 = regular ? (a.slot ? a.slot[q] : u64(q) * a.kAll) : 0;
-    if (!regular)
+    if (m != k)
+      knn_other_count<T>(a, W.pos, W.key, q, k, m, lane);
+    else
     {
-      if (lane == 0)
-      {
-        s0 = atomicAdd(&a.ctr->out, (unsigned long long)m);
-        atomicAdd(&a.ctr->irregular, 1u);
-      }
-      s0 = __shfl_sync(~0u, s0, 0);
-    }
-    u32* ids = regular ? a.slotIds : a.outIds;
-    double* dist = regular ? a.slotDist : a.outDist;
-    if (regular || s0 + m <= a.outCap)
+      const u64 s0 = a.slot ? a.slot[q] : u64(q) * a.kAll;
       for (u32 i = lane; i < m; i += 32)
       {
-        ids[s0 + i] = W.pos[i];
-        dist[s0 + i] = __longlong_as_double((long long)W.key[i]);
+        a.slotIds[s0 + i] = W.pos[i];
+        a.slotDist[s0 + i] = __longlong_as_double((long long)W.key[i]);
       }
-    if (lane == 0)
-    {
-      a.start[q] = regular ? s0 : s0 | (u64(kFromOut) << 32);
-      a.count[q] = m;
+      if (lane == 0)
+      {
+        a.start[q] = s0;
+        a.count[q] = m;
+      }
     }
     __syncwarp();
   }
@@ -877,12 +905,12 @@ __global__ void __launch_bounds__(kScanThreads) scan_apply_kernel(const u32* __r
     off[n] = tileSums[gridDim.x];
 }
 
-// warp per query: copies its entries from where they are (its slot, the irregular ones' array, or the plain
-// kernels' result) to CSR order
+// warp per query: copies its entries from where they are (its slot and the results after the first k, or the
+// plain kernels' result) to CSR order
 __global__ void csr_move_kernel(const u64* __restrict__ start, const u32* __restrict__ count, const u64* __restrict__ off, u64 nq,
-                                const u32* __restrict__ slotIds, const double* __restrict__ slotDist, const u32* __restrict__ ids,
-                                const double* __restrict__ dist, const u32* __restrict__ fbIds, const double* __restrict__ fbDist,
-                                u32* __restrict__ outIds, double* __restrict__ outDist)
+                                const u64* __restrict__ slot, const u32* __restrict__ kArr, u32 kAll, const u32* __restrict__ slotIds,
+                                const double* __restrict__ slotDist, const u32* __restrict__ ids, const double* __restrict__ dist,
+                                const u32* __restrict__ fbIds, const double* __restrict__ fbDist, u32* __restrict__ outIds, double* __restrict__ outDist)
 {
   const u32 lane = threadIdx.x & 31;
   for (u64 q = (blockIdx.x * u64(blockDim.x) + threadIdx.x) >> 5; q < nq; q += (u64(gridDim.x) * blockDim.x) >> 5)
@@ -890,16 +918,18 @@ __global__ void csr_move_kernel(const u64* __restrict__ start, const u32* __rest
     const u32 c = count[q];
     if (!c)
       continue;
-    const u64 s = start[q];
-    const u32 from = u32(s >> 32) & (kFromFallback | kFromOut);
-    const u64 src = s & ~(u64(kFromFallback | kFromOut) << 32);
-    const u32* si = from == 0 ? slotIds : from == kFromOut ? ids : fbIds;
-    const double* sd = from == 0 ? slotDist : from == kFromOut ? dist : fbDist;
-    const u64 d = off[q];
+    const u64 s = start[q], d = off[q];
+    const u32 from = u32(s >> 32) & (kFromFallback | kMoreThanK);
+    const u64 at = s & ~(u64(kFromFallback | kMoreThanK) << 32);
+    const bool more = from == kMoreThanK;
+    const u64 src = more ? (slot ? slot[q] : q * kAll) : at;
+    const u32 k = more ? (kArr ? kArr[q] : kAll) : c;
+    const u32* si = from == kFromFallback ? fbIds : slotIds;
+    const double* sd = from == kFromFallback ? fbDist : slotDist;
     for (u32 i = lane; i < c; i += 32)
     {
-      outIds[d + i] = si[src + i];
-      outDist[d + i] = sd[src + i];
+      outIds[d + i] = i < k ? si[src + i] : ids[at + (i - k)];
+      outDist[d + i] = i < k ? sd[src + i] : dist[at + (i - k)];
     }
   }
 }
@@ -1176,15 +1206,17 @@ static int knn_filtered_impl(TreeState& t, const T* pts, const u32* dk, u64 nq, 
     return cuda_status(e, "allocating the kNN result");
   scan_reduce_kernel<<<u32(tiles), kScanThreads, 0, st>>>(cnt, nq, tileSums.as<u64>());
   scan_tiles_kernel<<<1, kScanThreads, 0, st>>>(tileSums.as<u64>(), tiles);
-  scan_apply_kernel<<<u32(tiles), kScanThreads, 0, st>>>(cnt, nq, tileSums.as<u64>(), r.offsets.as<u64>());
   if ((e = read_back(&total, tileSums.as<u64>() + tiles, sizeof(u64), st)))
     return cuda_status(e, "counting the kNN result");
   ResultState moved;
-  if ((e = result_alloc(moved, 0, sizeof(u32) * std::max<u64>(total, 1), sizeof(double) * std::max<u64>(total, 1), st)))
+  if ((e = result_alloc(moved, sizeof(u64) * (nq + 1), sizeof(u32) * std::max<u64>(total, 1), sizeof(double) * std::max<u64>(total, 1), st)))
     return cuda_status(e, "allocating the result");
-  csr_move_kernel<<<blocks_for(nq * 32), 256, 0, st>>>(start, cnt, r.offsets.as<u64>(), nq, r.ids.as<u32>(), r.dist.as<double>(),
+  scan_apply_kernel<<<u32(tiles), kScanThreads, 0, st>>>(cnt, nq, tileSums.as<u64>(), moved.offsets.as<u64>());
+  csr_move_kernel<<<blocks_for(nq * 32), 256, 0, st>>>(start, cnt, moved.offsets.as<u64>(), nq, a.slot, dk, kAll, r.ids.as<u32>(), r.dist.as<double>(),
                                                         a.outIds, a.outDist, fbr.ids.as<u32>(), fbr.dist.as<double>(), moved.ids.as<u32>(),
                                                         moved.dist.as<double>());
+  std::swap(r.offsets.p, moved.offsets.p);
+  std::swap(r.offsets.bytes, moved.offsets.bytes);
   std::swap(r.ids.p, moved.ids.p);
   std::swap(r.ids.bytes, moved.ids.bytes);
   std::swap(r.dist.p, moved.dist.p);
