@@ -1351,10 +1351,24 @@ struct MinMax<double>
   __device__ __forceinline__ double get() const { return Ord<double>::val((u64(hi) << 32) | lo); }
 };
 
+// A node's least or greatest coordinate that is a zero: with the sign that std::min and std::max keep, which is that
+// of the first one in order (children, then own entities).
+template<typename T>
+__device__ __noinline__ T first_zero(T zero, const T* children, u32 cc, u32 stride, const T* own, u32 n)
+{
+  for (u32 k = 0; k < cc; ++k)
+    if (children[u64(k) * stride] == T(0))
+      return children[u64(k) * stride];
+  for (u32 e = 0; e < n; ++e)
+    if (own[u64(e) * 6] == T(0))
+      return own[u64(e) * 6];
+  return zero;
+}
+
 // ot_dynamic_hash_core.h:1425-1450 (children first, then own entities), one depth per launch. Eight
 // lanes per node: lane k takes child k and every eighth entity, so that neighbouring lanes read
 // neighbouring boxes, and the eight partial boxes are combined by shuffles (min and max are exact, in
-// any order). One lane per node read its entities one after another, 32 lines per load: 0.70 ms for the 65.8M
+// any order, but for the sign of a zero: first_zero). One lane per node read its entities one after another, 32 lines per load: 0.70 ms for the 65.8M
 // FP32 boxes of 4096 trees, 0.22 ms for 8M FP64 boxes.
 template<typename T>
 __global__ void __launch_bounds__(256) mbr_level_kernel(u32 d, const u32* __restrict__ levelCount, const uint4* __restrict__ link,
@@ -1413,8 +1427,12 @@ __global__ void __launch_bounds__(256) mbr_level_kernel(u32 d, const u32* __rest
       }
     if (ok && lane8 < 3)
     {
-      const T lo = lane8 == 0 ? mn[0].get() : lane8 == 1 ? mn[1].get() : mn[2].get();
-      const T hi = lane8 == 0 ? mx[0].get() : lane8 == 1 ? mx[1].get() : mx[2].get();
+      T lo = lane8 == 0 ? mn[0].get() : lane8 == 1 ? mn[1].get() : mn[2].get();
+      T hi = lane8 == 0 ? mx[0].get() : lane8 == 1 ? mx[1].get() : mx[2].get();
+      if (lo == T(0))
+        lo = first_zero<T>(lo, nodeBox + u64(fc) * 6 + lane8, cc, 6, sortedGeom + u64(L.y) * 6 + lane8, L.z - L.y);
+      if (hi == T(0))
+        hi = first_zero<T>(hi, nodeMax + u64(fc) * 3 + lane8, cc, 3, sortedGeom + u64(L.y) * 6 + 3 + lane8, L.z - L.y);
       nodeBox[u64(node) * 6 + lane8] = lo;
       nodeBox[u64(node) * 6 + 3 + lane8] = hi - lo;
       nodeMax[u64(node) * 3 + lane8] = hi;
@@ -1451,12 +1469,12 @@ __global__ void __launch_bounds__(256) root_box_kernel(const uint4* __restrict__
       mx[c] = smax(mx[c], p[c]);
     }
   }
-  // (one thread over 256 partial boxes took 87 us)
+  // (one thread over 256 partial boxes took 87 us; in this order the first lane keeps the first of two zeros)
 #pragma unroll
   for (int c = 0; c < 3; ++c)
   {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
+    for (int o = 1; o < 32; o <<= 1)
     {
       mn[c] = smin(mn[c], __shfl_xor_sync(0xffffffffu, mn[c], o));
       mx[c] = smax(mx[c], __shfl_xor_sync(0xffffffffu, mx[c], o));
