@@ -1167,8 +1167,9 @@ static int status_of(u32 h)
 
 // Runs launch(appender, err) until the append buffer was large enough; items end in c.items. `most` bounds
 // the items (queries times entities): below kItemFloor of them the buffer holds that bound, as a
-// second run costs the whole search again and a larger pooled buffer costs nothing (rays through 1M
-// boxes have 75 hits each where the guess was 16: their search ran twice, 2 x 3.4 ms).
+// second run costs the whole search again and a larger pooled buffer costs no time (rays through 1M
+// boxes have 75 hits each where the guess was 16: their search ran twice, 2 x 3.4 ms). It takes 64 MiB, with
+// distances 128; where the device has no room for it, the guess has to do.
 // workBytes: size of the batched kernels' work buffer (c.work()). launch clears the counters (c.clear)
 // before each search that it runs.
 constexpr u64 kItemFloor = u64(8) << 20;
@@ -1179,10 +1180,23 @@ static int collect(Collected& c, bool withDist, u64 guess, u64 most, size_t work
   c.workBytes = workBytes;
   if ((e = c.count.ensure(32 + workBytes, st)))
     return cuda_status(e, "allocating counters");
-  u64 cap = std::max<u64>(std::max<u64>(guess, 1024), std::min(most, kItemFloor));
+  const u64 least = std::max<u64>(guess, 1024);
+  u64 cap = std::max(least, std::min(most, kItemFloor));
+  const auto reserve = [&] {
+    const cudaError_t a = c.items.ensure(sizeof(u64) * cap, st);
+    return a || !withDist ? a : c.dist.ensure(sizeof(double) * cap, st);
+  };
   for (int attempt = 0; attempt < 3; ++attempt)
   {
-    if ((e = c.items.ensure(sizeof(u64) * cap, st)) || (withDist && (e = c.dist.ensure(sizeof(double) * cap, st))))
+    e = reserve();
+    if (e == cudaErrorMemoryAllocation && attempt == 0 && cap > least)
+    {
+      cudaGetLastError();
+      c.items.release();
+      cap = least;
+      e = reserve();
+    }
+    if (e)
       return cuda_status(e, "allocating result buffer");
     Appender a{ c.items.as<u64>(), withDist ? c.dist.as<double>() : nullptr, c.count.as<unsigned long long>(), cap, true };
     if (int rc = launch(a, c.errp()))
