@@ -1984,6 +1984,9 @@ static int collide_impl(const TreeState& a, const TreeState& b, bool self, doubl
     return cuda_status(e, "filtering pairs");
   swap(c.items, keys);
   c.m = k;
+  // (the order needs about as much room as these)
+  keys.release();
+  list.release();
   r.filterTests = tests;
   r.rechecks = rechecks;
   return finish_pairs(c, a.n, b.n, r, st);

@@ -45,3 +45,13 @@ def test_small_results(dtype):
         for f, w in zip(calls, want):
             assert all(np.array_equal(a, b) for a, b in zip(f(), w) if b is not None)
     assert sum(len(w[1]) for w in want) > 1000
+
+
+def test_collisions():
+    rng = np.random.default_rng(127)
+    c, h = rng.random((1_000_000, 3)) * 100, 0.5 * (0.5 + rng.random((1_000_000, 3)))
+    t = otg.Tree("boxes").create(np.concatenate([c - h, c + h], 1), max_depth=8, max_elements=20)
+    want = t.collision_self()
+    assert len(want) > 2_000_000
+    with pool_of(160 << 20):
+        assert np.array_equal(t.collision_self(), want)
