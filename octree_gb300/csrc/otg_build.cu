@@ -1351,24 +1351,40 @@ struct MinMax<double>
   __device__ __forceinline__ double get() const { return Ord<double>::val((u64(hi) << 32) | lo); }
 };
 
-// A node's least or greatest coordinate that is a zero: with the sign that std::min and std::max keep, which is that
-// of the first one in order (children, then own entities).
+// Dimension c of a node box that begins or ends at zero: with the sign that std::min and std::max keep, which is that of
+// the first zero in order (children, then own entities). Out of line, with few arguments: 8M boxes see it rarely.
 template<typename T>
-__device__ __noinline__ T first_zero(T zero, const T* children, u32 cc, u32 stride, const T* own, u32 n)
+__device__ __noinline__ void first_zeros(u32 node, u32 c, const uint4* link, const T* sortedGeom, T* nodeBox, T* nodeMax)
 {
-  for (u32 k = 0; k < cc; ++k)
-    if (children[u64(k) * stride] == T(0))
-      return children[u64(k) * stride];
-  for (u32 e = 0; e < n; ++e)
-    if (own[u64(e) * 6] == T(0))
-      return own[u64(e) * 6];
-  return zero;
+  const uint4 L = link[node];
+  const u32 fc = L.x & kFirstChildMask, cc = L.x >> kChildShift;
+  T lo = nodeBox[u64(node) * 6 + c], hi = nodeMax[u64(node) * 3 + c];
+  bool lookLo = lo == T(0), lookHi = hi == T(0);
+  const auto see = [&](T l, T h) {
+    if (lookLo && l == T(0))
+    {
+      lo = l;
+      lookLo = false;
+    }
+    if (lookHi && h == T(0))
+    {
+      hi = h;
+      lookHi = false;
+    }
+  };
+  for (u32 k = 0; k < cc && (lookLo || lookHi); ++k)
+    see(nodeBox[u64(fc + k) * 6 + c], nodeMax[u64(fc + k) * 3 + c]);
+  for (u32 e = L.y; e < L.z && (lookLo || lookHi); ++e)
+    see(sortedGeom[u64(e) * 6 + c], sortedGeom[u64(e) * 6 + 3 + c]);
+  nodeBox[u64(node) * 6 + c] = lo;
+  nodeBox[u64(node) * 6 + 3 + c] = hi - lo;
+  nodeMax[u64(node) * 3 + c] = hi;
 }
 
 // ot_dynamic_hash_core.h:1425-1450 (children first, then own entities), one depth per launch. Eight
 // lanes per node: lane k takes child k and every eighth entity, so that neighbouring lanes read
 // neighbouring boxes, and the eight partial boxes are combined by shuffles (min and max are exact, in
-// any order, but for the sign of a zero: first_zero). One lane per node read its entities one after another, 32 lines per load: 0.70 ms for the 65.8M
+// any order, but for the sign of a zero: first_zeros). One lane per node read its entities one after another, 32 lines per load: 0.70 ms for the 65.8M
 // FP32 boxes of 4096 trees, 0.22 ms for 8M FP64 boxes.
 template<typename T>
 __global__ void __launch_bounds__(256) mbr_level_kernel(u32 d, const u32* __restrict__ levelCount, const uint4* __restrict__ link,
@@ -1427,15 +1443,13 @@ __global__ void __launch_bounds__(256) mbr_level_kernel(u32 d, const u32* __rest
       }
     if (ok && lane8 < 3)
     {
-      T lo = lane8 == 0 ? mn[0].get() : lane8 == 1 ? mn[1].get() : mn[2].get();
-      T hi = lane8 == 0 ? mx[0].get() : lane8 == 1 ? mx[1].get() : mx[2].get();
-      if (lo == T(0))
-        lo = first_zero<T>(lo, nodeBox + u64(fc) * 6 + lane8, cc, 6, sortedGeom + u64(L.y) * 6 + lane8, L.z - L.y);
-      if (hi == T(0))
-        hi = first_zero<T>(hi, nodeMax + u64(fc) * 3 + lane8, cc, 3, sortedGeom + u64(L.y) * 6 + 3 + lane8, L.z - L.y);
+      const T lo = lane8 == 0 ? mn[0].get() : lane8 == 1 ? mn[1].get() : mn[2].get();
+      const T hi = lane8 == 0 ? mx[0].get() : lane8 == 1 ? mx[1].get() : mx[2].get();
       nodeBox[u64(node) * 6 + lane8] = lo;
       nodeBox[u64(node) * 6 + 3 + lane8] = hi - lo;
       nodeMax[u64(node) * 3 + lane8] = hi;
+      if (lo == T(0) || hi == T(0))
+        first_zeros<T>(node, lane8, link, sortedGeom, nodeBox, nodeMax);
     }
   }
 }
