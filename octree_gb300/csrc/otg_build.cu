@@ -1603,10 +1603,16 @@ static int build_impl(TreeState& t, const T* ent, const void* box, u64 n, cudaSt
   // buffers
   const u64 maxNodes = n + u64(D) * (n / (t.maxElem + 1) + 1) + 2;
   t.maxNodes = maxNodes;
-  if ((e = t.keysA.ensure(sizeof(K) * n)) || (e = t.keysB.ensure(sizeof(K) * n)) || (e = t.sortedIds.ensure(sizeof(u32) * n)) ||
-      (e = t.valsB.ensure(sizeof(u32) * n)) || (e = t.sortedGeom.ensure(sizeof(T) * W * n)) || (e = t.nodeLink.ensure(sizeof(uint4) * maxNodes)) ||
-      (e = t.nodeKey.ensure(sizeof(u64) * maxNodes)) || (e = t.nodeBox.ensure(sizeof(T) * 6 * maxNodes)) ||
-      (e = t.nodeDepth.ensure(maxNodes)) || (e = t.levelCount.ensure(sizeof(u32) * 64)) ||
+  // An Insert leaves node arrays of the tree's own size, from the pool; here they are sized by a bound, so a Create on the
+  // same tree needs larger ones. From the pool again that costs next to nothing; with cudaMalloc and cudaFree, which wait
+  // for the device, 0.67 ms for 4M points.
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  const bool pooled = cudaStreamIsCapturing(st, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone;
+  const auto room = [&](DevBuf& b, size_t need) { return b.pooled && pooled ? b.ensure_pooled(need, st) : b.ensure(need); };
+  if ((e = t.keysA.ensure(sizeof(K) * n)) || (e = t.keysB.ensure(sizeof(K) * n)) || (e = room(t.sortedIds, sizeof(u32) * n)) ||
+      (e = room(t.valsB, sizeof(u32) * n)) || (e = room(t.sortedGeom, sizeof(T) * W * n)) || (e = room(t.nodeLink, sizeof(uint4) * maxNodes)) ||
+      (e = room(t.nodeKey, sizeof(u64) * maxNodes)) || (e = room(t.nodeBox, sizeof(T) * 6 * maxNodes)) ||
+      (e = room(t.nodeDepth, maxNodes)) || (e = t.levelCount.ensure(sizeof(u32) * 64)) ||
       (e = t.splitQueue.ensure(2 * sizeof(u32) * (n / (t.maxElem + 1) + 2))) || (e = t.space.ensure(sizeof(Space<T>))) ||
       (e = t.sortScratch.ensure(chunked ? ChunkScratch::bytes() : SortScratch::bytes(n, plan.passes, plan.radix))) || (e = t.bboxBits.ensure(sizeof(U) * 6)) ||
       (e = t.rasterTab.ensure(tabBytes)) || (e = t.minTab.ensure(sizeof(T) * minTabEntries)) ||
@@ -3481,12 +3487,10 @@ static int insert_impl(TreeState& t, const T* pts, u64 n2, cudaStream_t st)
 
   // 6. the new tree
   prof.mark("write", st);
-  // (at least as large as the arrays they replace: a Create sizes its node arrays by a bound, and one that
-  // follows on this tree then finds room and pays no cudaMalloc / cudaFree, 0.67 ms for 4M points)
   DevBuf ids, geom, link, key, box, depth;
-  if ((e = ids.ensure_pooled(std::max(sizeof(u32) * nt, t.sortedIds.bytes), st)) || (e = geom.ensure_pooled(std::max(sizeof(T) * 3 * nt, t.sortedGeom.bytes), st)) ||
-      (e = link.ensure_pooled(std::max(sizeof(uint4) * F, t.nodeLink.bytes), st)) || (e = key.ensure_pooled(std::max(sizeof(u64) * F, t.nodeKey.bytes), st)) ||
-      (e = box.ensure_pooled(std::max(sizeof(T) * 6 * F, t.nodeBox.bytes), st)) || (e = depth.ensure_pooled(std::max(size_t(F), t.nodeDepth.bytes), st)))
+  if ((e = ids.ensure_pooled(sizeof(u32) * nt, st)) || (e = geom.ensure_pooled(sizeof(T) * 3 * nt, st)) ||
+      (e = link.ensure_pooled(sizeof(uint4) * F, st)) || (e = key.ensure_pooled(sizeof(u64) * F, st)) ||
+      (e = box.ensure_pooled(sizeof(T) * 6 * F, st)) || (e = depth.ensure_pooled(F, st)))
     return cuda_status(e, "allocating the inserted tree");
   insert_old_entities_kernel<T><<<blocks_for(n), 256, 0, st>>>(oldOwner.as<u32>(), u32(n), startNew.as<u32>(), t.sortedIds.as<u32>(), t.sortedGeom.as<T>(),
                                                                ids.as<u32>(), geom.as<T>());

@@ -55,3 +55,17 @@ def test_collisions():
     assert len(want) > 2_000_000
     with pool_of(160 << 20):
         assert np.array_equal(t.collision_self(), want)
+
+
+def test_insert():
+    """The new arrays are as large as the tree, not as the bound that a Create sizes its own by."""
+    rng = np.random.default_rng(131)
+    p, q = rng.random((1_000_000, 3)), rng.random((200_000, 3))
+    box = np.array([[0.0, 0, 0, 1, 1, 1]])
+    for limit in (1 << 30, 96 << 20):
+        t = otg.Tree("points").create(p, max_depth=8, max_elements=20, box=box)
+        with pool_of(limit):
+            t.insert(q)
+            off, ids, dist = t.knn(q[:100], 1)
+            del t
+        assert (dist == 0).all()
