@@ -1246,7 +1246,7 @@ int use_images(TreeState& t, TreeView<double>& tv, u64 tests, cudaStream_t st)
       return OTG_OK;
   }
   if (int rc = ensure_image32(t, st, isBox))
-    return rc;
+    return rc == OTG_ERR_OUT_OF_MEMORY ? OTG_OK : rc; // without room for them the exact tests answer as they are
   tv.nodeImg = t.nodeBox32.as<float4>();
   if (isBox)
     tv.boxImg = t.boxImg32.as<float4>();
