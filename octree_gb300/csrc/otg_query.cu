@@ -1905,7 +1905,11 @@ static int ray_impl(const TreeState& t, const void* rays, u64 nq, double tol, do
   }
   else
   {
-    const bool plain = algo == OTG_ALGO_PLAIN_FP64;
+    // Many rays through point trees of a node or two leave most of a warp per ray without a point, and FP64 tests cost
+    // a lane what they cost 32: one ray per thread then. 20k rays on 2000 trees: FP64 of 8, 16, 32 points 235, 246 and 384 us
+    // by warps, 111, 137 and 319 by threads (64 points 395, 442); FP32 of 16 86 and 75 (24 points 87, 88). 2000 rays: warps.
+    const u64 few = (sizeof(T) == 8 ? 32 : 16) * std::max<u64>(t.trees, 1);
+    const bool plain = algo == OTG_ALGO_PLAIN_FP64 || (!tv.isBox && t.n <= few && nq >= 4096);
     if (plain)
       if (cudaError_t e = M.ensure(sizeof(T) * nq, st))
         return cuda_status(e, "allocating ray thresholds");
