@@ -304,9 +304,25 @@ __device__ __forceinline__ void run_order_general(u32* ids, double* dist, u64* s
   }
 }
 
+// a run that a warp does not sort: into the list for run_sort_block_kernel, or only counted (longCount[1]) where it is too
+// long for that: the caller then orders everything another way and spares the block sorts (64 views of 500k
+// boxes, 89k ids of which one view has more than 8192: 58 us of 0.36 ms)
+constexpr u32 kBlockRunMax = 8192;
+__device__ __forceinline__ void list_long_run(u32 run, u64 len, u32* longCount, u32* longRuns, u32 longCap)
+{
+  if (len > kBlockRunMax)
+  {
+    atomicAdd(longCount + 1, 1u);
+    return;
+  }
+  const u32 at = atomicAdd(longCount, 1u);
+  if (at < longCap)
+    longRuns[at] = run;
+}
+
 // One warp per query sorts its run in place: ids as words in registers, distances by packed words, or by the general
 // order where those give up. Runs above kRunSortMax go to the list longRuns (longCount[0] counts them)
-// for run_sort_block_kernel. Bound by issue: the general order for every run took 0.149 ms for the distances of 60k rays
+// for run_sort_block_kernel (list_long_run). Bound by issue: the general order for every run took 0.149 ms for the distances of 60k rays
 // (now 0.050), 8.1 us for the ids of 10k ranges of about 60 points (now 4.0) and 38.6 us for those of a forest's 1M ranges
 // of a few boxes (33.9; 60 at the occupancy that the compiler's choice of registers for 256 ids left).
 template<bool DIST>
@@ -326,11 +342,7 @@ __global__ void __launch_bounds__(kRunSortWarps * 32, DIST ? 0 : 8) run_sort_ker
     if (len64 > kRunSortMax)
     {
       if (lane == 0)
-      {
-        const u32 at = atomicAdd(longCount, 1u);
-        if (at < longCap)
-          longRuns[at] = u32(q);
-      }
+        list_long_run(u32(q), len64, longCount, longRuns, longCap);
       continue;
     }
     const u32 len = u32(len64);
@@ -370,13 +382,12 @@ __global__ void __launch_bounds__(kRunSortWarps * 32, DIST ? 0 : 8) run_sort_ker
   }
 }
 
-// One block per listed run sorts it in place with a bitonic network in shared memory (dynamic: 12 or
-// 4 bytes per item); runs above kBlockRunMax are only counted, in longCount[1].
-constexpr u32 kBlockRunMax = 8192;
+// One block per listed run (at most kBlockRunMax items) sorts it in place with a bitonic network in shared memory
+// (dynamic: 12 or 4 bytes per item).
 constexpr int kBlockSortThreads = 512;
 template<bool DIST>
 __global__ void __launch_bounds__(kBlockSortThreads) run_sort_block_kernel(const u64* __restrict__ off, u32* __restrict__ ids, double* __restrict__ dist,
-                                                                         u32* __restrict__ longCount, const u32* __restrict__ longRuns, u32 longCap)
+                                                                         const u32* __restrict__ longCount, const u32* __restrict__ longRuns, u32 longCap)
 {
   extern __shared__ u64 runMem[];
   u64* sd = runMem;
@@ -386,14 +397,7 @@ __global__ void __launch_bounds__(kBlockSortThreads) run_sort_block_kernel(const
   {
     const u32 q = longRuns[r];
     const u64 b = off[q];
-    const u64 len64 = off[q + 1] - b;
-    if (len64 > kBlockRunMax)
-    {
-      if (threadIdx.x == 0)
-        atomicAdd(longCount + 1, 1u);
-      continue;
-    }
-    const u32 len = u32(len64);
+    const u32 len = u32(min(off[q + 1] - b, u64(kBlockRunMax)));
     u32 P = 512;
     while (P < len)
       P <<= 1;
@@ -588,11 +592,7 @@ __global__ void __launch_bounds__(256) pair_write_kernel(const u64* __restrict__
     const u64 prev = __shfl_up_sync(~0u, at, 1);
     const u32 first = u32((lane ? prev : base) - base), len = u32(at - base) - first;
     if (len > kRunSortMax)
-    {
-      const u32 to = atomicAdd(longCount, 1u);
-      if (to < longCap)
-        longRuns[to] = u32(a0) + lane;
-    }
+      list_long_run(u32(a0) + lane, len, longCount, longRuns, longCap);
     for (u32 mid = __ballot_sync(~0u, len > kPairRankMax && len <= kRunSortMax); mid; mid &= mid - 1)
     {
       const u32 r = u32(__ffs(int(mid))) - 1;

@@ -1269,7 +1269,8 @@ static int order_by_runs(Collected& c, u64 nq, ResultState& r, bool withDist, cu
   u32 h[2] = { 0, 0 };
   if ((e = cudaGetLastError()) || (e = read_back(h, longCount, sizeof(h), st)))
     return cuda_status(e, "finishing result");
-  if (h[0])
+  done = h[1] == 0;
+  if (done && h[0])
   {
     const u32 longGrid = std::min<u32>(h[0], 152 * 2);
     if (withDist)
@@ -1281,10 +1282,10 @@ static int order_by_runs(Collected& c, u64 nq, ResultState& r, bool withDist, cu
     }
     else
       run_sort_block_kernel<false><<<longGrid, kBlockSortThreads, kBlockRunMax * 4, st>>>(off, r.ids.as<u32>(), nullptr, longCount, longRuns, u32(longCap));
-    if ((e = cudaGetLastError()) || (e = read_back(h, longCount, sizeof(h), st)))
+    e = cudaStreamSynchronize(st);
+    if (e || (e = cudaGetLastError()))
       return cuda_status(e, "finishing result");
   }
-  done = h[1] == 0;
   return OTG_OK;
 }
 
@@ -1457,16 +1458,16 @@ static int finish_pairs(Collected& c, u64 nA, u64 nB, ResultState& r, cudaStream
     u32 h[2] = { 0, 0 };
     if ((e = cudaGetLastError()) || (e = read_back(h, longCount, sizeof(h), st)))
       return cuda_status(e, "ordering pairs");
-    if (h[0])
+    done = h[1] == 0;
+    if (done && h[0])
     {
       const u32 grid = std::min<u32>(h[0], 152 * 4);
       run_sort_block_kernel<false><<<grid, kBlockSortThreads, kBlockRunMax * 4, st>>>(off.as<u64>(), bs.as<u32>(), nullptr, longCount, longRuns,
                                                                                     u32(longCap));
       pair_long_write_kernel<<<grid, 256, 0, st>>>(off.as<u64>(), bs.as<u32>(), r.ids.as<uint2>(), longCount, longRuns, u32(longCap));
-      if ((e = cudaGetLastError()) || (e = read_back(h, longCount, sizeof(h), st)))
+      if ((e = cudaGetLastError()))
         return cuda_status(e, "ordering pairs");
     }
-    done = h[1] == 0;
   }
   if (!done)
   {
