@@ -469,7 +469,7 @@ __device__ __forceinline__ float cell_estimate_margin(const Space<T>& s, int d, 
 // decided where the largest size clears the powers of two beside it by 3 m; the location keeps the
 // cells' bits from that level up, decided where the centre in units of the level's cells clears the
 // integers by 2 m. The rest take the tables' binary searches, five steps per dimension and table, which
-// set the kernel's time: 65.8M FP32 boxes of 4096 trees 1.07 ms, now 0.49; 8M FP64 boxes 0.182 ms, now 0.099.
+// set the kernel's time: 65.8M FP32 boxes of 4096 trees 1.07 ms, now 0.44; 8M FP64 boxes 0.182 ms, now 0.099.
 template<typename T>
 __device__ __forceinline__ bool box_key_estimate(const T* e, u32 res, const float* minF, const float* rastF, const float* margF, u32 D, u64& key)
 {
@@ -833,7 +833,6 @@ struct GatherUnit<16>
 };
 constexpr int kGatherPerThread = 8;
 
-// vec: both arrays start on a multiple of the unit (the tree's always does; a caller's may not)
 // a load that brings its 256 bytes into L2
 template<typename U>
 __device__ __forceinline__ U load_near(const U* p)
@@ -847,6 +846,7 @@ __device__ __forceinline__ U load_near(const U* p)
     asm volatile("ld.global.nc.L2::256B.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
   return v;
 }
+// vec: both arrays start on a multiple of the unit (the tree's always does; a caller's may not).
 // A block of a single tree's gather takes units a grid apart (its points are read at random, and few blocks leave
 // room for the emission). A forest's block (kGatherRuns) takes G * 256 consecutive units, so that the blocks in
 // flight read a few tens of trees: 65.8M boxes of 4096 trees 0.76 ms, 1.01 with units a grid apart; four trees

@@ -273,7 +273,7 @@ struct TreeState
   // mutex, and every stream that uses them waits for the event recorded after their kernels.
   std::mutex imageMutex;
   cudaEvent_t imageReady = nullptr;
-  u64 imageTests = 0; // entity tests of the box queries since the build (use_box_images)
+  u64 imageTests = 0; // entity tests of the box queries since the build (use_images)
   // set_entities changed the geometry: entities may lie outside their nodes
   bool respanned = false;
   // a bulk Insert changed the tree: nodes may own entities beside their children and child links

@@ -1239,7 +1239,8 @@ int use_images(TreeState& t, TreeView<double>& tv, u64 tests, cudaStream_t st)
   {
     // building the images moves 80 bytes of every box (40 of a point) and a test that they spare reads 48
     // and takes some 30 FP64 operations: worth it from about one test per entity on, so that a tree
-    // rebuilt for a few queries does not pay for them
+    // rebuilt for a few queries does not pay for them (1M boxes built anew, then 2000, 4000, 8000 and 64000 ranges of 128
+    // estimated tests: 114, 143, 213 and 1070 us by exact tests, 114, 127, 142 and 310 with the images built by the call)
     std::lock_guard<std::mutex> g(t.imageMutex);
     t.imageTests += tests;
     if (!(isBox ? t.boxImage32 : t.image32) && t.imageTests < t.n)

@@ -161,7 +161,7 @@ static void plan_sort(K*& k, u32*& v, K*& kB, u32*& vB, u64 cap, const unsigned 
   cudaMemsetAsync(scratch.p, 0, SortScratch::bytes(cap, passes), st);
   SortScratch ss;
   ss.carve(scratch.p, cap, passes);
-  radix_histogram_kernel<K><<<blocks_for(cap), 256, 0, st>>>(k, cap, 0, passes, ss.hist, m);
+  radix_histogram_kernel<K><<<blocks_for(cap), 256, 0, st>>>(k, cap, passes, ss.hist, m);
   if (onesweep_passes_devn<K>(k, v, kB, vB, cap, m, passes, false, ss, err, st))
   {
     std::swap(k, kB);

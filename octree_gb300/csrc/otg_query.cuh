@@ -27,12 +27,13 @@ struct TreeView
   const u32* qTree;   // forest: tree (= root node) of each query; null for a single tree
   const u64* treeOff; // forest: first entity of each tree (ids are returned relative to it)
   const unsigned char* nodeDepth; // depth of each node below its tree's root
-  // FP32 images (point trees of FP64 entities, built on demand): outward-rounded node boxes (two
-  // float4 per node) and round-to-nearest entities; null where a kernel takes the FP64 tests only
+  // FP32 images (FP64 trees, built on demand): outward-rounded node boxes (two float4 per node),
+  // round-to-nearest points, and outward-rounded boxes {min}, {max} (two float4 per entity); null where a
+  // kernel takes the FP64 tests only
   const float4* nodeImg = nullptr;
   const float4* pointImg = nullptr;
   bool inNodes = true; // every entity lies in its node's box (not after set_entities)
-  const float4* boxImg = nullptr; // box trees: {min rounded down}, {max rounded up} (two float4 per entity)
+  const float4* boxImg = nullptr;
 };
 
 // root node and id base of query q (node t is the root of tree t in a forest)
@@ -261,7 +262,7 @@ static inline int sort_pairs_u64(u64* keys, u32* vals, u64 m, u32 bits, cudaStre
   cudaMemsetAsync(scratch.p, 0, SortScratch::bytes(m, passes), st);
   SortScratch ss;
   ss.carve(scratch.p, m, passes);
-  radix_histogram_kernel<u64><<<blocks_for(m), 256, 0, st>>>(keys, m, 0, passes, ss.hist);
+  radix_histogram_kernel<u64><<<blocks_for(m), 256, 0, st>>>(keys, m, passes, ss.hist);
   bool inB = onesweep_passes<u64>(keys, vals, k1.as<u64>(), v1.as<u32>(), m, passes, false, ss, err, st);
   if (inB)
   {
@@ -284,7 +285,7 @@ static inline int sort_pairs_u32(u32* keys, u32* vals, u64 m, u32 bits, cudaStre
   cudaMemsetAsync(scratch.p, 0, SortScratch::bytes(m, passes), st);
   SortScratch ss;
   ss.carve(scratch.p, m, passes);
-  radix_histogram_kernel<u32><<<blocks_for(m), 256, 0, st>>>(keys, m, 0, passes, ss.hist);
+  radix_histogram_kernel<u32><<<blocks_for(m), 256, 0, st>>>(keys, m, passes, ss.hist);
   bool inB = onesweep_passes<u32>(keys, vals, k1.as<u32>(), v1.as<u32>(), m, passes, false, ss, err, st);
   if (inB)
   {

@@ -29,7 +29,7 @@ struct RadixPlan
 // ends in a depth of five bits that is at most D, so only its lowest bits are sorted by: 26 key bits of
 // depth 6 are 24, three passes instead of four (8M FP64 boxes: 0.24 ms of passes, then 0.19). Nine-bit digits (wide)
 // where they save a pass: a pass of them costs a tenth more (512 counters per warp instead of 256, more
-// statuses, and three blocks still fit an SM): 65.8M boxes of a forest of depth 4, 18 bits, 1.34 ms in three passes, 1.08 in two.
+// statuses, and three blocks still fit an SM): 65.8M boxes of a forest of depth 4, 18 bits, 1.13 ms in three passes, 0.78 in two.
 inline RadixPlan radix_plan(u32 bits, u32 low, u32 gap, bool wideAllowed)
 {
   RadixPlan r = {};

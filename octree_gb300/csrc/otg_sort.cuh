@@ -90,11 +90,11 @@ __device__ __forceinline__ u32 lanemask_lt()
   return m;
 }
 
-// All-pass digit histograms of `keys` (shift0 + 8p for p < passes) accumulated into hist[p][256].
+// All-pass digit histograms of `keys` (bits from 8p for p < passes) accumulated into hist[p][256].
 // nDev (optional): the element count in device memory (at most n), for launches recorded before
 // the count is known (graph replay)
 template<typename K>
-__global__ void __launch_bounds__(256) radix_histogram_kernel(const K* __restrict__ keys, u64 n, u32 shift0, u32 passes, u32* __restrict__ hist,
+__global__ void __launch_bounds__(256) radix_histogram_kernel(const K* __restrict__ keys, u64 n, u32 passes, u32* __restrict__ hist,
                                                              const unsigned long long* __restrict__ nDev = nullptr)
 {
   if (nDev)
@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(256) radix_histogram_kernel(const K* __restric
   {
     K k = keys[i];
     for (u32 p = 0; p < passes; ++p)
-      atomicAdd(&sh[p][(k >> (shift0 + kRadixBits * p)) & (kRadix - 1)], 1u);
+      atomicAdd(&sh[p][(k >> (kRadixBits * p)) & (kRadix - 1)], 1u);
   }
   __syncthreads();
   for (u32 p = 0; p < passes; ++p)
@@ -457,9 +457,6 @@ inline size_t onesweep_smem_bytes()
   return (sizeof(K) + sizeof(u32)) * kSortTile;
 }
 
-// Runs the passes of a sort whose histograms are already in scratch.hist (zeroed scratch otherwise).
-// Pass p reads buffer (p even ? 0 : 1) and writes the other one; returns true when the sorted
-// result is in (k1, v1). iotaValues: the first pass generates values 0..n-1 instead of reading v0.
 inline bool sort_staging_enabled()
 {
   static const bool on = [] {
@@ -469,7 +466,9 @@ inline bool sort_staging_enabled()
   return on;
 }
 
-// the passes of a plan, RADIX digits each
+// The passes of a plan, RADIX digits each, of a sort whose histograms are already in scratch.hist (zeroed scratch
+// otherwise). Pass p reads buffer (p even ? 0 : 1) and writes the other one; returns true when the sorted
+// result is in (k1, v1). iotaValues: the first pass generates values 0..n-1 instead of reading v0.
 template<typename K, int RADIX>
 inline bool onesweep_plan_passes(K* k0, u32* v0, K* k1, u32* v1, u64 n, const RadixPlan& plan, bool iotaValues, SortScratch& s, u32* err, cudaStream_t st)
 {
